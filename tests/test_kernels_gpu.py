@@ -60,6 +60,31 @@ def test_gemm_simt(M, N, K, adt, wdt):
     assert (x.double() - ref_linear(a, w, bias, None, add0, add1)).abs().max() <= 2e-5 * max(1.0, ref.abs().max().item())
 
 
+@pytest.mark.parametrize("N,K", [(1, 4), (70, 36), (130, 100), (64, 260), (2048, 2048), (200, 8192), (51200, 64)])
+def test_gemm_f32_rows(N, K):
+    """32-bit operands with whole 16-byte rows: every height of tile and its edges, K of less than a k-block to
+    many; and a row is the same number whatever rows are beside it (the tile, and so how K is shared, changes).
+    The bound: K products of relative error 2^-24 each, summed in four parts."""
+    o = ops()
+    M = 200 if N < 51200 else 40
+    a, w = rnd(M, K, seed=1), rnd(N, K, scale=K ** -0.5, seed=2)
+    bias, add0, add1 = rnd(N, seed=3), rnd(M, N, seed=4), rnd(M, N, seed=5)
+    ref = ref_linear(a, w, bias, "gelu", add0, add1)
+    bound = 2 ** -24 * (8 + K ** 0.5) * (a.double().abs() @ w.double().abs().T + 4)
+    whole = o.gemm_simt(a, w, bias, "gelu", add0, add1)
+    assert ((whole.double() - ref).abs() <= bound).all()
+    for m in (1, 7, 8, 9, 16, 17, 32, 33, 64, 65, 128, 129):
+        if m > M:
+            break
+        part = o.gemm_simt(a[M - m:], w, bias, "gelu", add0[M - m:], add1[M - m:])
+        assert torch.equal(part, whole[M - m:]), m
+    rounded = o.gemm_simt(a[:5], w, bias, None, out_dtype=torch.bfloat16)
+    assert torch.equal(rounded, o.gemm_simt(a[:5], w, bias, None).bfloat16())
+    x = add0.clone()
+    o.gemm_simt(a, w, bias, "gelu", x, add1, out=x)
+    assert torch.equal(x, whole)
+
+
 @pytest.mark.parametrize("M", [1, 3, 8, 9, 16, 33, 64])
 @pytest.mark.parametrize("N,K", [(40, 160), (1000, 200), (2560, 2560), (130, 4104)])
 def test_gemm_skinny(M, N, K):
