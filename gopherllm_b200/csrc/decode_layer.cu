@@ -33,7 +33,13 @@
 // (whole tiles where that keeps nine blocks in ten busy; in phase 3, while there are no more tiles than
 // blocks, whole blocks to a tile, each with an equal share of the down part's and of the out part's
 // chunks); the two halves of a block split each of its runs of chunks in two.  Attention is a line of
-// (sequence, key/value head, page) units cut over the halves in the same way.
+// (key/value head, sequence, page) units cut over the halves in the same way.  A head of a sequence also
+// costs a half something beside its pages (fetching and turning the queries, storing the new key, merging), about
+// as much as two or three pages: it counts for DL_LEAD units more than it has pages, and the line runs head by
+// head, so that a half meets sequences of different lengths.  (Sequence by sequence and by pages alone, the
+// halves that got the short sequences walked through sixty heads of one page while the others waited: 64
+// sequences of 16 to 1,024 positions took 214 us a layer of Phi-2, now 126; 40 of 16 to 700 of Phi-1.5 82
+// with pages alone, 78 with DL_LEAD; equal lengths are unchanged.)
 //
 // The products run on tcgen05: the 128 weight rows of a tile are the M of the instruction, the tokens
 // (padded to 16, 32 or 64) its N, the accumulator lies in tensor memory; one thread issues the four
@@ -70,6 +76,7 @@ static_assert(GL_HEAD_DIM % 16 == 0 && GL_HEAD_DIM >= 16 && GL_HEAD_DIM <= 128, 
 // tile), and every access goes through dl_page_off.  Other row lengths spread over the banks by themselves.
 #define DL_PAGE_SWIZZLED ((DL_ROWB % 128) == 0)
 #define DL_PAGE_TILES (DL_PAGE_SWIZZLED ? DL_HD / 64 : 1)
+#define DL_LEAD 2                     // units a sequence's head counts for beside its pages
 #define DL_MAXG 8                     // query heads per key/value head
 #define DL_MAXB 64                    // sequences (= tokens) per step
 #define DL_GEN 32                     // the barrier's generation word, a cache line away from its arrival count
@@ -260,7 +267,7 @@ decode_layer_kernel(const __grid_constant__ LayerArgs a) {
     const unsigned acc_bar = empty0 + 8 * NS;             // the accumulator of a run of chunks is complete
     unsigned* tmem_slot = (unsigned*)(smem0 + NS * DL_STAGE + 16 * NS + 8);      // in the first half's part
     unsigned char* misc = smem + NS * DL_STAGE + 16 * NS + 16;
-    int* s_off = (int*)misc;                              // [MAXB + 1] first unit of each sequence in phase 2
+    int* s_off = (int*)misc;                              // [MAXB + 1] first unit of each sequence in a head's stretch of phase 2
     int* s_first = s_off + DL_MAXB + 1;                   // [MAXB] first page each sequence reads
     int* s_n = s_first + DL_MAXB;                         // [MAXB] pages each sequence reads
     int* s_flag = s_n + DL_MAXB;                          // [7] (200 ints so far: what follows stays 16-byte aligned)
@@ -290,7 +297,7 @@ decode_layer_kernel(const __grid_constant__ LayerArgs a) {
             s_off[b] = off;
             s_first[b] = lo / GL_PAGE;
             s_n[b] = pos / GL_PAGE + 1 - lo / GL_PAGE;
-            off += s_n[b] * p.nKV;
+            off += DL_LEAD + s_n[b];
         }
         s_off[p.M] = off;
     }
@@ -300,7 +307,7 @@ decode_layer_kernel(const __grid_constant__ LayerArgs a) {
     __syncthreads();
     tc_fence_after();
     const unsigned tmem = *tmem_slot + half * TMEM_COLS;
-    // the sequence whose units hold unit L of the attention's line: the last b with s_off[b] <= L
+    // the sequence whose units hold unit L of a head's stretch of the attention's line: the last b with s_off[b] <= L
     auto seq_of = [&](int L) {
         int lo = 0, hi = p.M - 1;
         while (lo < hi) {
@@ -309,9 +316,22 @@ decode_layer_kernel(const __grid_constant__ LayerArgs a) {
         }
         return lo;
     };
-    const int totalA = s_off[p.M];
+    const int headA = s_off[p.M], totalA = headA * p.nKV;
     const int perA = (totalA + GC - 1) / GC;
     const int a0 = min(totalA, c * perA), a1 = min(totalA, a0 + perA);
+    // The next run of pages at or behind unit L of this block's stretch: ``cnt`` pages from the pi-th on of head g of
+    // sequence b; L moves to the first of them.  False where only units without a page are left.
+    auto pages_at = [&](int& L, int& b, int& g, int& pi, int& cnt) {
+        g = L / headA;
+        const int r = L - g * headA;
+        b = seq_of(r);
+        const int u = r - s_off[b], skip = max(0, DL_LEAD - u);
+        if (skip >= a1 - L) return false;
+        L += skip;
+        pi = u + skip - DL_LEAD;
+        cnt = min(s_n[b] - pi, a1 - L);
+        return true;
+    };
     const int total1 = (a.tiles_q + a.tiles_u) * a.kc1, total3 = a.tiles3 * a.kc3;
     // the products are cut over the launched blocks; the two halves of a block share every run of chunks
     const int cb = blockIdx.x;
@@ -424,10 +444,8 @@ decode_layer_kernel(const __grid_constant__ LayerArgs a) {
             const CUtensorMap* pmap = second ? &a.v_pages : &a.k_pages;
             int L = a0;
             while (L < a1) {
-                const int b = seq_of(L);
-                const int nb = s_n[b];
-                const int g = (L - s_off[b]) / nb, pi = (L - s_off[b]) - g * nb;
-                const int cnt = min(nb - pi, a1 - L);
+                int b, g, pi, cnt;
+                if (!pages_at(L, b, g, pi, cnt)) break;
                 for (int j0 = 0; j0 < cnt; j0 += 32) {
                     const int mine = j0 + lane;
                     const int pg = mine < cnt ? gl_checked(p.pages[(size_t)b * p.max_pages + gl_checked(s_first[b] + pi + mine, p.max_pages, GL_BAD_POSITION)],
@@ -677,10 +695,9 @@ decode_layer_kernel(const __grid_constant__ LayerArgs a) {
         const int OSZ = G * DL_HD + 2 * G;                // floats of one partial result
         int L = a0;
         while (L < a1) {
-            const int b = seq_of(L);
+            int b, g, pi0, cnt;
+            if (!pages_at(L, b, g, pi0, cnt)) break;
             const int nb = s_n[b];
-            const int g = (L - s_off[b]) / nb, pi0 = (L - s_off[b]) - g * nb;
-            const int cnt = min(nb - pi0, a1 - L);
             const int pos = p.seq_ctx[b];
             const int lo = (p.window > 0 && pos - p.window + 1 > 0) ? pos - p.window + 1 : 0;
             const size_t head_off = (size_t)g * GL_PAGE * DL_HD;
@@ -820,7 +837,7 @@ decode_layer_kernel(const __grid_constant__ LayerArgs a) {
             }
             cons_sync();
             // which blocks hold pages of this (sequence, head), and this block's number among them
-            const int Ls = s_off[b] + g * nb;
+            const int Ls = g * headA + s_off[b] + DL_LEAD;
             const int first = Ls / perA, last = (Ls + nb - 1) / perA;
             const int nseg = last - first + 1, ord = c - first;
             float* part = a.scratchA + ((size_t)(b * p.nKV + g) * a.maxsegA) * OSZ;

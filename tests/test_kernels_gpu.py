@@ -754,9 +754,25 @@ def test_decode_layer(M, nH, nKV, hd, D, I, rot, window, rms, act, bias):
     """norm -> (attention over the paged cache | feed-forward) -> residual sum as one kernel, against the
     same layer written out in 64-bit: the residual stream, and the cache (the new token's rotated key and
     its value where they belong, everything else, NaN filling included, untouched)."""
-    o = ops()
     rng = np.random.default_rng(M + hd)
     ctxs = [0, 63, 64, 200, 129][:M] if M <= 5 else [int(c) for c in rng.integers(0, 300, size=M)]
+    check_decode_layer(M, nH, nKV, hd, D, I, rot, window, rms, act, bias, ctxs)
+
+
+@pytest.mark.parametrize("window", [0, 70])
+@pytest.mark.parametrize("ctxs", [
+    [0] * 20 + [1500] + [0] * 20,               # one long sequence among many of a single page
+    [63, 64, 65, 0] * 16,                       # a page's edges only
+    [1000 - 15 * i for i in range(64)],         # every length from long to short
+    [5],
+])
+def test_decode_layer_unequal_lengths(ctxs, window):
+    """The pages of all sequences' heads are cut into equal stretches, where a head counts for more than its pages."""
+    check_decode_layer(len(ctxs), 4, 2, 64, 256, 328, 32, window, False, "gelu_new", True, ctxs)
+
+
+def check_decode_layer(M, nH, nKV, hd, D, I, rot, window, rms, act, bias, ctxs):
+    o = ops()
     dtype = torch.bfloat16
     L = max(ctxs) + 1
     k = rnd(M, L, nKV, hd, seed=1).to(dtype).float()
