@@ -390,3 +390,32 @@ def test_later_layers_repeat_the_recorded_launches_of_an_equal_layer(dtype):
         for step in range(5):
             err, bound = tiny.close(rep[1 + step][i].cpu().numpy(), ref[lens[i] + step], dtype)
             assert err <= bound, (i, step, err, bound)
+
+
+def test_captured_32_bit_steps_are_the_launched_ones():
+    """Single-token steps of a small 32-bit model replay a graph from the third step of a shape on: bit for bit what the
+    launches give, across a page's edge, as the batch shrinks, and for a shape that comes back."""
+    import gopherllm_b200 as gl
+    cfg = tiny.TINY["A"][0]
+    V, rng = cfg["vocab_size"], np.random.default_rng(31)
+    seqs = [tiny.prompt(rng, n, V) for n in (75, 20, 31)]
+    lens = [58, 3, 14]
+
+    def run(graphs):
+        m = gl.load(tiny.folder("A"), dtype="float32", max_tokens=3 * 128)
+        assert m.engine.use_graphs
+        m.engine.use_graphs = graphs
+        slots = [m.open_sequence() for _ in seqs]
+        outs = [m.step([(slots[i], seqs[i][:lens[i]]) for i in range(3)])]
+        for step in range(17):
+            live = range(3) if step < 8 or step > 12 else range(2)
+            outs.append(m.step([(slots[i], [seqs[i][min(lens[i] + step, len(seqs[i]) - 1)]]) for i in live]))
+        captured = sum(1 for g in m.engine._graphs.values() if g)
+        m.engine.check_device()
+        m.close()
+        return outs, captured
+
+    (own, none), (rep, captured) = run(False), run(True)
+    assert none == 0 and captured == 2
+    for a, b in zip(own, rep):
+        assert torch.equal(a, b)
