@@ -73,7 +73,7 @@ __device__ __forceinline__ float am_shape(float dot, const MixedAttnArgs& a, flo
 template <typename TA, typename TC, int NACC>
 __global__ void __launch_bounds__(AM_ROWS * 32)
 attn_pairs_kernel(MixedAttnArgs a, int stage_rows) {
-    extern __shared__ float smem[];
+    extern __shared__ __align__(16) float smem[];
     gl_grid_wait();
     const int hd = a.hd, vd = a.vd, ks = hd + 1;
     float* Ks = smem;                       // [stage_rows][hd+1]
@@ -178,7 +178,7 @@ attn_pairs_kernel(MixedAttnArgs a, int stage_rows) {
 template <typename TA, typename TC, int NACC>
 __global__ void __launch_bounds__(AM_DWARPS * 32)
 attn_pairs_decode_kernel(MixedAttnArgs a) {
-    extern __shared__ float smem[];
+    extern __shared__ __align__(16) float smem[];
     gl_grid_launch_dependents();
     gl_grid_wait();
     const int hd = a.hd, vd = a.vd;
@@ -279,15 +279,15 @@ attn_pairs_decode_kernel(MixedAttnArgs a) {
 __device__ __forceinline__ float am_dot(const float* q, const __nv_bfloat16* k, int hd) {
     float acc = 0.f;
     if ((hd & 7) == 0) {
-        for (int d = 0; d < hd; d += 8) {
+#pragma unroll 8
+        for (int d = 0; d < hd; d += 8) {               // (q lies in shared memory on a 16-byte boundary)
             const uint4 raw = *(const uint4*)(k + d);
+            const float4 qa = *(const float4*)(q + d), qb = *(const float4*)(q + d + 4);
             const __nv_bfloat162* p2 = (const __nv_bfloat162*)&raw;
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const float2 f = __bfloat1622float2(p2[e]);
-                acc = fmaf(q[d + 2 * e], f.x, acc);
-                acc = fmaf(q[d + 2 * e + 1], f.y, acc);
-            }
+            const float2 f0 = __bfloat1622float2(p2[0]), f1 = __bfloat1622float2(p2[1]);
+            const float2 f2 = __bfloat1622float2(p2[2]), f3 = __bfloat1622float2(p2[3]);
+            acc = fmaf(qa.x, f0.x, acc); acc = fmaf(qa.y, f0.y, acc); acc = fmaf(qa.z, f1.x, acc); acc = fmaf(qa.w, f1.y, acc);
+            acc = fmaf(qb.x, f2.x, acc); acc = fmaf(qb.y, f2.y, acc); acc = fmaf(qb.z, f3.x, acc); acc = fmaf(qb.w, f3.y, acc);
         }
     } else {
         for (int d = 0; d < hd; ++d) acc = fmaf(q[d], __bfloat162float(k[d]), acc);
@@ -300,10 +300,14 @@ __device__ __forceinline__ float am_dot(const float* q, const float* k, int hd) 
     return acc;
 }
 
-template <typename TA, typename TC, int NACC, int GQ>
+// VEC: values in bfloat16 whose rows are 8, 16, .. 256 numbers: a lane takes eight columns of a row and the warp as many
+// rows at a time as fit it, so that a page's values are 16-byte loads asked for together; the lanes' sums over their
+// rows meet at the end.  (One column a lane and 16 keys at a time, a page cost four trips to memory and 64 x 2 loads of
+// two bytes a lane: 4 sequences of 64 to 1,000 positions, 32 heads of 64 on 8 key heads with a table, 65 us, now 31.)
+template <typename TA, typename TC, int NACC, int GQ, bool VEC>
 __global__ void __launch_bounds__(AM_GTHREADS)
 attn_group_decode_kernel(MixedAttnArgs a) {
-    extern __shared__ float smem[];
+    extern __shared__ __align__(16) float smem[];
     gl_grid_launch_dependents();
     gl_grid_wait();
     const int hd = a.hd, vd = a.vd;
@@ -332,11 +336,14 @@ attn_group_decode_kernel(MixedAttnArgs a) {
     const int runs = a.mix ? 1 : gq / per;              // value heads of this block
     const int vh = a.mix ? warp : head0 / share + warp;
     const bool has_values = a.mix ? warp < a.nKV : warp < runs;
-    float acc[GQ][NACC];
+    constexpr int NA = VEC ? 8 : NACC;
+    float acc[GQ][NA];
 #pragma unroll
     for (int g = 0; g < GQ; ++g)
 #pragma unroll
-        for (int i = 0; i < NACC; ++i) acc[g][i] = 0.f;
+        for (int i = 0; i < NA; ++i) acc[g][i] = 0.f;
+    const int per_row = VEC ? vd / 8 : 32, at_once = 32 / per_row;      // VEC: lanes a row, rows at a time
+    const int my_key = lane / per_row, my_col = (lane - my_key * per_row) * 8;
     float m = -INFINITY, l = 0.f;                       // warp g < gq keeps head g's running maximum and sum
     const int* pg = a.pages + (size_t)b * a.max_pages;
     for (int page_i = page_first; page_i <= page_last; ++page_i) {
@@ -372,10 +379,42 @@ attn_group_decode_kernel(MixedAttnArgs a) {
                 if (g < gq) {
                     const float c = corr[g];
 #pragma unroll
-                    for (int i = 0; i < NACC; ++i) acc[g][i] *= c;
+                    for (int i = 0; i < NA; ++i) acc[g][i] *= c;
                 }
             }
             const int kmin = max(0, lo - j0), kmax = min(GL_PAGE, p - j0 + 1);   // written keys inside the window
+            if constexpr (VEC) {
+                constexpr int KB = 8;
+                for (int k0 = 0; k0 < GL_PAGE; k0 += KB * at_once) {
+                    if (k0 + KB * at_once <= kmin || k0 >= kmax) continue;
+                    uint4 v[KB];
+#pragma unroll
+                    for (int kk = 0; kk < KB; ++kk) {
+                        const int k = k0 + kk * at_once + my_key;
+                        v[kk] = k >= kmin && k < kmax ? *(const uint4*)(vp + (size_t)k * vs + my_col) : make_uint4(0, 0, 0, 0);
+                    }
+#pragma unroll
+                    for (int kk = 0; kk < KB; ++kk) {
+                        const int k = k0 + kk * at_once + my_key;
+                        const __nv_bfloat162* p2 = (const __nv_bfloat162*)&v[kk];
+                        float f[8];
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            const float2 t2 = __bfloat1622float2(p2[e]);
+                            f[2 * e] = t2.x;
+                            f[2 * e + 1] = t2.y;
+                        }
+#pragma unroll
+                        for (int g = 0; g < GQ; ++g) {
+                            if (g < gq && (a.mix || g / per == warp)) {
+                                const float pk = k < GL_PAGE ? sc[g * GL_PAGE + k] : 0.f;
+#pragma unroll
+                                for (int e = 0; e < 8; ++e) acc[g][e] = fmaf(pk, f[e], acc[g][e]);
+                            }
+                        }
+                    }
+                }
+            } else {
             // sixteen keys' values are asked for before the first is used: one after the other, every key
             // would cost a trip to memory
             constexpr int KB = NACC <= 2 ? 16 : 8;
@@ -403,6 +442,7 @@ attn_group_decode_kernel(MixedAttnArgs a) {
                     }
                 }
             }
+            }
         }
     }
     // the range's sums as they are, with its maximum and sum: the mixing kernel puts the ranges together
@@ -416,10 +456,20 @@ attn_group_decode_kernel(MixedAttnArgs a) {
         for (int g = 0; g < GQ; ++g) {
             if (g < gq && (a.mix || g / per == warp)) {
                 float* o = a.parts + ((((size_t)b * a.nH + (size_t)head0 + g) * nVal + (a.mix ? vh : 0)) * a.splits + split) * vd;
+                if constexpr (VEC) {
 #pragma unroll
-                for (int i = 0; i < NACC; ++i) {
-                    const int d = lane + 32 * i;
-                    if (d < vd) o[d] = acc[g][i];
+                    for (int e = 0; e < 8; ++e)
+                        for (int w = per_row; w < 32; w <<= 1) acc[g][e] += __shfl_xor_sync(0xffffffffu, acc[g][e], w);
+                    if (my_key == 0) {
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) o[my_col + e] = acc[g][e];
+                    }
+                } else {
+#pragma unroll
+                    for (int i = 0; i < NACC; ++i) {
+                        const int d = lane + 32 * i;
+                        if (d < vd) o[d] = acc[g][i];
+                    }
                 }
             }
         }
@@ -459,7 +509,7 @@ struct MergeProjectArgs {
 
 __global__ void __launch_bounds__(AP_THREADS)
 merge_project_kernel(MergeProjectArgs a) {
-    extern __shared__ float smem[];
+    extern __shared__ __align__(16) float smem[];
     float* coef = smem;                                 // [AP_TOKENS][64]
     float* y = coef + AP_TOKENS * 64;                   // [AP_TOKENS][R]
     gl_grid_launch_dependents();
@@ -545,10 +595,11 @@ GL_API int gl_merge_project(const MergeProjectArgs* args, cudaStream_t stream) {
 }
 
 // out[b, h, :] = sum_g M[h, g] * (sum_s parts[b, g, c(h), s, :] e^(m_gs - m_g)) / (sum_s l_gs e^(m_gs - m_g))
+#define AM_MIX_THREADS 512
 template <typename TA>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(AM_MIX_THREADS)
 head_mix_split_kernel(MixedAttnArgs a) {
-    extern __shared__ float coef[];                     // [heads taken][splits]: M[h, g] e^(m_gs - m_g) / sum_g
+    extern __shared__ __align__(16) float coef[];       // [heads taken][splits]: M[h, g] e^(m_gs - m_g) / sum_g
     gl_grid_launch_dependents();
     gl_grid_wait();
     const int b = blockIdx.y, h = blockIdx.x;
@@ -561,6 +612,45 @@ head_mix_split_kernel(MixedAttnArgs a) {
             float y = 0.f;
 #pragma unroll 8
             for (int s = 0; s < a.splits; ++s) y = fmaf(coef[s], src[(size_t)s * a.vd + d], y);
+            gl_store((TA*)a.out + (row * a.nH + h) * a.vd + d, y);
+        }
+        return;
+    }
+    if (blockDim.x == AM_MIX_THREADS) {
+        // With a table a result is a sum over every head's ranges: the heads' factors by a warp each, then the sum cut over
+        // groups of threads, a thread four columns of a group's heads, and the groups' parts added in order.  (One thread a
+        // column walked all heads x ranges: 32 heads x 16 ranges x 64 columns, 4 sequences, took 65 us, now 9.9.)
+        const int warp = threadIdx.x >> 5, warps = blockDim.x >> 5, lane = threadIdx.x & 31, S = a.splits;
+        for (int g = warp; g < a.nH; g += warps) {
+            am_range_factors(a.ml + ((size_t)b * a.nH + g) * S * 2, S, a.sinks, g, coef + g * S);
+            const float w = a.mix[h * a.nH + g];
+            if (lane < S) coef[g * S + lane] *= w;
+            if (lane + 32 < S) coef[g * S + lane + 32] *= w;
+        }
+        __syncthreads();
+        const int cols = a.vd / 4, groups = blockDim.x / cols, grp = threadIdx.x / cols, d4 = threadIdx.x - grp * cols;
+        float4* sums = (float4*)(coef + ((a.nH * S + 3) & ~3));                  // [groups][cols]
+        if (grp < groups) {
+            const int ga = grp * a.nH / groups, gb = (grp + 1) * a.nH / groups, c = h / (a.nH / a.nKV);
+            float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int g = ga; g < gb; ++g) {
+                const float4* src = (const float4*)(a.parts + (((size_t)b * a.nH + g) * a.nKV + c) * S * a.vd) + d4;
+                const float* f = coef + g * S;
+#pragma unroll 8
+                for (int s = 0; s < S; ++s) {
+                    const float4 p = src[(size_t)s * cols];
+                    y.x = fmaf(f[s], p.x, y.x); y.y = fmaf(f[s], p.y, y.y);
+                    y.z = fmaf(f[s], p.z, y.z); y.w = fmaf(f[s], p.w, y.w);
+                }
+            }
+            sums[grp * cols + d4] = y;
+        }
+        __syncthreads();
+        const float* flat = (const float*)sums;
+        const size_t row = (size_t)a.seq_qstart[b];
+        for (int d = threadIdx.x; d < a.vd; d += blockDim.x) {
+            float y = 0.f;
+            for (int i = 0; i < groups; ++i) y += flat[i * a.vd + d];
             gl_store((TA*)a.out + (row * a.nH + h) * a.vd + d, y);
         }
         return;
@@ -596,18 +686,75 @@ head_mix_split_kernel(MixedAttnArgs a) {
     }
 }
 
-template <typename TA, typename TC, int NACC>
-static int launch_group_decode(const MixedAttnArgs& a, cudaStream_t stream) {
+// Blocks of AM_MIX_THREADS where there is a table and the values' rows are whole 16-byte pieces (the kernel tells by the block).
+template <typename TA>
+static int launch_head_mix_split(const MixedAttnArgs& a, cudaStream_t stream) {
+    const size_t factors = (((size_t)(a.mix ? a.nH : 1) * a.splits + 3) & ~(size_t)3) * sizeof(float);
+    const size_t with_sums = factors + AM_MIX_THREADS * sizeof(float4);
+    const bool wide = a.mix && a.splits <= 64 && a.vd % 4 == 0 && a.vd <= 4 * AM_MIX_THREADS && with_sums <= 48 * 1024;
+    return gl_launch(head_mix_split_kernel<TA>, dim3(a.nH, a.B), dim3(wide ? AM_MIX_THREADS : a.vd <= 64 ? 64 : 128),
+                     wide ? with_sums : factors, stream, 1, a);
+}
+
+template <typename TA, typename TC, int NACC, bool VEC>
+static int launch_group_decode_as(const MixedAttnArgs& a, cudaStream_t stream) {
     const int group = a.nH / a.nKV, gq = group < 8 ? group : 8;
     const size_t smem = ((size_t)gq * a.hd + (size_t)gq * GL_PAGE + gq) * sizeof(float);
     const dim3 grid(a.nKV * (group / gq), a.B, a.splits);
-    if (gq <= 1) return gl_launch(attn_group_decode_kernel<TA, TC, NACC, 1>, grid, dim3(AM_GTHREADS), smem, stream, 1, a);
-    if (gq <= 2) return gl_launch(attn_group_decode_kernel<TA, TC, NACC, 2>, grid, dim3(AM_GTHREADS), smem, stream, 1, a);
-    if (gq <= 4) return gl_launch(attn_group_decode_kernel<TA, TC, NACC, 4>, grid, dim3(AM_GTHREADS), smem, stream, 1, a);
-    return gl_launch(attn_group_decode_kernel<TA, TC, NACC, 8>, grid, dim3(AM_GTHREADS), smem, stream, 1, a);
+    if (gq <= 1) return gl_launch(attn_group_decode_kernel<TA, TC, NACC, 1, VEC>, grid, dim3(AM_GTHREADS), smem, stream, 1, a);
+    if (gq <= 2) return gl_launch(attn_group_decode_kernel<TA, TC, NACC, 2, VEC>, grid, dim3(AM_GTHREADS), smem, stream, 1, a);
+    if (gq <= 4) return gl_launch(attn_group_decode_kernel<TA, TC, NACC, 4, VEC>, grid, dim3(AM_GTHREADS), smem, stream, 1, a);
+    return gl_launch(attn_group_decode_kernel<TA, TC, NACC, 8, VEC>, grid, dim3(AM_GTHREADS), smem, stream, 1, a);
+}
+
+template <typename TA, typename TC, int NACC>
+static int launch_group_decode(const MixedAttnArgs& a, cudaStream_t stream) {
+    if constexpr (sizeof(TC) == 2) {
+        if (a.vd >= 8 && a.vd <= 256 && (a.vd & (a.vd - 1)) == 0 && am_value_stride(a) % 8 == 0 && ((uintptr_t)a.v_cache & 15) == 0)
+            return launch_group_decode_as<TA, TC, 1, true>(a, stream);
+    }
+    return launch_group_decode_as<TA, TC, NACC, false>(a, stream);
 }
 
 // out[t, h, :] = sum_g M[h, g] pairs[t, g, c(h), :]   (without a table: pairs[t, h, 0, :])
+// Where the pairs' rows are whole 16-byte pieces and a value head's query heads are at most AM_MIX_HEADS, a thread takes four
+// columns of one value head for all of them: every pair is read once and not once per query head (2,128 tokens, 32 heads on
+// 8 value heads of 64: 154 us, now 36).
+#define AM_MIX_HEADS 8
+template <typename TA, int GROUP>
+__global__ void __launch_bounds__(256)
+head_mix_group_kernel(MixedAttnArgs a) {
+    gl_grid_launch_dependents();
+    gl_grid_wait();
+    const int cols = a.vd / 4, group = a.nH / a.nKV;
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= (long long)a.T * a.nKV * cols) return;
+    const int d4 = (int)(i % cols), c = (int)((i / cols) % a.nKV);
+    const long long t = i / ((long long)cols * a.nKV);
+    float4 y[GROUP];
+#pragma unroll
+    for (int k = 0; k < GROUP; ++k) y[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4* src = (const float4*)a.pairs + ((size_t)t * a.nH * a.nKV + c) * cols + d4;
+    const float* mix = a.mix + (size_t)c * group * a.nH;
+#pragma unroll 4
+    for (int g = 0; g < a.nH; ++g) {
+        const float4 p = src[(size_t)g * a.nKV * cols];
+#pragma unroll
+        for (int k = 0; k < GROUP; ++k)
+            if (k < group) {
+                const float w = mix[k * a.nH + g];
+                y[k].x = fmaf(w, p.x, y[k].x); y[k].y = fmaf(w, p.y, y[k].y);
+                y[k].z = fmaf(w, p.z, y[k].z); y[k].w = fmaf(w, p.w, y[k].w);
+            }
+    }
+#pragma unroll
+    for (int k = 0; k < GROUP; ++k)
+        if (k < group) {
+            TA* o = (TA*)a.out + ((size_t)t * a.nH + c * group + k) * a.vd + 4 * d4;
+            gl_store(o, y[k].x); gl_store(o + 1, y[k].y); gl_store(o + 2, y[k].z); gl_store(o + 3, y[k].w);
+        }
+}
+
 template <typename TA>
 __global__ void __launch_bounds__(256)
 head_mix_kernel(MixedAttnArgs a) {
@@ -631,6 +778,20 @@ head_mix_kernel(MixedAttnArgs a) {
     gl_store((TA*)a.out + i, y);
 }
 
+template <typename TA>
+static int launch_head_mix(const MixedAttnArgs& a, cudaStream_t stream) {
+    const int group = a.nH / a.nKV;
+    if (a.mix && group <= AM_MIX_HEADS && a.vd % 4 == 0 && ((uintptr_t)a.pairs & 15) == 0) {
+        const long long n = (long long)a.T * a.nKV * (a.vd / 4);
+        const dim3 grid((unsigned)((n + 255) / 256));
+        if (group <= 2) return gl_launch(head_mix_group_kernel<TA, 2>, grid, dim3(256), 0, stream, 1, a);
+        if (group <= 4) return gl_launch(head_mix_group_kernel<TA, 4>, grid, dim3(256), 0, stream, 1, a);
+        return gl_launch(head_mix_group_kernel<TA, AM_MIX_HEADS>, grid, dim3(256), 0, stream, 1, a);
+    }
+    const long long n = (long long)a.T * a.nH * a.vd;
+    return gl_launch(head_mix_kernel<TA>, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, stream, 1, a);
+}
+
 template <typename TA, typename TC, int NACC>
 static int launch_mixed(const MixedAttnArgs& a, cudaStream_t stream) {
     const int pairs = a.nH * (a.mix ? a.nKV : 1);
@@ -644,7 +805,7 @@ static int launch_mixed(const MixedAttnArgs& a, cudaStream_t stream) {
     if (a.max_qlen == 1 && by_key_head && NACC <= 4 && a.parts && a.ml && a.splits > 0) {
         rc = launch_group_decode<TA, TC, NACC>(a, stream);
         if (rc != 0) return rc;
-        return gl_launch(head_mix_split_kernel<TA>, dim3(a.nH, a.B), dim3(a.vd <= 64 ? 64 : 128), (size_t)(a.mix ? a.nH : 1) * a.splits * sizeof(float), stream, 1, a);
+        return launch_head_mix_split<TA>(a, stream);
     } else if (a.max_qlen == 1) {
         const size_t smem = ((size_t)a.hd + (size_t)AM_DWARPS * (a.vd + 2)) * sizeof(float);
         rc = gl_launch(attn_pairs_decode_kernel<TA, TC, NACC>, dim3(pairs, a.B), dim3(AM_DWARPS * 32), smem, stream, 1, a);
@@ -665,8 +826,7 @@ static int launch_mixed(const MixedAttnArgs& a, cudaStream_t stream) {
         rc = gl_launch(kern, dim3((a.max_qlen + AM_ROWS - 1) / AM_ROWS, pairs, a.B), dim3(AM_ROWS * 32), smem, stream, 1, a, stage_rows);
     }
     if (rc != 0) return rc;
-    const long long n = (long long)a.T * a.nH * a.vd;
-    return gl_launch(head_mix_kernel<TA>, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, stream, 1, a);
+    return launch_head_mix<TA>(a, stream);
 }
 
 // the kernel that puts a one-token step's ranges together, behind a kernel of another library that left them
@@ -674,11 +834,9 @@ GL_API int gl_head_mix_split(const MixedAttnArgs* args, int act_dtype, cudaStrea
     const MixedAttnArgs& a = *args;
     if (a.B <= 0) return GL_OK;
     if (!a.parts || !a.ml || a.splits <= 0 || a.vd <= 0) return GL_ERR_SHAPE;
-    const dim3 grid(a.nH, a.B), block(a.vd <= 64 ? 64 : 128);
-    const size_t smem = (size_t)(a.mix ? a.nH : 1) * a.splits * sizeof(float);
     int rc;
-    if (act_dtype == GL_F32) rc = gl_launch(head_mix_split_kernel<float>, grid, block, smem, stream, 1, a);
-    else if (act_dtype == GL_BF16) rc = gl_launch(head_mix_split_kernel<__nv_bfloat16>, grid, block, smem, stream, 1, a);
+    if (act_dtype == GL_F32) rc = launch_head_mix_split<float>(a, stream);
+    else if (act_dtype == GL_BF16) rc = launch_head_mix_split<__nv_bfloat16>(a, stream);
     else return GL_ERR_DTYPE;
     return rc == 0 ? GL_OK : GL_ERR_LAUNCH;
 }
@@ -687,10 +845,8 @@ GL_API int gl_head_mix_split(const MixedAttnArgs* args, int act_dtype, cudaStrea
 GL_API int gl_head_mix(const MixedAttnArgs* args, int act_dtype, cudaStream_t stream) {
     const MixedAttnArgs& a = *args;
     if (a.T <= 0) return GL_OK;
-    const long long n = (long long)a.T * a.nH * a.vd;
-    const dim3 grid((unsigned)((n + 255) / 256));
-    if (act_dtype == GL_F32) return gl_launch(head_mix_kernel<float>, grid, dim3(256), 0, stream, 1, a) == 0 ? GL_OK : GL_ERR_LAUNCH;
-    if (act_dtype == GL_BF16) return gl_launch(head_mix_kernel<__nv_bfloat16>, grid, dim3(256), 0, stream, 1, a) == 0 ? GL_OK : GL_ERR_LAUNCH;
+    if (act_dtype == GL_F32) return launch_head_mix<float>(a, stream) == 0 ? GL_OK : GL_ERR_LAUNCH;
+    if (act_dtype == GL_BF16) return launch_head_mix<__nv_bfloat16>(a, stream) == 0 ? GL_OK : GL_ERR_LAUNCH;
     return GL_ERR_DTYPE;
 }
 

@@ -792,3 +792,29 @@ def test_neighbouring_dims_turned_piece_by_piece(half):
             at += n
         written = sum(qlens)
         assert int((k[..., 0] != 7.0).sum()) <= written * G and int((v.float() != 7.0).any(-1).sum()) <= written * G
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("heads,groups,dim,vdim", [(8, 2, 64, 64), (4, 4, 16, 16), (8, 8, 64, 32), (16, 2, 32, 32), (8, 2, 16, 128),
+                                                   (3, 3, 24, 8), (6, 3, 24, 40), (4, 2, 16, 30)])
+def test_attention_with_a_table_over_the_heads(heads, groups, dim, vdim, dtype):
+    """A result is a sum over all heads' weights applied to the own value head: one token a sequence with contexts cut into
+    ranges (some of them empty), and prompts, with values of whole 16-byte pieces, of a power of two of them, and neither."""
+    from gopherllm_b200 import ops
+    g = torch.Generator().manual_seed(heads + vdim)
+    mix = torch.eye(heads) + 0.3 * torch.randn(heads, heads, generator=g)
+    tol = 3e-2 * 2 if dtype == torch.bfloat16 else 1e-4        # (about two heads' worth of weight in a sum)
+    for qlens, ctxs in (([1] * 6, [0, 1, 63, 64, 200, 700]), ([40, 2, 70], [70, 190, 0])):
+        if max(qlens) > 1 and vdim == 128:
+            continue
+        k, v, pages, ctx, keys, vals = _paged(qlens, ctxs, groups, dim, vdim, g)
+        q = torch.randn(sum(qlens), heads * dim, generator=g).to(torch.bfloat16)
+        for kw, lo in (({}, lambda p: 0), (dict(window=70), lambda p: max(0, p - 69))):
+            got = ops.attention_mixed(q.to(DEV).to(dtype), k.to(dtype), v.to(dtype), ctx, pages, heads, groups, dim, vdim, mix=mix.to(DEV),
+                                      score_scale=0.2, **kw).cpu().double()
+            want = torch.empty(sum(qlens), heads, vdim, dtype=torch.float64)
+            for c in range(groups):
+                y = _attend(q.view(-1, heads, dim), keys, [x[:, c:c + 1].expand(-1, groups, -1) for x in vals], qlens, ctxs, 0.2, lo)
+                own = slice(c * (heads // groups), (c + 1) * (heads // groups))
+                want[:, own] = torch.einsum("hg,tgv->thv", mix.double()[own], y.view(-1, heads, vdim))
+            assert (got - want.reshape(sum(qlens), -1)).abs().max() < tol, (kw, qlens, float((got - want.reshape(sum(qlens), -1)).abs().max()))
