@@ -9,6 +9,13 @@
 // two passes, this one rescales on the fly, which differs by rounding only).
 // A query at position p sees keys lo..p, lo = 0 or p-window+1
 // (model.go:2707-2710); nothing else masks.
+//
+// A sequence that brings one token has one query row for a block of eight warps: there the
+// warps share the row's pages (page i with warp i mod 8, straight from the cache, no tiles),
+// and their softmaxes are merged in the warps' order.  What bounds such a row is the chain of
+// trips to memory, a page after the other: 4 sequences of 16 to 300 positions, 32 heads of 64,
+// took 57 us a launch with one warp walking all pages, now 28.  The form depends on the
+// sequence's own run alone, so a row still does not depend on the batch around it.
 #include "common.cuh"
 
 struct AttnArgs {
@@ -26,6 +33,27 @@ struct AttnArgs {
 };
 
 #define AG_ROWS 8
+
+// q . k with k in ascending order; rows of whole 16-byte pieces are read as such
+__device__ __forceinline__ float ag_dot(const float* q, const float* k, int hd) {
+    float s = 0.f;
+    if ((hd & 3) == 0 && ((uintptr_t)k & 15) == 0) {
+#pragma unroll 8
+        for (int d = 0; d < hd; d += 4) {
+            const float4 v = *(const float4*)(k + d);
+            s = fmaf(q[d], v.x, s); s = fmaf(q[d + 1], v.y, s); s = fmaf(q[d + 2], v.z, s); s = fmaf(q[d + 3], v.w, s);
+        }
+    } else {
+        for (int d = 0; d < hd; ++d) s = fmaf(q[d], k[d], s);
+    }
+    return s;
+}
+__device__ __forceinline__ float ag_dot(const float* q, const __nv_bfloat16* k, int hd) {
+    float s = 0.f;
+#pragma unroll 8
+    for (int d = 0; d < hd; ++d) s = fmaf(q[d], gl_load(k + d), s);
+    return s;
+}
 
 template <typename TA, typename TC, int NACC>
 __global__ void __launch_bounds__(AG_ROWS * 32)
@@ -62,6 +90,68 @@ attn_generic_kernel(AttnArgs a) {
     float m = -INFINITY, l = 0.f;
 
     const int* pg = a.pages + (size_t)b * a.max_pages;
+    if (qlen == 1) {
+        // (the block's row 0: p_first is its position and lo_cta its first key)
+        __syncthreads();
+        const float* q0 = Qs;
+        for (int page_i = lo_cta / GL_PAGE + warp; page_i <= p_first / GL_PAGE; page_i += AG_ROWS) {
+            const int page = gl_checked(pg[gl_checked(page_i, a.max_pages, GL_BAD_POSITION)], a.n_pages > 0 ? a.n_pages : 0x7fffffff, GL_BAD_PAGE);
+            const TC* kp = (const TC*)a.k_cache + ((size_t)page * a.nKV + g) * GL_PAGE * hd;
+            const TC* vp = (const TC*)a.v_cache + ((size_t)page * a.nKV + g) * GL_PAGE * hd;
+#pragma unroll 1
+            for (int half = 0; half < GL_PAGE / 32; ++half) {
+                const int j0 = page_i * GL_PAGE + half * 32, j = j0 + lane;
+                const bool ok = j >= lo_cta && j <= p_first;
+                const float s = ok ? ag_dot(q0, kp + (size_t)(half * 32 + lane) * hd, hd) : -INFINITY;
+                const float m_new = fmaxf(m, gl_warp_max(s));
+                if (m_new == -INFINITY) continue;
+                const float pj = ok ? expf(s - m_new) : 0.f;
+                const float corr = expf(m - m_new);            // m = -inf gives 0
+                l = l * corr + gl_warp_sum(pj);
+                m = m_new;
+#pragma unroll
+                for (int i = 0; i < NACC; ++i) acc[i] *= corr;
+                const TC* vr = vp + (size_t)half * 32 * hd;
+                // rows outside [lo, p] were never written or given back: they are not read
+                const int k0 = max(0, lo_cta - j0), k1 = min(32, p_first - j0 + 1);
+#pragma unroll 8
+                for (int k = 0; k < 32; ++k) {
+                    const float pk = __shfl_sync(0xffffffffu, pj, k);
+#pragma unroll
+                    for (int i = 0; i < NACC; ++i) {
+                        const int d = lane + 32 * i;
+                        if (d < hd && k >= k0 && k < k1) acc[i] = fmaf(pk, gl_load(vr + (size_t)k * hd + d), acc[i]);
+                    }
+                }
+            }
+        }
+        float* part = Ks;                                      // [AG_ROWS][hd + 2]: a warp's sums, its maximum and its weight
+        float* mine = part + warp * (hd + 2);
+#pragma unroll
+        for (int i = 0; i < NACC; ++i)
+            if (lane + 32 * i < hd) mine[lane + 32 * i] = acc[i];
+        if (lane == 0) { mine[hd] = m; mine[hd + 1] = l; }
+        __syncthreads();
+        float top = -INFINITY;
+#pragma unroll
+        for (int w = 0; w < AG_ROWS; ++w) top = fmaxf(top, part[w * (hd + 2) + hd]);
+        float f[AG_ROWS], den = 0.f;
+#pragma unroll
+        for (int w = 0; w < AG_ROWS; ++w) {
+            const float mw = part[w * (hd + 2) + hd];
+            f[w] = mw > -INFINITY ? expf(mw - top) : 0.f;
+            den = fmaf(f[w], part[w * (hd + 2) + hd + 1], den);
+        }
+        const float inv = den > 0.f ? 1.0f / den : 0.f;
+        TA* o = (TA*)a.out + ((size_t)a.seq_qstart[b] * a.nH + h) * hd;
+        for (int d = threadIdx.x; d < hd; d += AG_ROWS * 32) {
+            float y = 0.f;
+#pragma unroll
+            for (int w = 0; w < AG_ROWS; ++w) y = fmaf(f[w], part[w * (hd + 2) + d], y);
+            gl_store(o + d, y * inv);
+        }
+        return;
+    }
     for (int page_i = lo_cta / GL_PAGE; page_i <= p_last / GL_PAGE; ++page_i) {
         const int page = gl_checked(pg[gl_checked(page_i, a.max_pages, GL_BAD_POSITION)], a.n_pages > 0 ? a.n_pages : 0x7fffffff, GL_BAD_PAGE);
         const TC* kp = (const TC*)a.k_cache + ((size_t)page * a.nKV + g) * GL_PAGE * hd;

@@ -437,6 +437,16 @@ def test_attention_generic(dtype, nH, nKV, hd, window):
     run_attention("generic", dtype, nH, nKV, hd, window, [0, 130, 63, 5], [70, 1, 66, 9])
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("nH,nKV,hd", [(4, 2, 64), (2, 2, 33), (3, 1, 256)])
+@pytest.mark.parametrize("window", [0, 100])
+def test_attention_generic_one_token(dtype, nH, nKV, hd, window):
+    """Sequences of one token, whose pages the warps of a block share: fewer pages than warps, more, page edges, and
+    beside a sequence of several tokens."""
+    run_attention("generic", dtype, nH, nKV, hd, window, [0, 63, 64, 511, 512, 1100], [1] * 6)
+    run_attention("generic", dtype, nH, nKV, hd, window, [200, 30, 64], [1, 5, 1])
+
+
 def run_attention(kernel, dtype, nH, nKV, hd, window, ctxs, qlens):
     o = ops()
     B, L = len(ctxs), max(c + q for c, q in zip(ctxs, qlens))
