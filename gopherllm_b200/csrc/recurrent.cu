@@ -1,7 +1,7 @@
 // Mixers that carry a fixed-size state from token to token instead of a growing cache:
 // matrix memories with outer-product updates (an exponentially gated one with a normaliser and a
-// running maximum, and one whose per-channel forget gate also sets what is written) and a
-// selective state-space scan behind a short causal convolution.
+// running maximum, and one whose per-channel forget gate also sets what is written) and the short
+// causal convolution (the selective state-space scan behind it is in selective_scan.cu).
 //
 // A step brings, for every sequence of the batch, a run of one or more tokens; the state of a
 // sequence lives in its row of a 32-bit table (row = the sequence's slot), is read when the run
@@ -14,35 +14,9 @@
 // state in registers for the whole run, and the tokens' inputs are staged in shared memory a few
 // tokens at a time.
 #include "common.cuh"
+#include "recurrent_common.cuh"
 
-#define RC_THREADS 128
 #define MS_THREADS 256     // the matrix memories' blocks
-#define SS_CHUNK 16         // tokens the selective scan stages at a time
-
-__device__ __forceinline__ float rc_sigmoid(float x) { return 1.0f / (1.0f + expf(-x)); }
-__device__ __forceinline__ float rc_silu(float x) { return x / (1.0f + expf(-x)); }
-__device__ __forceinline__ float rc_log_sigmoid(float x) { return fminf(x, 0.0f) - log1pf(expf(-fabsf(x))); }
-__device__ __forceinline__ float rc_softplus(float x) { return x > 20.0f ? x : log1pf(expf(x)); }
-// e^x for a decay that is applied at every token: near one the factor comes from expm1f, which is
-// rounded once; expf's last-bit errors near one do not average out over a thousand tokens of a slowly
-// decaying state.
-__device__ __forceinline__ float rc_decay(float x) {
-    if (x > -0.5f && x <= 0.f) {
-        // 1 + (e^x - 1) with e^x - 1 from its series to x^9/9! (below 2^-28 here), Horner in 32-bit
-        float p = 2.755731922e-6f;
-        p = fmaf(p, x, 2.48015873e-5f);
-        p = fmaf(p, x, 1.984126984e-4f);
-        p = fmaf(p, x, 1.388888889e-3f);
-        p = fmaf(p, x, 8.333333333e-3f);
-        p = fmaf(p, x, 4.166666667e-2f);
-        p = fmaf(p, x, 1.666666667e-1f);
-        p = fmaf(p, x, 0.5f);
-        p = fmaf(p, x, 1.0f);
-        return fmaf(p, x, 1.0f);
-    }
-    if (x > -0.5f) return 1.0f + expm1f(x);
-    return expf(x);
-}
 
 // ---------------------------------------------------------------------------
 // Matrix memories.  Per head a state S [D, V]; a token's output is S^T q.
@@ -93,8 +67,13 @@ struct MemoryScanArgs {
 
 // FULL: D == R * DPT and D a multiple of 4, so a thread's rows are DPT / 4 groups of four consecutive ones read
 // as float4 and no row needs a bounds check.
+// Blocks an SM, stated: left to itself the compiler gave eight rows a thread 80 registers or 125 depending on what else the
+// file held, and with two blocks an SM instead of three one token of 16 sequences took 13 % longer.
+__host__ __device__ constexpr int ms_blocks(int dpt, int kind) {
+    return dpt >= 32 ? 1 : kind == 2 ? (dpt >= 4 ? 2 : 3) : dpt >= 8 ? 3 : 4;
+}
 template <typename TA, int DPT, int KIND, bool FULL>
-__global__ void __launch_bounds__(MS_THREADS)
+__global__ void __launch_bounds__(MS_THREADS, ms_blocks(DPT, KIND))
 memory_scan_kernel(MemoryScanArgs a, int R, int CH) {
     extern __shared__ __align__(16) float smem[];
     // (launched in order, not early: placed beside the kernel before, the blocks of a scan sat several to an SM
@@ -847,204 +826,6 @@ GL_API int gl_conv_silu(const ConvArgs* args, int act_dtype, cudaStream_t stream
         if (rc == 0 && a.taps > 1) rc = gl_launch(conv_tail_kernel<__nv_bfloat16>, g2, dim3(256), 0, stream, 1, a);
         return rc;
     }
-    return GL_ERR_DTYPE;
-}
-
-// ---------------------------------------------------------------------------
-// Selective scan.  Per channel c and state n:
-//   dt = softplus(dtp[t, c]);  S[c, n] <- e^(dt A[c, n]) S[c, n] + dt x[t, c] B[t, n],  A = -e^(A_log)
-//   y[t, c] = (sum_n S[c, n] C[t, n] + D[c] x[t, c]) * silu(z[t, c])
-// A channel's states are spread over G adjacent lanes, NPT states a lane (fewer states a lane and more lanes
-// when the grid would otherwise leave the SMs with a warp or two each: a thread walks the tokens in order).
-// ---------------------------------------------------------------------------
-struct SelectiveScanArgs {
-    const void* x;            // [T, C] activation type (the convolution's output)
-    const float* dtp;         // [T, C] 32-bit: the step size before softplus, bias included
-    const void* bc;           // [T, 2N] activation type: B then C
-    const void* z;            // activation type, row pitch z_ld, first column z_off
-    void* out;                // [T, C] activation type
-    const float* a_log;       // [C, N]
-    const float* d_skip;      // [C]
-    float* state;             // [slots, state_stride], S [C, N] first
-    const int* seq_slot;
-    const int* seq_qstart;
-    const int* seq_qlen;
-    int B, C, N, z_ld, z_off, state_stride;
-    // a long run cut into chunks of chunk_len tokens that are walked side by side (n_chunks > 1):
-    //   first every chunk from a zero state, keeping its last state and the sum of its step sizes;
-    //   then a carry over the chunks, S_start[k+1] = e^(A sum_k) S_start[k] + last_k (the decays of a chunk
-    //   multiply to e^(A sum of its step sizes));  then every chunk again from its true start, with outputs.
-    float* chunk_state;       // [B, n_chunks, C, N]
-    float* chunk_dt;          // [B, n_chunks, C]
-    int chunk_len, n_chunks;
-};
-
-// MODE 0: a run in one piece.  MODE 1: a chunk from a zero state, no outputs.  MODE 2: a chunk from its start.
-template <typename TA, int SS_NPT, int MODE>
-__global__ void __launch_bounds__(RC_THREADS)
-selective_scan_kernel(SelectiveScanArgs a, int G) {
-    extern __shared__ float smem[];
-    // (launched in order, not early: placed beside the kernel before, the blocks of a scan sat several to an SM
-    // for its whole length, and a prompt of 2,048 tokens took 25 ms instead of 16)
-    gl_grid_wait();
-    const int N = a.N, C = a.C;
-    const int CPB = RC_THREADS / G;
-    const int b = blockIdx.y, c0 = blockIdx.x * CPB;
-    const int g = threadIdx.x % G, cl = threadIdx.x / G;
-    const int c = c0 + cl;
-    const bool live = c < C;
-    const int qlen = a.seq_qlen[b], qstart = a.seq_qstart[b];
-    const int chunk = MODE == 0 ? 0 : blockIdx.z;
-    const int t_begin = MODE == 0 ? 0 : chunk * a.chunk_len;
-    const int t_end = MODE == 0 ? qlen : min(qlen, t_begin + a.chunk_len);
-    if (t_begin >= qlen) return;                      // (the whole block: this sequence has no such chunk)
-    float* Bs = smem;                                 // [CHUNK][N]
-    float* Cs = Bs + SS_CHUNK * N;                    // [CHUNK][N]
-    float* ds = Cs + SS_CHUNK * N;                    // [CHUNK][CPB] step sizes
-    float* xs = ds + SS_CHUNK * CPB;                  // [CHUNK][CPB]
-    float* zs = xs + SS_CHUNK * CPB;                  // [CHUNK][CPB]
-    float* S_g = a.state + (size_t)a.seq_slot[b] * a.state_stride + (size_t)(live ? c : 0) * N;
-    float* S_c = MODE == 0 ? S_g : a.chunk_state + (((size_t)b * a.n_chunks + chunk) * C + (live ? c : 0)) * N;
-    float S[SS_NPT], A[SS_NPT];
-#pragma unroll
-    for (int i = 0; i < SS_NPT; ++i) {
-        const int n = g + G * i;
-        const bool ok = live && n < N;
-        S[i] = (ok && MODE != 1) ? (MODE == 0 ? S_g[n] : S_c[n]) : 0.f;
-        A[i] = ok ? -expf(a.a_log[(size_t)c * N + n]) : 0.f;
-    }
-    float dt_sum = 0.f;
-    for (int s0 = t_begin; s0 < t_end; s0 += SS_CHUNK) {
-        const int ns = min(SS_CHUNK, t_end - s0);
-        __syncthreads();
-        for (int e = threadIdx.x; e < ns * N; e += RC_THREADS) {
-            const int s = e / N, n = e - s * N;
-            const TA* row = (const TA*)a.bc + (size_t)(qstart + s0 + s) * 2 * N;
-            Bs[e] = gl_load(row + n);
-            Cs[e] = gl_load(row + N + n);
-        }
-        for (int e = threadIdx.x; e < ns * CPB; e += RC_THREADS) {
-            const int s = e / CPB, j = e - s * CPB;
-            const size_t t = (size_t)(qstart + s0 + s);
-            const bool ok = c0 + j < C;
-            ds[e] = ok ? rc_softplus(a.dtp[t * C + c0 + j]) : 0.f;
-            xs[e] = ok ? gl_load((const TA*)a.x + t * C + c0 + j) : 0.f;
-            zs[e] = ok ? gl_load((const TA*)a.z + t * a.z_ld + a.z_off + c0 + j) : 0.f;
-        }
-        __syncthreads();
-#pragma unroll 4
-        for (int s = 0; s < ns; ++s) {
-            const float dt = ds[s * CPB + cl], x = xs[s * CPB + cl];
-            const float dx = dt * x;
-            if (MODE == 1) dt_sum += dt;
-            const float* Bt = Bs + s * N;
-            const float* Ct = Cs + s * N;
-            float y = 0.f;
-#pragma unroll
-            for (int i = 0; i < SS_NPT; ++i) {
-                const int n = g + G * i;
-                if (n < N) {
-                    S[i] = fmaf(rc_decay(dt * A[i]), S[i], dx * Bt[n]);
-                    y = fmaf(S[i], Ct[n], y);
-                }
-            }
-            for (int o = G >> 1; o > 0; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
-            if (g == 0) ds[s * CPB + cl] = y;           // the step size has been used: its place takes the sum
-        }
-        if (MODE == 1) continue;
-        __syncthreads();
-        // the skip connection and the gate do not go from token to token: all of the chunk's outputs at once
-        for (int e = threadIdx.x; e < ns * CPB; e += RC_THREADS) {
-            const int s = e / CPB, j = e - s * CPB;
-            if (c0 + j < C) {
-                const float y = fmaf(a.d_skip[c0 + j], xs[e], ds[e]);
-                gl_store((TA*)a.out + (size_t)(qstart + s0 + s) * C + c0 + j, y * rc_silu(zs[e]));
-            }
-        }
-    }
-    if (live && (MODE != 2 || t_end == qlen)) {       // the state row takes the run's last state
-        float* dst = MODE == 1 ? S_c : S_g;
-#pragma unroll
-        for (int i = 0; i < SS_NPT; ++i) {
-            const int n = g + G * i;
-            if (n < N) dst[n] = S[i];
-        }
-    }
-    if (MODE == 1 && live && g == 0) a.chunk_dt[((size_t)b * a.n_chunks + chunk) * C + c] = dt_sum;
-}
-
-// Between the two walks: every chunk's start state from the run's start state and the chunks' last states.
-__global__ void __launch_bounds__(128)
-selective_carry_kernel(SelectiveScanArgs a) {
-    gl_grid_launch_dependents();
-    gl_grid_wait();
-    const int b = blockIdx.y;
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (long long)a.C * a.N) return;
-    const int c = (int)(i / a.N);
-    const int chunks = (a.seq_qlen[b] + a.chunk_len - 1) / a.chunk_len;
-    float S = a.state[(size_t)a.seq_slot[b] * a.state_stride + i];
-    const float A = -expf(a.a_log[i]);
-    for (int k = 0; k < chunks; ++k) {
-        float* slot = a.chunk_state + ((size_t)b * a.n_chunks + k) * a.C * a.N + i;
-        const float last = *slot;
-        *slot = S;
-        S = fmaf(expf(A * a.chunk_dt[((size_t)b * a.n_chunks + k) * a.C + c]), S, last);
-    }
-}
-
-template <typename TA, int NPT>
-static int launch_selective_scan(const SelectiveScanArgs& a, cudaStream_t stream) {
-    int G = 1;
-    while (G * NPT < a.N) G <<= 1;
-    if (G > 32) return GL_ERR_SHAPE;
-    const int CPB = RC_THREADS / G;
-    const size_t smem = (size_t)SS_CHUNK * (2 * a.N + 3 * CPB) * sizeof(float);
-    if (smem > 48 * 1024) return GL_ERR_SMEM;
-    if (a.n_chunks <= 1) {
-        const dim3 grid((a.C + CPB - 1) / CPB, a.B);
-        return gl_launch_in_order(selective_scan_kernel<TA, NPT, 0>, grid, dim3(RC_THREADS), smem, stream, a, G);
-    }
-    const dim3 grid((a.C + CPB - 1) / CPB, a.B, a.n_chunks);
-    int rc = gl_launch_in_order(selective_scan_kernel<TA, NPT, 1>, grid, dim3(RC_THREADS), smem, stream, a, G);
-    if (rc != 0) return rc;
-    const long long n = (long long)a.C * a.N;
-    rc = gl_launch(selective_carry_kernel, dim3((unsigned)((n + 127) / 128), a.B), dim3(128), 0, stream, 1, a);
-    if (rc != 0) return rc;
-    return gl_launch_in_order(selective_scan_kernel<TA, NPT, 2>, grid, dim3(RC_THREADS), smem, stream, a, G);
-}
-
-static int selective_scan_blocks(const SelectiveScanArgs& a, int npt) {
-    int G = 1;
-    while (G * npt < a.N) G <<= 1;
-    if (G > 32) return -1;
-    const int CPB = RC_THREADS / G;
-    return ((a.C + CPB - 1) / CPB) * a.B * (a.n_chunks > 1 ? a.n_chunks : 1);
-}
-
-template <typename TA>
-static int dispatch_selective_scan(const SelectiveScanArgs& a, cudaStream_t stream) {
-    static int sms = 0;
-    if (!sms) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (sms <= 0) sms = 148;
-    }
-    const int want = 4 * sms;
-    const int b8 = selective_scan_blocks(a, 8), b2 = selective_scan_blocks(a, 2), b1 = selective_scan_blocks(a, 1);
-    if (b8 >= want || (b2 < 0 && b1 < 0)) return launch_selective_scan<TA, 8>(a, stream);
-    if (b2 >= want || b1 < 0) return b2 >= 0 ? launch_selective_scan<TA, 2>(a, stream) : launch_selective_scan<TA, 8>(a, stream);
-    return launch_selective_scan<TA, 1>(a, stream);
-}
-
-GL_API int gl_selective_scan(const SelectiveScanArgs* args, int act_dtype, cudaStream_t stream) {
-    const SelectiveScanArgs& a = *args;
-    if (a.B <= 0) return GL_OK;
-    if (a.C <= 0 || a.N <= 0 || a.N > 256 || a.B > 65535) return GL_ERR_SHAPE;
-    if (a.n_chunks > 1 && (!a.chunk_state || !a.chunk_dt || a.chunk_len <= 0 || a.n_chunks > 65535)) return GL_ERR_SHAPE;
-    if (act_dtype == GL_F32) return dispatch_selective_scan<float>(a, stream);
-    if (act_dtype == GL_BF16) return dispatch_selective_scan<__nv_bfloat16>(a, stream);
     return GL_ERR_DTYPE;
 }
 

@@ -296,3 +296,36 @@ def test_replay_of_a_trace(tmp_path):
     check(got4, ra[69:70], "float32", "step 4")
     assert not m.engine.cache.live_slots()
     m.close()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("C,N,qlens", [(40, 16, [1, 1, 1]), (40, 16, [1, 2, 3, 4, 5, 15]), (24, 4, [16, 17, 33]), (72, 24, [31, 6]),
+                                       (16, 40, [20, 1]), (3000, 16, [5, 40] * 8)])
+def test_selective_scan_forms(C, N, qlens, dtype):
+    """Runs that end inside a group of tokens and inside a staged chunk, one token a sequence, states of fewer lanes than a
+    group, of no power of two and too many to fetch ahead, and many sequences, against the recurrence in 64-bit."""
+    from types import SimpleNamespace
+    from gopherllm_b200 import ops
+    g = torch.Generator().manual_seed(C + N)
+    T, B, dev = sum(qlens), len(qlens), "cuda:0"
+    rn = lambda *s: torch.randn(*s, generator=g)
+    x, bc, z = rn(T, C).to(dtype), rn(T, 2 * N).to(dtype), rn(T, C + 8).to(dtype)
+    dtp, a_log, d_skip, state = rn(T, C) - 3, rn(C, N), rn(C), rn(B + 1, C * N)
+    starts = [sum(qlens[:i]) for i in range(B)]
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=dev)
+    ctx = SimpleNamespace(seq_slot=i32(list(range(1, B + 1))), seq_qstart=i32(starts), seq_qlen=i32(qlens), n_seqs=B, max_qlen=max(qlens), n_tokens=T)
+    kept = state.to(dev)
+    got = ops.selective_scan(x.to(dev), dtp.to(dev), bc.to(dev), z.to(dev), 8, a_log.to(dev), d_skip.to(dev), kept, ctx).cpu().double()
+    xd, bd, zd = x.double(), bc.double(), z.double()[:, 8:]
+    dt, A = torch.nn.functional.softplus(dtp.double()), -torch.exp(a_log.double())
+    want = torch.empty(T, C, dtype=torch.float64)
+    for b in range(B):
+        S = state[b + 1].double().view(C, N)
+        for t in range(starts[b], starts[b] + qlens[b]):
+            S = torch.exp(dt[t][:, None] * A) * S + (dt[t] * xd[t])[:, None] * bd[t, :N]
+            want[t] = (S @ bd[t, N:] + d_skip.double() * xd[t]) * torch.nn.functional.silu(zd[t])
+        scale = max(1.0, S.abs().max().item())
+        assert (kept[b + 1].cpu().double() - S.reshape(-1)).abs().max() <= 2e-6 * max(qlens) * scale      # 2^-22 a token
+    tol = 2e-5 if dtype == torch.float32 else 2 ** -8
+    assert (got - want).abs().max() <= tol * max(1.0, want.abs().max().item())
+    assert torch.equal(kept[0].cpu(), state[0])
