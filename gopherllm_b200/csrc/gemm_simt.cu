@@ -168,7 +168,7 @@ gemm_f32_kernel(GemmArgs g, const __grid_constant__ CUtensorMap map_a, const __g
     cg::cluster_group cluster = cg::this_cluster();
     const int S = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int m0 = (int)blockIdx.z * BM, n0 = (int)blockIdx.y * BN;
+    const int m0 = (int)blockIdx.y * BM, n0 = ((int)blockIdx.x / S) * BN;     // (columns on the grid's long side)
     unsigned char* smem = smem_raw + ((1024u - (gl_smem_u32(smem_raw) & 1023u)) & 1023u);
     const unsigned base = gl_smem_u32(smem);
     __shared__ alignas(8) unsigned long long bars[2 * STAGES];
@@ -330,8 +330,8 @@ static int launch_f32(const GemmArgs& g, cudaStream_t stream) {
     // clusters of S blocks that run at once
     static int at_once[FG_SEGS + 1] = {};
     static std::mutex mu;
-    const dim3 tiles(1, (g.N + SH::BN - 1) / SH::BN, (g.M + SH::BM - 1) / SH::BM);
-    if (tiles.y > 65535 || tiles.z > 65535) return GL_ERR_SHAPE;
+    const long tiles_n = ((long)g.N + SH::BN - 1) / SH::BN, tiles_m = ((long)g.M + SH::BM - 1) / SH::BM;
+    if (tiles_m > 65535) return GL_ERR_SHAPE;
     {
         std::lock_guard<std::mutex> lock(mu);
         if (!at_once[1]) {
@@ -364,7 +364,7 @@ static int launch_f32(const GemmArgs& g, cudaStream_t stream) {
     // Blocks a tile: the waves of clusters, each as long as a block's k-blocks; meeting in a cluster costs about as
     // much as FG_MEET of them (a barrier over the SMs and the peers' shared memory), so short products are not cut.
     const long k_blocks = (g.K + FG_BK - 1) / FG_BK, seg_blocks = (k_blocks + FG_SEGS - 1) / FG_SEGS;
-    const long n_tiles = (long)tiles.y * tiles.z, FG_MEET = SH::THREADS > 32 ? 2 : 4;
+    const long n_tiles = tiles_n * tiles_m, FG_MEET = SH::THREADS > 32 ? 2 : 4;
     int S = 1;
     long best = -1;
     for (int s = 1; s <= FG_SEGS; s *= 2) {
@@ -373,7 +373,7 @@ static int launch_f32(const GemmArgs& g, cudaStream_t stream) {
         const long cost = waves * ((mine < k_blocks ? mine : k_blocks) + (s > 1 ? FG_MEET : 0));
         if (best < 0 || cost < best) { best = cost; S = s; }
     }
-    if (gl_launch(gemm_f32_kernel<SH, TO>, dim3(S, tiles.y, tiles.z), dim3(SH::THREADS), SH::smem(S), stream, S, g, map_a, map_w) != 0)
+    if (gl_launch(gemm_f32_kernel<SH, TO>, dim3((unsigned)(S * tiles_n), (unsigned)tiles_m), dim3(SH::THREADS), SH::smem(S), stream, S, g, map_a, map_w) != 0)
         return GL_ERR_LAUNCH;
     return GL_OK;
 }

@@ -64,7 +64,7 @@ def test_gemm_simt(M, N, K, adt, wdt):
 def test_gemm_f32_rows(N, K):
     """32-bit operands with whole 16-byte rows: every height of tile and its edges, K of less than a k-block to
     many; and a row is the same number whatever rows are beside it (the tile, and so how K is shared, changes).
-    The bound: K products of relative error 2^-24 each, summed in four parts."""
+    The bound: K products of relative error 2^-24 each, summed in eight parts."""
     o = ops()
     M = 200 if N < 51200 else 40
     a, w = rnd(M, K, seed=1), rnd(N, K, scale=K ** -0.5, seed=2)
@@ -83,6 +83,17 @@ def test_gemm_f32_rows(N, K):
     x = add0.clone()
     o.gemm_simt(a, w, bias, "gelu", x, add1, out=x)
     assert torch.equal(x, whole)
+
+
+@pytest.mark.parametrize("M", [1, 9, 20])
+def test_gemm_f32_many_columns(M):
+    """More column tiles than a grid's short sides hold (65,535), for each tile of 32 or 64 columns; the bound as above."""
+    o = ops()
+    N, K = 65535 * 64 + 65, 4
+    a, w = rnd(M, K, seed=1), rnd(N, K, seed=2)
+    got = o.gemm_simt(a, w)
+    bound = 2 ** -24 * (8 + K ** 0.5) * (a.double().abs() @ w.double().abs().T)
+    assert ((got.double() - a.double() @ w.double().T).abs() <= bound).all()
 
 
 @pytest.mark.parametrize("M", [1, 3, 8, 9, 16, 33, 64])
