@@ -327,14 +327,18 @@ gemm_f32_kernel(GemmArgs g, const __grid_constant__ CUtensorMap map_a, const __g
 
 template <typename SH, typename TO>
 static int launch_f32(const GemmArgs& g, cudaStream_t stream) {
-    // clusters of S blocks that run at once
-    static int at_once[FG_SEGS + 1] = {};
+    // clusters of S blocks that run at once, on each device (a kernel's shared memory is allowed device by device)
+    struct AtOnce { int n[FG_SEGS + 1] = {}; };
+    static std::unordered_map<int, AtOnce> devices;
     static std::mutex mu;
     const long tiles_n = ((long)g.N + SH::BN - 1) / SH::BN, tiles_m = ((long)g.M + SH::BM - 1) / SH::BM;
     if (tiles_m > 65535) return GL_ERR_SHAPE;
+    int dev = 0, at_once[FG_SEGS + 1];
+    if (cudaGetDevice(&dev) != cudaSuccess) return GL_ERR_LAUNCH;
     {
         std::lock_guard<std::mutex> lock(mu);
-        if (!at_once[1]) {
+        AtOnce& known = devices[dev];
+        if (!known.n[1]) {
             if (cudaFuncSetAttribute(gemm_f32_kernel<SH, TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SH::smem(1)) != cudaSuccess) {
                 cudaGetLastError();
                 return GL_ERR_SMEM;
@@ -352,9 +356,10 @@ static int launch_f32(const GemmArgs& g, cudaStream_t stream) {
                 cfg.numAttrs = 1;
                 int n = 0;
                 if (cudaOccupancyMaxActiveClusters(&n, gemm_f32_kernel<SH, TO>, &cfg) != cudaSuccess || n < 1) { cudaGetLastError(); n = 1; }
-                at_once[S] = n;
+                known.n[S] = n;
             }
         }
+        memcpy(at_once, known.n, sizeof(at_once));
     }
     CUtensorMap map_a, map_w;
     int rc = gl_cached_map(&map_a, g.a, (uint64_t)g.M, (uint64_t)g.K, SH::A_ROWS, FG_BK, 4);

@@ -85,6 +85,17 @@ def test_gemm_f32_rows(N, K):
     assert torch.equal(x, whole)
 
 
+@pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs a second device")
+def test_gemm_f32_on_each_device():
+    """What a kernel is allowed (shared memory) is a device's own: the tile of 64 x 128 asks for more than the default."""
+    o = ops()
+    for dev in (0, 1):
+        with torch.cuda.device(dev):
+            a, w = (x.to(f"cuda:{dev}") for x in (rnd(200, 512, seed=1), rnd(2048, 512, seed=2)))
+            got = o.gemm_simt(a, w)
+            assert (got.double() - a.double() @ w.double().T).abs().max() <= 1e-3
+
+
 @pytest.mark.parametrize("M", [1, 9, 20])
 def test_gemm_f32_many_columns(M):
     """More column tiles than a grid's short sides hold (65,535), for each tile of 32 or 64 columns; the bound as above."""
