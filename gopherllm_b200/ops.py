@@ -1210,33 +1210,64 @@ class _MemoryChunkArgs(Structure):
 
 MEMORY_CHUNKS_MAX_ROWS = 128     # rows a head the chunked walk of the matrix memories takes (a column's rows in registers)
 USE_MEMORY_CHUNKS = True
-# The gated and the bounded-forget memories walk a run token by token or as chunks side by side: in chunks from
-# SCAN_CHUNKED_FROM tokens on, and shorter runs where that is expected to take less time.  Token by token a launch
-# takes as long as its longest run, or with many sequences as long as the machine needs for all of them (near the line
-# something of both); in chunks it takes some time for its passes and for every sequence, and the machine's time for all
-# tokens.  (us a token of the longest run; state elements times tokens a us in one piece; the passes' us; the same rate in
-# chunks), fitted to runs of 200 to 2,040 tokens, 1 to 16 sequences.  us a launch, one piece / chunks, of a memory of
-# 8 x 128 x 256: 1 x 1,000 tokens 503 / 250, 1 x 500 257 / 145, 4 of 64 to 1,000 800 / 470, 8 of 100 to 500 637 / 639,
-# 16 x 500 1788 / 1813; of 32 x 32 x 64: 345 / 177, 177 / 120, 498 / 273, 342 / 279, 505 / 796.
+# The gated and the bounded-forget memories walk a run token by token or as chunks side by side.  In 32 bits the order of
+# a state's sums follows the longest run alone and not how many sequences run beside it: chunks of SCAN_CHUNK_TOKENS from
+# SCAN_CHUNKED_FROM tokens on.  In bfloat16 also shorter runs, where chunks are expected to take clearly less time, and
+# shorter chunks: the order of the (32-bit) sums then depends on the lengths of all the step's runs.
+# Token by token a launch takes as long as its longest run, or with many sequences as long as the machine needs for all
+# of them (near the line something of both); in chunks it takes some time for its passes and for every sequence, and the
+# machine's time for all tokens.  (us a token of the longest run; state elements times tokens a us in one piece; the
+# passes' us; the same rate in chunks), fitted to runs of 200 to 2,040 tokens, 1 to 16 sequences.  us a launch, one
+# piece / chunks, of a memory of 8 x 128 x 256: 1 x 1,000 tokens 503 / 250, 1 x 500 257 / 145, 4 of 64 to 1,000 800 / 470,
+# 8 of 100 to 500 637 / 639, 16 x 500 1788 / 1813; of 32 x 32 x 64: 345 / 177, 177 / 120, 498 / 273, 342 / 279, 505 / 796.
+# MEMORY_CHUNK_GAIN: over nine memories of 1,024 to 524,288 elements and 22 batches of 1 to 17 runs of 64 to 1,000 tokens
+# chunks lost up to 14 % in 4 of the 48 cases where the expected gain was below 15 % (16 x 500 tokens of 32 x 128 x 128:
+# 2923 / 3381 us), and won 16 % to 6.8 times in the 172 where it was more.
 MEMORY_CHUNK_COST = {0: (0.5, 1.17e6, 55.0, 1.2e6), 1: (0.35, 1.04e6, 50.0, 0.8e6)}
 MEMORY_CHUNK_SEQUENCE = 8.0
+MEMORY_CHUNK_GAIN = 1.15
 # Chunks of 64 tokens, of 32 where the tokens are few (1 x 1,000 tokens 237 and 218 us with 64, 242 and 190 with 32; 1 x 500
 # 173 and 168, 133 and 132; 1 x 2,040 468 and 320, 474 and 340, and 469 and 399 with 128).
 MEMORY_CHUNK_TOKENS, MEMORY_CHUNK_TOKENS_FEW, MEMORY_CHUNK_FEW_TOKENS = 64, 32, 1200
 
 
 def memory_walks_chunks(kind: int, n_seqs: int, tokens: int, longest: int, elements: int) -> bool:
-    """Whether a gated or a bounded-forget memory of ``elements`` numbers walks a step's runs (``tokens`` in all) in chunks."""
+    """Whether a gated or a bounded-forget memory of ``elements`` numbers is expected to walk a step's runs (``tokens`` in
+    all) in chunks in clearly less time."""
     a_token, rate, passes, chunk_rate = MEMORY_CHUNK_COST[kind]
     run, all_runs = a_token * longest, tokens * elements / rate
-    return max(run, all_runs) + 0.5 * min(run, all_runs) > passes + MEMORY_CHUNK_SEQUENCE * n_seqs + tokens * elements / chunk_rate
+    chunks = passes + MEMORY_CHUNK_SEQUENCE * n_seqs + tokens * elements / chunk_rate
+    return max(run, all_runs) + 0.5 * min(run, all_runs) > MEMORY_CHUNK_GAIN * chunks
+
+
+def memory_chunk_tokens(kind: int, exact: bool, n_seqs: int, tokens: int, longest: int, H: int, D: int, V: int) -> int:
+    """Tokens a chunk of a memory's walk over runs of ``tokens`` in all, 0: token by token.  ``exact``: 32-bit inputs."""
+    if not USE_MEMORY_CHUNKS or kind not in (MEMORY_GATED, MEMORY_BOUNDED_FORGET, MEMORY_DECAY) or D > MEMORY_CHUNKS_MAX_ROWS:
+        return 0
+    if kind == MEMORY_DECAY:
+        if longest < DECAY_CHUNKED_FROM:
+            return 0
+        n = DECAY_CHUNK_TOKENS if longest >= DECAY_LONG_RUN else DECAY_CHUNK_TOKENS_SHORT
+    elif longest < SCAN_CHUNKED_FROM and (exact or not memory_walks_chunks(kind, n_seqs, tokens, longest, H * D * V)):
+        return 0
+    elif exact:
+        n = SCAN_CHUNK_TOKENS
+    else:
+        n = min(SCAN_CHUNK_TOKENS, MEMORY_CHUNK_TOKENS if tokens > MEMORY_CHUNK_FEW_TOKENS else MEMORY_CHUNK_TOKENS_FEW)
+    # every (sequence, chunk) keeps a whole state: many long sequences take longer chunks (not where the order of the sums
+    # must not depend on how many there are)
+    while (n_seqs * -(-longest // n) * H * D * V * 4 > MEMORY_CHUNKS_MAX_BYTES and n < 1024
+           and (kind == MEMORY_DECAY or not exact)):
+        n *= 2
+    chunks = -(-longest // n)
+    return n if (chunks > 1 or kind == MEMORY_DECAY) and n_seqs * chunks <= 65535 else 0        # (the grid's third size)
 
 
 # The plain decay's chunked walk pays from shorter runs on and with shorter chunks than the other kinds' (its gates
 # cost one pass, its rows are updated in pairs): a prompt of 256 / 512 / 1,024 / 2,048 tokens of ten such layers
 # at width 2,048 took 4.7 / 6.7 / 11.0 / 19.5 ms token by token, 3.7 / 4.5 / 6.0 / 9.9 ms in chunks of 32,
 # 4.0 / 4.5 / 6.0 / 8.9 ms in chunks of 64 and 4.6 / 5.0 / 6.1 / 9.0 ms in chunks of 128.
-MEMORY_CHUNKS_MAX_BYTES = 1 << 30     # of chunk states a launch of the plain decay may hold
+MEMORY_CHUNKS_MAX_BYTES = 1 << 30     # of chunk states a launch may hold before its chunks get longer
 DECAY_CHUNKED_FROM = 256
 DECAY_LONG_RUN = 512
 DECAY_CHUNK_TOKENS = 64          # runs of at least DECAY_LONG_RUN tokens
@@ -1261,7 +1292,8 @@ def memory_scan(kind: int, proj: torch.Tensor, state: torch.Tensor, ctx, H: int,
     times q_scale and k_scale.  Either ``decay`` [H] (keep = decay[h], take = 1) or ``gates`` with ``a_log`` and
     ``dt_bias`` [H]: dt = softplus(gates[t, f_off + h] + dt_bias[h]), keep = exp(-exp(a_log[h]) dt), take = dt.
     Long runs of the gated, the bounded-forget and the plain-decay kind (heads of up to MEMORY_CHUNKS_MAX_ROWS rows)
-    are walked as chunks side by side; which form runs depends on the lengths of the step's runs alone."""
+    are walked as chunks side by side: in 32 bits (and of the plain decay) by the step's longest run alone, in bfloat16 by
+    the lengths of all its runs."""
     _need(proj, "proj")
     rot_half = 0
     if kind == MEMORY_DECAY:
@@ -1301,20 +1333,9 @@ def memory_scan(kind: int, proj: torch.Tensor, state: torch.Tensor, ctx, H: int,
         _need(lower, "lower", torch.float32, (H * D,))
     out = empty((T, H * V), torch.float32, proj.device)
     gated, plain = kind == MEMORY_GATED, kind == MEMORY_DECAY
-    if plain:
-        chunk_tokens = DECAY_CHUNK_TOKENS if ctx.max_qlen >= DECAY_LONG_RUN else DECAY_CHUNK_TOKENS_SHORT
-        in_chunks = ctx.max_qlen >= DECAY_CHUNKED_FROM
-    else:
-        chunk_tokens = min(SCAN_CHUNK_TOKENS, MEMORY_CHUNK_TOKENS if T > MEMORY_CHUNK_FEW_TOKENS else MEMORY_CHUNK_TOKENS_FEW)
-        in_chunks = kind in MEMORY_CHUNK_COST and (ctx.max_qlen >= SCAN_CHUNKED_FROM
-                                                   or memory_walks_chunks(kind, ctx.n_seqs, T, ctx.max_qlen, H * D * V))
-    # every (sequence, chunk) keeps a whole state: many long sequences take longer chunks
-    while (ctx.n_seqs * -(-ctx.max_qlen // chunk_tokens) * H * D * V * 4 > MEMORY_CHUNKS_MAX_BYTES
-           and chunk_tokens < 1024):
-        chunk_tokens *= 2
-    chunks = -(-ctx.max_qlen // chunk_tokens)
-    if (USE_MEMORY_CHUNKS and in_chunks and D <= MEMORY_CHUNKS_MAX_ROWS and chunks > 1
-            and ctx.n_seqs * chunks <= 65535):                         # (the grid's third size)
+    chunk_tokens = memory_chunk_tokens(kind, proj.dtype == torch.float32, ctx.n_seqs, T, ctx.max_qlen, H, D, V)
+    if chunk_tokens:
+        chunks = -(-ctx.max_qlen // chunk_tokens)
         # a long run: chunks of tokens side by side, a lane a column (two walks and a carry between them)
         cols = V + (1 if gated else 0)
         chunk_state = empty((ctx.n_seqs, chunks, H, D, cols), torch.float32, proj.device)

@@ -156,3 +156,33 @@ def test_command_line_inspects_and_writes_a_random_folder(tmp_path, capsys):
     _, t = pv.read_folder(folder)
     logits = pv.forward(vm.GAMMA, t, [1, 2, 3, 4, 5])
     assert torch.isfinite(logits).all()
+
+
+def test_chunks_of_a_memory():
+    """Which runs the memories walk in chunks, and how long those are: in 32 bits and for the plain decay by the longest run
+    alone, in bfloat16 by what is expected to be faster; chunks get longer where their states would take too much memory."""
+    from gopherllm_b200 import ops
+    n = ops.memory_chunk_tokens
+    for kind in (ops.MEMORY_GATED, ops.MEMORY_BOUNDED_FORGET):
+        for sizes in ((8, 128, 256), (32, 32, 64), (2, 16, 32)):
+            for longest in (1, 127, 300, 500, 1023, 1024, 2040):
+                for batch in (1, 2, 4, 16, 64):
+                    assert n(kind, True, batch, batch * longest, longest, *sizes) == (128 if longest >= 1024 else 0)
+    gated = lambda *a: n(ops.MEMORY_GATED, False, *a, 8, 128, 256)
+    assert gated(1, 1, 1) == 0 and gated(1, 200, 200) == 0
+    assert gated(1, 500, 500) == 32 and gated(1, 1000, 1000) == 32
+    assert gated(4, 2128, 1000) == 64 and gated(1, 2040, 2040) == 64
+    assert gated(8, 2400, 500) == 0 and gated(16, 8000, 500) == 0          # near the line, or as fast token by token
+    forget = lambda *a: n(ops.MEMORY_BOUNDED_FORGET, False, *a, 32, 32, 64)
+    assert forget(1, 1000, 1000) == 32 and forget(4, 2128, 1000) == 64 and forget(16, 8000, 500) == 0
+    assert n(ops.MEMORY_GATED, False, 1, 150, 150, 4, 128, 128) == 0 and n(ops.MEMORY_GATED, False, 16, 8000, 500, 32, 128, 128) == 0
+    for exact in (True, False):
+        assert n(ops.MEMORY_GATED, exact, 1, 2040, 2040, 4, 256, 64) == 0      # more rows than a thread holds
+        assert n(ops.MEMORY_DELTA, exact, 1, 2040, 2040, 8, 128, 128) == 0
+        assert n(ops.MEMORY_DECAY, exact, 1, 255, 255, 32, 128, 64) == 0
+        assert n(ops.MEMORY_DECAY, exact, 1, 256, 256, 32, 128, 64) == 32 and n(ops.MEMORY_DECAY, exact, 1, 512, 512, 32, 128, 64) == 64
+        # 64 x 32 chunks of 1 MB: 2 GB of states with chunks of 64 tokens, 1 GB with 128
+        assert n(ops.MEMORY_DECAY, exact, 64, 64 * 2048, 2048, 32, 128, 64) == 128
+    assert n(ops.MEMORY_GATED, False, 64, 64 * 2048, 2048, 8, 128, 256) == 128
+    assert n(ops.MEMORY_GATED, True, 64, 64 * 2048, 2048, 8, 128, 256) == 128
+    assert n(ops.MEMORY_GATED, False, 40000, 80000, 1024, 1, 1, 1) == 0        # more chunks than a grid's third side holds

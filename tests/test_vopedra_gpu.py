@@ -329,3 +329,97 @@ def test_selective_scan_forms(C, N, qlens, dtype):
     tol = 2e-5 if dtype == torch.float32 else 2 ** -8
     assert (got - want).abs().max() <= tol * max(1.0, want.abs().max().item())
     assert torch.equal(kept[0].cpu(), state[0])
+
+
+def _memory_call(kind, H, D, V, qlens, dtype, seed, only=None):
+    """A gated (0) or bounded-forget (1) memory's run: its inputs on the CPU, and the call on the GPU with a fresh copy of the
+    states.  ``only``: the run of that sequence alone, with the inputs it has among the others."""
+    from types import SimpleNamespace
+    from gopherllm_b200 import ops
+    g = torch.Generator().manual_seed(seed)
+    rn = lambda *s: torch.randn(*s, generator=g)
+    B, T, dev = len(qlens), sum(qlens), "cuda:0"
+    pad = -(-2 * H // 8) * 8
+    proj = rn(T, 2 * H * D + H * V + (pad if kind == 0 else 0)).to(dtype)
+    lower = torch.rand(H * D, generator=g) * 0.9
+    state = rn(B + 1, ops.memory_state_size(kind, H, D, V)) * 0.3
+    if only is not None:
+        at = sum(qlens[:only])
+        proj, state, qlens = proj[at:at + qlens[only]], state[[0, only + 1]], [qlens[only]]
+        B, T = 1, qlens[0]
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=dev)
+    ctx = SimpleNamespace(seq_slot=i32(list(range(1, B + 1))), seq_qstart=i32([sum(qlens[:i]) for i in range(B)]), seq_qlen=i32(qlens),
+                          tok_seq=i32([b for b in range(B) for _ in range(qlens[b])]), n_seqs=B, max_qlen=max(qlens), n_tokens=T)
+    HD = H * D
+
+    def call():
+        kept, x = state.to(dev), proj.to(dev)
+        if kind == 0:
+            out = ops.memory_scan(0, x, kept, ctx, H, D, V, 0, HD, 2 * HD, 2 * HD + H * V, 2 * HD + H * V + H, cap=15.0, q_scale=D ** -0.5)
+        else:
+            out = ops.memory_scan(1, x, kept, ctx, H, D, V, 0, 0, 2 * HD, 0, HD, lower=lower.to(dev))
+        return out.cpu(), kept.cpu()
+    return proj, lower, state, call
+
+
+def _memory_in_64_bits(kind, H, D, V, qlens, proj, lower, state):
+    proj, HD = proj.double(), H * D
+    q, v = proj[:, :HD].view(-1, H, D), proj[:, 2 * HD:2 * HD + H * V].view(-1, H, V)
+    second = proj[:, HD:2 * HD].view(-1, H, D)
+    out, rows, t = torch.empty(proj.shape[0], H, V, dtype=torch.float64), state.double().clone(), 0
+    for b, n in enumerate(qlens):
+        row = rows[b + 1]
+        S = row[:HD * V].view(H, D, V).clone()
+        if kind == 0:
+            norm, m = row[HD * V:HD * V + HD].view(H, D).clone(), row[HD * V + HD:HD * V + HD + H].clone()
+            gates = proj[:, 2 * HD + H * V:]
+            gi = 15.0 * torch.tanh(gates[:, :H] / 15.0)
+            gf = torch.nn.functional.logsigmoid(15.0 * torch.tanh(gates[:, H:2 * H] / 15.0))
+        for _ in range(n):
+            if kind == 0:
+                m2 = torch.maximum(gf[t] + m, gi[t])
+                keep, take, m = torch.exp(gf[t] + m - m2), torch.exp(gi[t] - m2), m2
+                S = keep[:, None, None] * S + take[:, None, None] * second[t][:, :, None] * v[t][:, None, :]
+                norm = keep[:, None] * norm + take[:, None] * second[t]
+                qt = q[t] * D ** -0.5
+                den = torch.maximum((norm * qt).sum(-1).abs(), torch.exp(-m)) + 1e-6
+                out[t] = torch.einsum("hdv,hd->hv", S, qt) / den[:, None]
+            else:
+                low = lower.double().view(H, D)
+                f = low + (1 - low) * torch.sigmoid(second[t])
+                S = f[:, :, None] * S + (1 - f)[:, :, None] * v[t][:, None, :]
+                out[t] = torch.einsum("hdv,hd->hv", S, torch.nn.functional.silu(q[t]))
+            t += 1
+        rows[b + 1, :HD * V] = S.reshape(-1)
+        if kind == 0:
+            rows[b + 1, HD * V:HD * V + HD], rows[b + 1, HD * V + HD:HD * V + HD + H] = norm.reshape(-1), m
+    return out.reshape(-1, H * V), rows
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H,D,V", [(2, 16, 32), (3, 24, 40), (2, 128, 64)])
+@pytest.mark.parametrize("kind", [0, 1])
+def test_memories_token_by_token_and_in_chunks(kind, H, D, V, dtype, monkeypatch):
+    """The gated and the bounded-forget memory from states that are not zero, unequal runs beside one another (one token, whole
+    chunks, ragged last ones), in both forms and with every length of chunk, against the recurrence in 64 bits.  The bound:
+    a token adds a few roundings of 2^-24 to a sum and to the decays in front of it; a gated result is a quotient of two."""
+    from gopherllm_b200 import ops
+    qlens = [1, 33, 64, 129, 200]
+    proj, lower, state, call = _memory_call(kind, H, D, V, qlens, dtype, 7 + D)
+    want, rows = _memory_in_64_bits(kind, H, D, V, qlens, proj, lower, state)
+    for chunk in (0, 32, 64, 128, 256):
+        monkeypatch.setattr(ops, "memory_chunk_tokens", lambda *a: chunk)
+        got, kept = call()
+        for x, y, what in ((got, want, "results"), (kept, rows, "states")):
+            bound = 2 ** -22 * max(qlens) * max(1.0, float(y.abs().max()))
+            assert (x.double() - y).abs().max() <= bound, (what, chunk, float((x.double() - y).abs().max()), bound)
+        assert torch.equal(kept[0], state[0])
+
+
+@pytest.mark.parametrize("kind,H,D,V,n", [(0, 8, 128, 256, 300), (1, 32, 32, 64, 500), (0, 2, 16, 32, 1100)])
+def test_32_bit_states_do_not_depend_on_how_many_run_beside(kind, H, D, V, n):
+    """A prompt alone and among others of its length: the same state, bit for bit."""
+    together = _memory_call(kind, H, D, V, [n] * 4, torch.float32, 5)[3]()[1]
+    for b in range(4):
+        alone = _memory_call(kind, H, D, V, [n] * 4, torch.float32, 5, only=b)[3]()[1]
+        assert torch.equal(alone[1], together[b + 1]), b
