@@ -89,7 +89,7 @@ selective_scan_kernel(SelectiveScanArgs a, int G) {
         const int n = g + G * i;
         const bool ok = live && n < N;
         S[i] = (ok && MODE != 1) ? (WHOLE ? S_g[n] : S_c[n]) : 0.f;
-        A[i] = ok ? -expf(a.a_log[(size_t)c * N + n]) : 0.f;
+        A[i] = ok ? -expf(a.a_log[(size_t)c * N + n]) : -1.f;      // (not zero: an infinite step times zero would be NaN)
     }
     float dt_sum = 0.f;
     // A thread's share of a chunk's inputs travels while the chunk before is walked and waits in registers: a chunk's trip

@@ -331,6 +331,29 @@ def test_selective_scan_forms(C, N, qlens, dtype):
     assert torch.equal(kept[0].cpu(), state[0])
 
 
+@pytest.mark.parametrize("N", [16, 24, 5])
+@pytest.mark.parametrize("qlens", [[1, 1], [7, 20]])
+def test_selective_scan_with_an_endless_step(N, qlens):
+    """A step size that overflows to infinity forgets the state and writes infinity: nothing turns into NaN, also where the
+    lanes that share a channel hold more places than it has states."""
+    from types import SimpleNamespace
+    from gopherllm_b200 import ops
+    C, T, B, dev = 40, sum(qlens), len(qlens), "cuda:0"
+    g = torch.Generator().manual_seed(N)
+    up = lambda *s: torch.rand(*s, generator=g) + 0.1
+    x, bc, z, dtp, a_log, d_skip, state = up(T, C), up(T, 2 * N), up(T, C), up(T, C), up(C, N), up(C), up(B, C * N)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=dev)
+    starts = [sum(qlens[:i]) for i in range(B)]
+    for b, at in enumerate(starts):
+        dtp[at + qlens[b] // 2, ::3] = float("inf")
+    ctx = SimpleNamespace(seq_slot=i32(list(range(B))), seq_qstart=i32(starts), seq_qlen=i32(qlens), n_seqs=B, max_qlen=max(qlens), n_tokens=T)
+    got = ops.selective_scan(x.to(dev), dtp.to(dev), bc.to(dev), z.to(dev), 0, a_log.to(dev), d_skip.to(dev), state.to(dev), ctx).cpu()
+    for b, at in enumerate(starts):
+        hit = at + qlens[b] // 2
+        assert torch.isfinite(got[at:hit]).all() and torch.isfinite(got[at:at + qlens[b], 1::3]).all()
+        assert (got[hit:at + qlens[b], ::3] == float("inf")).all()
+
+
 def _memory_call(kind, H, D, V, qlens, dtype, seed, only=None):
     """A gated (0) or bounded-forget (1) memory's run: its inputs on the CPU, and the call on the GPU with a fresh copy of the
     states.  ``only``: the run of that sequence alone, with the inputs it has among the others."""
