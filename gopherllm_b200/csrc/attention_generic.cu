@@ -88,6 +88,7 @@ attn_generic_kernel(AttnArgs a) {
 #pragma unroll
     for (int i = 0; i < NACC; ++i) acc[i] = 0.f;
     float m = -INFINITY, l = 0.f;
+    int seen = 0x7fffffff, lost = -1;      // one token: the first key of the first half page taken, and of the last one left out for a NaN
 
     const int* pg = a.pages + (size_t)b * a.max_pages;
     if (qlen == 1) {
@@ -104,7 +105,11 @@ attn_generic_kernel(AttnArgs a) {
                 const bool ok = j >= lo_cta && j <= p_first;
                 const float s = ok ? ag_dot(q0, kp + (size_t)(half * 32 + lane) * hd, hd) : -INFINITY;
                 const float m_new = fmaxf(m, gl_warp_max(s));
-                if (m_new == -INFINITY) continue;
+                if (m_new == -INFINITY) {
+                    if (__any_sync(0xffffffffu, s != s)) lost = j0;
+                    continue;
+                }
+                if (m == -INFINITY) seen = j0;
                 const float pj = ok ? expf(s - m_new) : 0.f;
                 const float corr = expf(m - m_new);            // m = -inf gives 0
                 l = l * corr + gl_warp_sum(pj);
@@ -125,16 +130,24 @@ attn_generic_kernel(AttnArgs a) {
                 }
             }
         }
-        float* part = Ks;                                      // [AG_ROWS][hd + 2]: a warp's sums, its maximum and its weight
+        // a warp's sums, its maximum and its weight.  Scores that are NaN behind scores that are not make the row NaN, as
+        // where one warp walks all pages (there a half page of nothing but NaN has no maximum and is left out only as long
+        // as nothing came before it).
+        float* part = Ks;                                      // [AG_ROWS][hd + 2]
+        int* nan_at = (int*)(part + AG_ROWS * (hd + 2));       // [AG_ROWS][2]
         float* mine = part + warp * (hd + 2);
 #pragma unroll
         for (int i = 0; i < NACC; ++i)
             if (lane + 32 * i < hd) mine[lane + 32 * i] = acc[i];
-        if (lane == 0) { mine[hd] = m; mine[hd + 1] = l; }
+        if (lane == 0) { mine[hd] = m; mine[hd + 1] = l; nan_at[2 * warp] = seen; nan_at[2 * warp + 1] = lost; }
         __syncthreads();
         float top = -INFINITY;
 #pragma unroll
-        for (int w = 0; w < AG_ROWS; ++w) top = fmaxf(top, part[w * (hd + 2) + hd]);
+        for (int w = 0; w < AG_ROWS; ++w) {
+            top = fmaxf(top, part[w * (hd + 2) + hd]);
+            seen = min(seen, nan_at[2 * w]);
+            lost = max(lost, nan_at[2 * w + 1]);
+        }
         float f[AG_ROWS], den = 0.f;
 #pragma unroll
         for (int w = 0; w < AG_ROWS; ++w) {
@@ -142,7 +155,7 @@ attn_generic_kernel(AttnArgs a) {
             f[w] = mw > -INFINITY ? expf(mw - top) : 0.f;
             den = fmaf(f[w], part[w * (hd + 2) + hd + 1], den);
         }
-        const float inv = den > 0.f ? 1.0f / den : 0.f;
+        const float inv = lost > seen ? NAN : den > 0.f ? 1.0f / den : 0.f;
         TA* o = (TA*)a.out + ((size_t)a.seq_qstart[b] * a.nH + h) * hd;
         for (int d = threadIdx.x; d < hd; d += AG_ROWS * 32) {
             float y = 0.f;

@@ -469,6 +469,24 @@ def test_attention_generic_one_token(dtype, nH, nKV, hd, window):
     run_attention("generic", dtype, nH, nKV, hd, window, [200, 30, 64], [1, 5, 1])
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_attention_generic_one_token_shows_a_nan(dtype):
+    """A key that is NaN makes the row NaN wherever it lies: alone on its page, a page's worth, in the middle, at the start."""
+    o = ops()
+    ctxs, bad = [64, 200, 700, 300, 300], [[64], range(128, 201), [650], [2], []]
+    B, nH, nKV, hd = len(ctxs), 4, 2, 64
+    k, v, q = rnd(B, 701, nKV, hd, seed=1), rnd(B, 701, nKV, hd, seed=2), (rnd(B, nH * hd, seed=3) / 8).to(dtype)
+    kc, vc, table = make_cache(k, v, [c + 1 for c in ctxs], dtype)
+    for b, places in enumerate(bad):
+        for p in places:
+            kc[int(table[b, p // 64]), :, p % 64] = float("nan")
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    out = torch.empty(B, nH * hd, dtype=dtype, device=DEV)
+    o.attention_generic(q, out, kc, vc, i32(list(range(B))), i32([1] * B), i32(ctxs), table, nH, nKV, hd, 1)
+    for b, places in enumerate(bad):
+        assert torch.isnan(out[b]).all() if len(places) else torch.isfinite(out[b]).all(), b
+
+
 def run_attention(kernel, dtype, nH, nKV, hd, window, ctxs, qlens):
     o = ops()
     B, L = len(ctxs), max(c + q for c, q in zip(ctxs, qlens))
