@@ -39,7 +39,10 @@
 // head, so that a half meets sequences of different lengths.  (Sequence by sequence and by pages alone, the
 // halves that got the short sequences walked through sixty heads of one page while the others waited: 64
 // sequences of 16 to 1,024 positions took 214 us a layer of Phi-2, now 126; 40 of 16 to 700 of Phi-1.5 82
-// with pages alone, 78 with DL_LEAD; equal lengths are unchanged.)
+// with pages alone, 78 with DL_LEAD.)  Where all sequences have as many pages no half can be given short ones:
+// there the line is (sequence, key/value head, page) and counts pages alone, so that a half reads heads that lie
+// side by side in a page (four steps of Phi-1.5, 40 x 60 positions: 6.03 ms, 6.27 head by head; 64 x 500: 10.2,
+// 10.5; Phi-2, 64 x 16: 9.97, 10.11).
 //
 // The products run on tcgen05: the 128 weight rows of a tile are the M of the instruction, the tokens
 // (padded to 16, 32 or 64) its N, the accumulator lies in tensor memory; one thread issues the four
@@ -270,7 +273,7 @@ decode_layer_kernel(const __grid_constant__ LayerArgs a) {
     int* s_off = (int*)misc;                              // [MAXB + 1] first unit of each sequence in a head's stretch of phase 2
     int* s_first = s_off + DL_MAXB + 1;                   // [MAXB] first page each sequence reads
     int* s_n = s_first + DL_MAXB;                         // [MAXB] pages each sequence reads
-    int* s_flag = s_n + DL_MAXB;                          // [7] (200 ints so far: what follows stays 16-byte aligned)
+    int* s_flag = s_n + DL_MAXB;                          // [7] 0: last to arrive, 1: equal pages (200 ints so far: what follows stays 16-byte aligned)
     float* red = (float*)(s_flag + 7);                    // [4]
     __nv_bfloat16* pw = (__nv_bfloat16*)(red + 4);        // [4 warps][8 heads][16 keys]
     float* mrg = (float*)(pw + 4 * 8 * 16);               // [64] + [4][hd][G] (+ the queries before that)
@@ -290,16 +293,21 @@ decode_layer_kernel(const __grid_constant__ LayerArgs a) {
         }
         mbar_init(acc_bar, 1);
         mbar_fence_init();
-        int off = 0;
+        int off = 0, n0 = 0;
+        bool same = true;
         for (int b = 0; b < p.M; ++b) {
             const int pos = p.seq_ctx[b];
             const int lo = (p.window > 0 && pos - p.window + 1 > 0) ? pos - p.window + 1 : 0;
+            const int n = pos / GL_PAGE + 1 - lo / GL_PAGE;
             s_off[b] = off;
             s_first[b] = lo / GL_PAGE;
-            s_n[b] = pos / GL_PAGE + 1 - lo / GL_PAGE;
-            off += DL_LEAD + s_n[b];
+            s_n[b] = n;
+            off += DL_LEAD + n;
+            if (b == 0) n0 = n;
+            same = same && n == n0;
         }
         s_off[p.M] = off;
+        s_flag[1] = same ? n0 : 0;
     }
     __syncwarp();
     if (threadIdx.x < 32) tmem_alloc(gl_smem_u32(tmem_slot), 2 * TMEM_COLS);      // both halves' accumulators
@@ -316,14 +324,24 @@ decode_layer_kernel(const __grid_constant__ LayerArgs a) {
         }
         return lo;
     };
-    const int headA = s_off[p.M], totalA = headA * p.nKV;
+    // s_off[M] units are a head's stretch of the line; where every sequence has as many pages (s_flag[1] of them) the line runs
+    // sequence by sequence and counts pages alone  (both are read again where they are used: registers are short here)
+    const int totalA = (s_flag[1] ? s_flag[1] * p.M : s_off[p.M]) * p.nKV;
     const int perA = (totalA + GC - 1) / GC;
     const int a0 = min(totalA, c * perA), a1 = min(totalA, a0 + perA);
     // The next run of pages at or behind unit L of this block's stretch: ``cnt`` pages from the pi-th on of head g of
     // sequence b; L moves to the first of them.  False where only units without a page are left.
     auto pages_at = [&](int& L, int& b, int& g, int& pi, int& cnt) {
-        g = L / headA;
-        const int r = L - g * headA;
+        if (const int same = s_flag[1]) {
+            const int head = L / same;
+            b = head / p.nKV;
+            g = head - b * p.nKV;
+            pi = L - head * same;
+            cnt = min(same - pi, a1 - L);
+            return true;
+        }
+        g = L / s_off[p.M];
+        const int r = L - g * s_off[p.M];
         b = seq_of(r);
         const int u = r - s_off[b], skip = max(0, DL_LEAD - u);
         if (skip >= a1 - L) return false;
@@ -837,7 +855,7 @@ decode_layer_kernel(const __grid_constant__ LayerArgs a) {
             }
             cons_sync();
             // which blocks hold pages of this (sequence, head), and this block's number among them
-            const int Ls = g * headA + s_off[b] + DL_LEAD;
+            const int Ls = s_flag[1] ? (b * p.nKV + g) * nb : g * s_off[p.M] + s_off[b] + DL_LEAD;
             const int first = Ls / perA, last = (Ls + nb - 1) / perA;
             const int nseg = last - first + 1, ord = c - first;
             float* part = a.scratchA + ((size_t)(b * p.nKV + g) * a.maxsegA) * OSZ;

@@ -815,6 +815,9 @@ def test_decode_layer(M, nH, nKV, hd, D, I, rot, window, rms, act, bias):
     [63, 64, 65, 0] * 16,                       # a page's edges only
     [1000 - 15 * i for i in range(64)],         # every length from long to short
     [5],
+    [130] * 33,                                 # as many pages each: cut sequence by sequence
+    [70 + i for i in range(50)],                # the same, with other positions in the last page
+    [0] * 64,
 ])
 def test_decode_layer_unequal_lengths(ctxs, window):
     """The pages of all sequences' heads are cut into equal stretches, where a head counts for more than its pages."""
