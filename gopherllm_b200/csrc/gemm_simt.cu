@@ -383,16 +383,130 @@ static int launch_f32(const GemmArgs& g, cudaStream_t stream) {
     return GL_OK;
 }
 
+// The same sums with the loop of gemm_simt_kernel: blocks of 256 threads, several an SM, no copies ahead, 64 x 64 results.
+// For short K with many tiles, where a block of gemm_f32_kernel (one an SM, its shared memory being mostly stages and sums
+// put by) spends more on starting and finishing a tile than on its few k-blocks.  Even and odd k, parts and pairs of parts as
+// there, so a row is the same number from either.  Sums of one and of two parts wait in shared memory (in registers they
+// would cost one of four blocks an SM); with more than four parts (TOP) those of four wait in registers and three blocks fit
+// (four, with the registers spilled or three quarters of them in shared memory, took 3 to 13 % longer).
+template <typename TO, bool TOP>
+__global__ void __launch_bounds__(256, TOP ? 3 : 4)
+gemm_f32_short_kernel(GemmArgs g) {
+    extern __shared__ float put[];                     // [levels that wait here][16][256], a thread's own place
+    __shared__ float As[SG_BK][SG_BM + 4];
+    __shared__ float Ws[SG_BK][SG_BN + 4];
+    const float *A = (const float*)g.a, *W = (const float*)g.w;
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    const int m0 = blockIdx.y * SG_BM, n0 = blockIdx.x * SG_BN;
+    const int k_blocks = (g.K + FG_BK - 1) / FG_BK, part = (k_blocks + FG_SEGS - 1) / FG_SEGS * FG_BK;
+    float acc[2][4][4], top[TOP ? 16 : 1];
+    auto clear = [&]() {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[0][i][j] = acc[1][i][j] = 0.f;
+    };
+    // the finished part, joined with the sums that wait on the levels of pairs in ``levels``
+    auto joined = [&](int levels, int i, int j) {
+        float q = acc[0][i][j] + acc[1][i][j];
+        const int at = (i * 4 + j) * 256 + tid;
+        if (levels & 1) q = put[at] + q;
+        if (levels & 2) q = put[16 * 256 + at] + q;
+        if (TOP && (levels & 4)) q = top[TOP ? i * 4 + j : 0] + q;
+        return q;
+    };
+    clear();
+    int seg = 0;
+    for (int k_at = 0;; k_at += part, ++seg) {
+        const int stop = min(k_at + part, g.K);
+        for (int k0 = k_at; k0 < stop; k0 += SG_BK) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int e = tid + i * 256, r = e >> 4, c = e & 15;
+                const int k = k0 + c;
+                float va = 0.f, vw = 0.f;
+                if (k < g.K) {
+                    if (m0 + r < g.M) va = A[(size_t)(m0 + r) * g.K + k];
+                    if (n0 + r < g.N) vw = W[(size_t)(n0 + r) * g.K + k];
+                }
+                As[c][r] = va;
+                Ws[c][r] = vw;
+            }
+            __syncthreads();
+#pragma unroll
+            for (int kk = 0; kk < SG_BK; ++kk) {
+                float av[4], wv[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) av[i] = As[kk][ty * 4 + i];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) wv[j] = Ws[kk][tx * 4 + j];
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) acc[kk & 1][i][j] = fmaf(av[i], wv[j], acc[kk & 1][i][j]);
+            }
+            __syncthreads();
+        }
+        if (stop == g.K) break;
+        const int levels = seg & ~(seg + 1);           // what pairs with the part so far: it waits on the next level
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float q = joined(levels, i, j);
+                if (levels == 0) put[(i * 4 + j) * 256 + tid] = q;
+                else if (levels == 1) put[(16 + i * 4 + j) * 256 + tid] = q;
+                else if (TOP) top[TOP ? i * 4 + j : 0] = q;
+            }
+        clear();
+    }
+    TO* O = (TO*)g.out;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int m = m0 + ty * 4 + i;
+        if (m >= g.M) continue;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int n = n0 + tx * 4 + j;
+            if (n >= g.N) continue;
+            float v = joined(seg, i, j);
+            if (g.bias) v += g.bias[n];
+            v = gl_activate<true>(v, g.act, g.act_p0, g.act_p1);
+            const size_t o = (size_t)m * g.N + n;
+            if (g.add0) v += g.add0[o];
+            if (g.add1) v += g.add1[o];
+            gl_store(O + o, v);
+        }
+    }
+}
+
+template <typename TO>
+static int launch_f32_short(const GemmArgs& g, cudaStream_t stream) {
+    const int k_blocks = (g.K + FG_BK - 1) / FG_BK, seg_blocks = (k_blocks + FG_SEGS - 1) / FG_SEGS, parts = (k_blocks + seg_blocks - 1) / seg_blocks;
+    const dim3 grid((g.N + SG_BN - 1) / SG_BN, (g.M + SG_BM - 1) / SG_BM);
+    if (grid.y > 65535) return GL_ERR_SHAPE;
+    const size_t smem = (size_t)(parts > 2 ? 2 : parts > 1 ? 1 : 0) * 16 * 256 * sizeof(float);
+    if (parts > 4) gemm_f32_short_kernel<TO, true><<<grid, 256, smem, stream>>>(g);
+    else gemm_f32_short_kernel<TO, false><<<grid, 256, smem, stream>>>(g);
+    return gl_check_launch();
+}
+
 // Rows of a tile: as few as hold all rows, since up to about 20 rows the weights' stream is the longer of the two and
 // beyond that every padded row costs FMA time.  The few rows' blocks are a warp each, so that enough of them fit an SM to
 // keep both the weights' stream and the FMA units busy.  From 33 rows on tiles of 64 x 128, whose shared-memory loads
-// are half as many a product as those of 32 x 64 (632 rows x 8192 x 2048: 43 against 22 TFLOP/s), unless the product is
+// are half as many a product as those of 32 x 64 (632 rows x 8192 x 2048: 40 against 22 TFLOP/s), unless the product is
 // too small to occupy the SMs with them: then a tile's own start and finish count (80 rows x 256 x 64: 24 us against 16).
+// Short K with many tiles: gemm_f32_short_kernel.  us with the TMA tiles / with it: 2,048 rows x 8192 x 32 230 / 78, x 64
+// 263 / 119, x 128 326 / 205, x 192 391 / 326, x 256 456 / 422, x 384 547 / 584; 632 x 2048 x 128 28 / 26; 200 x 4096 x 128
+// 20 / 22; 200 x 8192 x 256 64 / 80 (512 tiles of 64 x 64).  Below 64 also with few tiles: there is a k-block or two to fetch
+// ahead (64 x 2048 x 32 9.3 / 7.9, x 64 10.5 / 11.8).
 template <typename TO>
 static int dispatch_f32(const GemmArgs& g, cudaStream_t stream) {
     if (g.M <= 4) return launch_f32<FgShape<1, 1, 1, 4, 1, 5>, TO>(g, stream);
     if (g.M <= 8) return launch_f32<FgShape<1, 1, 1, 8, 1, 5>, TO>(g, stream);
     if (g.M <= 16) return launch_f32<FgShape<1, 1, 2, 8, 2, 4>, TO>(g, stream);
+    const long short_tiles = (long)((g.M + SG_BM - 1) / SG_BM) * ((g.N + SG_BN - 1) / SG_BN);
+    if (g.K < 64 || (g.K <= 128 && short_tiles >= 256) || (g.K <= 256 && short_tiles >= 1024)) return launch_f32_short<TO>(g, stream);
     const long big_tiles = (long)((g.M + 63) / 64) * ((g.N + 127) / 128), k_blocks = (g.K + FG_BK - 1) / FG_BK;
     if (g.M <= 32 || big_tiles * k_blocks < 8 * 148) return launch_f32<FgShape<1, 2, 4, 8, 4, 4>, TO>(g, stream);
     return launch_f32<FgShape<2, 2, 4, 8, 8, 3>, TO>(g, stream);

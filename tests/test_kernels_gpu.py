@@ -96,6 +96,23 @@ def test_gemm_f32_on_each_device():
             assert (got.double() - a.double() @ w.double().T).abs().max() <= 1e-3
 
 
+@pytest.mark.parametrize("K", [4, 36, 64, 68, 100, 128, 160, 192, 224, 256, 260, 320, 384])
+def test_gemm_f32_short_sums(K):
+    """Short K with many tiles takes another kernel: a row is the same number from either, and the epilogue is the same."""
+    o = ops()
+    M, N = 1000, 4200      # 1,056 tiles of 64 x 64
+    a, w = rnd(M, K, seed=1), rnd(N, K, scale=K ** -0.5, seed=2)
+    bias, add0, add1 = rnd(N, seed=3), rnd(M, N, seed=4), rnd(M, N, seed=5)
+    ref = ref_linear(a, w, bias, "gelu", add0, add1)
+    bound = 2 ** -24 * (8 + K ** 0.5) * (a.double().abs() @ w.double().abs().T + 4)
+    whole = o.gemm_simt(a, w, bias, "gelu", add0, add1)
+    assert ((whole.double() - ref).abs() <= bound).all()
+    for m in (1, 8, 16, 17, 40, 300):
+        assert torch.equal(o.gemm_simt(a[:m], w, bias, "gelu", add0[:m], add1[:m]), whole[:m]), m
+    assert torch.equal(o.gemm_simt(a, w[:130], bias[:130], "gelu", add0[:, :130].contiguous(), add1[:, :130].contiguous()), whole[:, :130])
+    assert torch.equal(o.gemm_simt(a, w, bias, out_dtype=torch.bfloat16), o.gemm_simt(a, w, bias).bfloat16())
+
+
 @pytest.mark.parametrize("M", [1, 9, 20])
 def test_gemm_f32_many_columns(M):
     """More column tiles than a grid's short sides hold (65,535), for each tile of 32 or 64 columns; the bound as above."""
