@@ -686,12 +686,13 @@ head_mix_split_kernel(MixedAttnArgs a) {
     }
 }
 
-// Blocks of AM_MIX_THREADS where there is a table and the values' rows are whole 16-byte pieces (the kernel tells by the block).
+// Blocks of AM_MIX_THREADS where there is a table and the ranges' sums are whole, aligned 16-byte pieces (the kernel tells by the
+// block).
 template <typename TA>
 static int launch_head_mix_split(const MixedAttnArgs& a, cudaStream_t stream) {
     const size_t factors = (((size_t)(a.mix ? a.nH : 1) * a.splits + 3) & ~(size_t)3) * sizeof(float);
     const size_t with_sums = factors + AM_MIX_THREADS * sizeof(float4);
-    const bool wide = a.mix && a.splits <= 64 && a.vd % 4 == 0 && a.vd <= 4 * AM_MIX_THREADS && with_sums <= 48 * 1024;
+    const bool wide = a.mix && a.splits <= 64 && a.vd % 4 == 0 && ((uintptr_t)a.parts & 15) == 0 && a.vd <= 4 * AM_MIX_THREADS && with_sums <= 48 * 1024;
     return gl_launch(head_mix_split_kernel<TA>, dim3(a.nH, a.B), dim3(wide ? AM_MIX_THREADS : a.vd <= 64 ? 64 : 128),
                      wide ? with_sums : factors, stream, 1, a);
 }

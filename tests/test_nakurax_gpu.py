@@ -818,3 +818,30 @@ def test_attention_with_a_table_over_the_heads(heads, groups, dim, vdim, dtype):
                 own = slice(c * (heads // groups), (c + 1) * (heads // groups))
                 want[:, own] = torch.einsum("hg,tgv->thv", mix.double()[own], y.view(-1, heads, vdim))
             assert (got - want.reshape(sum(qlens), -1)).abs().max() < tol, (kw, qlens, float((got - want.reshape(sum(qlens), -1)).abs().max()))
+
+
+@pytest.mark.parametrize("shift", [0, 1, 4])
+def test_ranges_put_together_from_any_address(shift):
+    """The C entry that puts a one-token step's ranges together under a table over the heads, with partial sums that begin on a
+    16-byte boundary and not."""
+    import ctypes
+    from gopherllm_b200 import ops
+    B, H, G, vd, splits = 3, 6, 3, 24, 5
+    g = torch.Generator().manual_seed(2)
+    n = B * H * G * splits * vd
+    parts = torch.randn(n + shift, generator=g).to(DEV)
+    ml = torch.stack([torch.randn(B, H, splits, generator=g), torch.rand(B, H, splits, generator=g) + 0.5], -1).to(DEV).contiguous()
+    mix = torch.randn(H, H, generator=g).to(DEV)
+    start = torch.arange(B, dtype=torch.int32, device=DEV)
+    out = torch.empty(B, H * vd, device=DEV)
+    a = ops._MixedAttnArgs()
+    a.out, a.mix, a.seq_qstart, a.ml, a.parts = out.data_ptr(), mix.data_ptr(), start.data_ptr(), ml.data_ptr(), parts.data_ptr() + 4 * shift
+    a.T, a.B, a.nH, a.nKV, a.hd, a.vd, a.max_qlen, a.splits = B, B, H, G, 16, vd, 1, splits
+    assert ops._lib("attention_mixed.cu").gl_head_mix_split(ctypes.byref(a), ctypes.c_int(0), ops._stream()) == 0
+    m, l = ml[..., 0].double(), ml[..., 1].double()
+    f = torch.exp(m - m.max(-1, keepdim=True).values)
+    f = f / (f * l).sum(-1, keepdim=True)
+    heads = torch.einsum("bgs,bgcsv->bgcv", f, parts[shift:].double().view(B, H, G, splits, vd))
+    own = torch.arange(H, device=DEV) // (H // G)
+    want = torch.stack([torch.einsum("g,bgv->bv", mix.double()[h], heads[:, :, own[h]]) for h in range(H)], 1).reshape(B, -1)
+    assert (out.double() - want).abs().max() <= 1e-5 * max(1.0, float(want.abs().max()))
