@@ -10,12 +10,15 @@
 // A query at position p sees keys lo..p, lo = 0 or p-window+1
 // (model.go:2707-2710); nothing else masks.
 //
-// A sequence that brings one token has one query row for a block of eight warps: there the
-// warps share the row's pages (page i with warp i mod 8, straight from the cache, no tiles),
-// and their softmaxes are merged in the warps' order.  What bounds such a row is the chain of
-// trips to memory, a page after the other: 4 sequences of 16 to 300 positions, 32 heads of 64,
-// took 57 us a launch with one warp walking all pages, now 28.  The form depends on the
-// sequence's own run alone, so a row still does not depend on the batch around it.
+// A sequence that brings one token has one query row for a block of eight warps: there, from
+// AG_SHARE_FROM pages on, the warps share the row's pages (page i with warp i mod 8, straight
+// from the cache, no tiles), and their softmaxes are merged in the warps' order.  What bounds
+// such a row is the chain of trips to memory, a page after the other: 4 sequences of 16 to 300
+// positions, 32 heads of 64 in 32 bits, took 57 us a launch with one warp walking all pages, now
+// 28; 1 x 2,000 385 and 102; 16 heads of 100 in bfloat16, 64 x 300, 200 and 101 (keys read two
+// bytes at a time: 268).  On fewer pages the tiles' wide loads are ahead (1 x 10 positions, 8
+// heads of 40: 12 us with tiles, 16 without; 1 x 100 23 and 29; 16 x 128 29 and 31).  The form
+// depends on the sequence's own run alone, so a row still does not depend on the batch around it.
 #include "common.cuh"
 
 struct AttnArgs {
@@ -33,8 +36,9 @@ struct AttnArgs {
 };
 
 #define AG_ROWS 8
+#define AG_SHARE_FROM 4               // pages a one-token row sees from which its block's warps share them
 
-// q . k with k in ascending order; rows of whole 16-byte pieces are read as such
+// q . k with k in ascending order; rows of whole 16-byte (of bfloat16 also 8-byte) pieces are read as such
 __device__ __forceinline__ float ag_dot(const float* q, const float* k, int hd) {
     float s = 0.f;
     if ((hd & 3) == 0 && ((uintptr_t)k & 15) == 0) {
@@ -48,16 +52,33 @@ __device__ __forceinline__ float ag_dot(const float* q, const float* k, int hd) 
     }
     return s;
 }
+__device__ __forceinline__ float ag_add2(float s, const float* q, unsigned pair) {
+    const float2 v = __bfloat1622float2(*(const __nv_bfloat162*)&pair);
+    return fmaf(q[1], v.y, fmaf(q[0], v.x, s));
+}
 __device__ __forceinline__ float ag_dot(const float* q, const __nv_bfloat16* k, int hd) {
     float s = 0.f;
+    if ((hd & 7) == 0 && ((uintptr_t)k & 15) == 0) {
+#pragma unroll 4
+        for (int d = 0; d < hd; d += 8) {
+            const uint4 v = *(const uint4*)(k + d);
+            s = ag_add2(s, q + d, v.x); s = ag_add2(s, q + d + 2, v.y); s = ag_add2(s, q + d + 4, v.z); s = ag_add2(s, q + d + 6, v.w);
+        }
+    } else if ((hd & 3) == 0 && ((uintptr_t)k & 7) == 0) {
 #pragma unroll 8
-    for (int d = 0; d < hd; ++d) s = fmaf(q[d], gl_load(k + d), s);
+        for (int d = 0; d < hd; d += 4) {
+            const uint2 v = *(const uint2*)(k + d);
+            s = ag_add2(s, q + d, v.x); s = ag_add2(s, q + d + 2, v.y);
+        }
+    } else {
+#pragma unroll 8
+        for (int d = 0; d < hd; ++d) s = fmaf(q[d], gl_load(k + d), s);
+    }
     return s;
 }
 
 template <typename TA, typename TC, int NACC>
-__global__ void __launch_bounds__(AG_ROWS * 32)
-attn_generic_kernel(AttnArgs a) {
+__device__ __forceinline__ void ag_rows(const AttnArgs& a) {
     extern __shared__ float smem[];
     const int hd = a.hd, ks = hd + 1;
     float* Ks = smem;                       // [GL_PAGE][hd+1]
@@ -91,7 +112,7 @@ attn_generic_kernel(AttnArgs a) {
     int seen = 0x7fffffff, lost = -1;      // one token: the first key of the first half page taken, and of the last one left out for a NaN
 
     const int* pg = a.pages + (size_t)b * a.max_pages;
-    if (qlen == 1) {
+    if (qlen == 1 && p_first / GL_PAGE - lo_cta / GL_PAGE + 1 >= AG_SHARE_FROM) {
         // (the block's row 0: p_first is its position and lo_cta its first key)
         __syncthreads();
         const float* q0 = Qs;
@@ -220,9 +241,21 @@ attn_generic_kernel(AttnArgs a) {
 }
 
 template <typename TA, typename TC, int NACC>
+__global__ void __launch_bounds__(AG_ROWS * 32)
+attn_generic_kernel(AttnArgs a) { ag_rows<TA, TC, NACC>(a); }
+
+// Heads of more than 96: as many blocks an SM as shared memory allows (a prompt of 1,000 tokens, 16 heads of 100 in bfloat16: 742 us
+// with the compiler's choice of registers, 627 so; the smaller heads lose by any limit, up to half of their rate).
+template <typename TA, typename TC, int NACC>
+__global__ void __launch_bounds__(AG_ROWS * 32, NACC <= 4 ? 4 : NACC <= 6 ? 3 : 2)
+attn_generic_wide_kernel(AttnArgs a) { ag_rows<TA, TC, NACC>(a); }
+
+template <typename TA, typename TC, int NACC>
 static int launch_generic(const AttnArgs& a, cudaStream_t stream) {
     const size_t smem = ((size_t)GL_PAGE * (a.hd + 1) + (size_t)GL_PAGE * a.hd + (size_t)AG_ROWS * a.hd) * sizeof(float);
-    auto kern = attn_generic_kernel<TA, TC, NACC>;
+    void (*kern)(AttnArgs);
+    if constexpr (NACC > 3) kern = attn_generic_wide_kernel<TA, TC, NACC>;
+    else kern = attn_generic_kernel<TA, TC, NACC>;
     if (smem > 48 * 1024) {
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
             cudaGetLastError();
