@@ -44,6 +44,13 @@ struct MixedAttnArgs {
     int chunk;                // > 0: a query sees the keys of its own chunk of positions alone (window is then 0)
 };
 
+static int am_sm_count() {
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms > 0 ? sms : 148;
+}
+
 __host__ __device__ __forceinline__ int am_value_stride(const MixedAttnArgs& a) { return a.vs > 0 ? a.vs : a.vd; }
 
 __host__ __device__ __forceinline__ int am_value_heads(const MixedAttnArgs& a) { return a.nVH > 0 ? a.nVH : a.nKV; }
@@ -300,13 +307,12 @@ __device__ __forceinline__ float am_dot(const float* q, const float* k, int hd) 
     return acc;
 }
 
-// VEC: values in bfloat16 whose rows are 8, 16, .. 256 numbers: a lane takes eight columns of a row and the warp as many
+// VEC: values in bfloat16 whose rows are 8, 16, .. 128 numbers: a lane takes eight columns of a row and the warp as many
 // rows at a time as fit it, so that a page's values are 16-byte loads asked for together; the lanes' sums over their
 // rows meet at the end.  (One column a lane and 16 keys at a time, a page cost four trips to memory and 64 x 2 loads of
-// two bytes a lane: 4 sequences of 64 to 1,000 positions, 32 heads of 64 on 8 key heads with a table, 65 us, now 31.)
+// two bytes a lane: 4 sequences of 64 to 1,000 positions, 32 heads of 64 on 8 key heads with a table, 65 us, now 27.)
 template <typename TA, typename TC, int NACC, int GQ, bool VEC>
-__global__ void __launch_bounds__(AM_GTHREADS)
-attn_group_decode_kernel(MixedAttnArgs a) {
+__device__ __forceinline__ void am_group_decode(const MixedAttnArgs& a) {
     extern __shared__ __align__(16) float smem[];
     gl_grid_launch_dependents();
     gl_grid_wait();
@@ -475,6 +481,25 @@ attn_group_decode_kernel(MixedAttnArgs a) {
         }
     }
 }
+
+template <typename TA, typename TC, int NACC, int GQ, bool VEC>
+__global__ void __launch_bounds__(AM_GTHREADS)
+attn_group_decode_kernel(MixedAttnArgs a) { am_group_decode<TA, TC, NACC, GQ, VEC>(a); }
+
+// Blocks an SM, where the compiler's choice of registers was not the best.  The 16-byte loads asked for ahead take 179 with
+// four heads a block and 205 with eight, one block an SM.  Two fit in 128, without spills up to four heads: 32 x 1,000
+// positions, 32 heads of 64 on 8 with a table 230 -> 155 us, and what the small heads had lost against one column a lane (64 sequences
+// of 16 to 512, 8 heads of 32 on 2, 54 us then, 77 with one block) is 46.  With eight heads they spill 184 bytes and still win
+// where an SM has two blocks to run (32 x 1,000, 32 of 64 on 4 with slopes 341 -> 230 us); a grid of one block an SM at most keeps
+// its registers (1 x 500, 32 of 64 on 4 with a table 30 us, 36 with two blocks).  One column a lane, values of up to 32 numbers
+// and four heads: four blocks (16 sequences of 16 to 2,000, 12 heads of 40 on 4: 87 us with three, 56 with four).
+template <typename TA, typename TC, int NACC, int GQ>
+__global__ void __launch_bounds__(AM_GTHREADS, 4)
+attn_group_decode_four_kernel(MixedAttnArgs a) { am_group_decode<TA, TC, NACC, GQ, false>(a); }
+
+template <typename TA, typename TC, int GQ>
+__global__ void __launch_bounds__(AM_GTHREADS, 2)
+attn_group_decode_two_kernel(MixedAttnArgs a) { am_group_decode<TA, TC, 1, GQ, true>(a); }
 
 // The factors on a head's ranges' sums, by one warp: coef[s] = e^(m_s - m) / (sum of all ranges, the sink's share in it),
 // from each range's maximum and sum (ml [splits, 2]); up to 64 ranges.
@@ -704,6 +729,14 @@ static int launch_group_decode_as(const MixedAttnArgs& a, cudaStream_t stream) {
     const dim3 grid(a.nKV * (group / gq), a.B, a.splits);
     if (gq <= 1) return gl_launch(attn_group_decode_kernel<TA, TC, NACC, 1, VEC>, grid, dim3(AM_GTHREADS), smem, stream, 1, a);
     if (gq <= 2) return gl_launch(attn_group_decode_kernel<TA, TC, NACC, 2, VEC>, grid, dim3(AM_GTHREADS), smem, stream, 1, a);
+    if constexpr (VEC) {
+        if (gq > 2 && gq <= 4) return gl_launch(attn_group_decode_two_kernel<TA, TC, 4>, grid, dim3(AM_GTHREADS), smem, stream, 1, a);
+        if (gq > 4 && (long long)grid.x * grid.y * grid.z > am_sm_count())
+            return gl_launch(attn_group_decode_two_kernel<TA, TC, 8>, grid, dim3(AM_GTHREADS), smem, stream, 1, a);
+    }
+    if constexpr (!VEC && NACC == 1 && sizeof(TC) == 2) {
+        if (gq > 2 && gq <= 4) return gl_launch(attn_group_decode_four_kernel<TA, TC, NACC, 4>, grid, dim3(AM_GTHREADS), smem, stream, 1, a);
+    }
     if (gq <= 4) return gl_launch(attn_group_decode_kernel<TA, TC, NACC, 4, VEC>, grid, dim3(AM_GTHREADS), smem, stream, 1, a);
     return gl_launch(attn_group_decode_kernel<TA, TC, NACC, 8, VEC>, grid, dim3(AM_GTHREADS), smem, stream, 1, a);
 }
