@@ -67,13 +67,22 @@ struct MemoryScanArgs {
 
 // FULL: D == R * DPT and D a multiple of 4, so a thread's rows are DPT / 4 groups of four consecutive ones read
 // as float4 and no row needs a bounds check.
-// Blocks an SM, stated: left to itself the compiler gave eight rows a thread 80 registers or 125 depending on what else the
-// file held, and with two blocks an SM instead of three one token of 16 sequences took 13 % longer.
-__host__ __device__ constexpr int ms_blocks(int dpt, int kind) {
-    return dpt >= 32 ? 1 : kind == 2 ? (dpt >= 4 ? 2 : 3) : dpt >= 8 ? 3 : 4;
+// Blocks an SM, stated: left to itself the compiler gives some of these kernels half as many registers or twice as many
+// depending on what else the file holds.  Chosen by time, each kind with 1 to 64 sequences of 1, 37 and 120 tokens and seven
+// sizes from 16 x 16 x 16 to 32 x 128 x 128: the bounded forget's eight whole rows want a fourth block for their last wave (4 x
+// 120 tokens of 32 x 128 x 128: 304 us with three, 230), the delta rule few blocks and all the registers its longer token takes,
+// one or two rows of it in 32 bits excepted (1 x 37 tokens of 16 x 64 x 64 in bfloat16: 25.6 us with three, 20.5), the gated kind's
+// eight rows three (one token of 16 sequences took 13 % longer with two).  The plain decay's four rows keep four (4 x 100 tokens of
+// 8 x 128 x 256 in 32 bits 120 us, 155 with three), though where the grid is smaller than the machine they lose to more
+// registers (4 x 100 of 4 x 128 x 128: 56 us, 51 in an earlier build).
+__host__ __device__ constexpr int ms_blocks(int bytes, int dpt, int kind, bool full) {
+    if (dpt >= 32) return 1;
+    if (kind == 2) return bytes == 2 || dpt >= 4 ? 2 : 3;
+    if (kind == 1 && full) return 4;
+    return dpt >= 8 ? 3 : 4;
 }
 template <typename TA, int DPT, int KIND, bool FULL>
-__global__ void __launch_bounds__(MS_THREADS, ms_blocks(DPT, KIND))
+__global__ void __launch_bounds__(MS_THREADS, ms_blocks(sizeof(TA), DPT, KIND, FULL))
 memory_scan_kernel(MemoryScanArgs a, int R, int CH) {
     extern __shared__ __align__(16) float smem[];
     // (launched in order, not early: placed beside the kernel before, the blocks of a scan sat several to an SM
