@@ -753,7 +753,9 @@ static int launch_group_decode(const MixedAttnArgs& a, cudaStream_t stream) {
 // out[t, h, :] = sum_g M[h, g] pairs[t, g, c(h), :]   (without a table: pairs[t, h, 0, :])
 // Where the pairs' rows are whole 16-byte pieces and a value head's query heads are at most AM_MIX_HEADS, a thread takes four
 // columns of one value head for all of them: every pair is read once and not once per query head (2,128 tokens, 32 heads on
-// 8 value heads of 64: 154 us, now 36).
+// 8 value heads of 64: 154 us, now 36).  It has a sixteenth to a thirty-second of the threads, so few results are quicker by a thread
+// each (us of both kernels of a prompt, a thread a result / this: 32 heads of 64 on 8, 20 tokens 11.0 / 11.4, 160 28.7 / 24.5; 8 of
+// 16 on 4, 80 tokens 6.6 / 7.9, 320 14.7 / 12.1; 16 of 128 on 8, 40 tokens 10.8 / 11.7).
 #define AM_MIX_HEADS 8
 template <typename TA, int GROUP>
 __global__ void __launch_bounds__(256)
@@ -815,7 +817,7 @@ head_mix_kernel(MixedAttnArgs a) {
 template <typename TA>
 static int launch_head_mix(const MixedAttnArgs& a, cudaStream_t stream) {
     const int group = a.nH / a.nKV;
-    if (a.mix && group <= AM_MIX_HEADS && a.vd % 4 == 0 && ((uintptr_t)a.pairs & 15) == 0) {
+    if (a.mix && group <= AM_MIX_HEADS && a.vd % 4 == 0 && ((uintptr_t)a.pairs & 15) == 0 && a.T >= 64 && (long long)a.T * a.nH * a.vd >= 32768) {
         const long long n = (long long)a.T * a.nKV * (a.vd / 4);
         const dim3 grid((unsigned)((n + 255) / 256));
         if (group <= 2) return gl_launch(head_mix_group_kernel<TA, 2>, grid, dim3(256), 0, stream, 1, a);

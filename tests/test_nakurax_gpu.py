@@ -796,7 +796,10 @@ def test_neighbouring_dims_turned_piece_by_piece(half):
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("heads,groups,dim,vdim", [(8, 2, 64, 64), (4, 4, 16, 16), (8, 8, 64, 32), (16, 2, 32, 32), (8, 2, 16, 128),
-                                                   (3, 3, 24, 8), (6, 3, 24, 40), (4, 2, 16, 30)])
+                                                   (3, 3, 24, 8), (6, 3, 24, 40), (4, 2, 16, 30),
+                                                   # more blocks than SMs with eight heads a block; one column a lane; one and
+                                                   # two heads a value head of many results
+                                                   (24, 3, 64, 64), (12, 4, 24, 24), (16, 8, 32, 64), (16, 16, 64, 64)])
 def test_attention_with_a_table_over_the_heads(heads, groups, dim, vdim, dtype):
     """A result is a sum over all heads' weights applied to the own value head: one token a sequence with contexts cut into
     ranges (some of them empty), and prompts, with values of whole 16-byte pieces, of a power of two of them, and neither."""
