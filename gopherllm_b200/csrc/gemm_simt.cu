@@ -192,15 +192,11 @@ gemm_f32_kernel(GemmArgs g, const __grid_constant__ CUtensorMap map_a, const __g
         tma_load_2d(base + (it % STAGES) * SH::STAGE, &map_a, (kb0 + it) * FG_BK, m0, bar_full + 8 * (it % STAGES));
     };
     const int iters = kb1 - kb0;
-    // the biases of the columns this thread finishes (one, or two in turn): asked for before the wait, not behind the sums
-    constexpr int BATCH = 8, NBIAS = BN > SH::THREADS ? BN / SH::THREADS : 1;
-    static_assert(NBIAS <= 2 && BATCH % NBIAS == 0 && (SH::THREADS % BN == 0 || BN % SH::THREADS == 0), "a thread's columns repeat");
-    float my_bias[NBIAS];
-#pragma unroll
-    for (int u = 0; u < NBIAS; ++u) {
-        const int n = n0 + rank * (BN / S) + ((tid + u * SH::THREADS) & (BN / S - 1));
-        my_bias[u] = g.bias && n < g.N ? g.bias[n] : 0.f;
-    }
+    // the bias of the column this thread finishes: asked for before the wait, not behind the sums
+    constexpr int BATCH = 8;
+    static_assert(BN <= SH::THREADS && SH::THREADS % BN == 0, "a thread finishes one column");
+    const int my_n = n0 + rank * (BN / S) + (tid & (BN / S - 1));
+    const float my_bias = g.bias && my_n < g.N ? g.bias[my_n] : 0.f;
     if (tid == 0)
         for (int it = 0; it < STAGES && it < iters; ++it) load_w(it);
     gl_grid_wait();
@@ -278,6 +274,9 @@ gemm_f32_kernel(GemmArgs g, const __grid_constant__ CUtensorMap map_a, const __g
         }
         if (seg < last) put_by(seg & ~(seg + 1), put + (__ffs(seg + 1) - 1) * (BM * BN));      // what pairs with it so far
     }
+    // a wait that ran out: the copies still on their way must not land in memory that is used for something else by then
+    if (tid == 0 && !ok)
+        for (int i = it - 1; i < min(iters, it - 1 + STAGES); ++i) mbar_wait(bar_full + 8 * (i % STAGES), (i / STAGES) & 1);
     // the block's sum over its parts, where the cluster can read it
     float* tile = S == FG_SEGS ? (float*)smem : put;
     __syncthreads();                                                          // (the stages are free now)
@@ -314,7 +313,7 @@ gemm_f32_kernel(GemmArgs g, const __grid_constant__ CUtensorMap map_a, const __g
             const int e = e0 + u * SH::THREADS, m = e >> log_cols, n = n0 + rank * cols + (e & (cols - 1));
             if (e < total && n < g.N) {
                 float r = v[u];
-                if (g.bias) r += my_bias[u % NBIAS];
+                if (g.bias) r += my_bias;
                 r = gl_activate<true>(r, g.act, g.act_p0, g.act_p1);
                 if (g.add0) r += a0[u];
                 if (g.add1) r += a1[u];
@@ -491,6 +490,13 @@ static int launch_f32_short(const GemmArgs& g, cudaStream_t stream) {
     return gl_check_launch();
 }
 
+static int fg_sms() {
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms > 0 ? sms : 148;
+}
+
 // Rows of a tile: as few as hold all rows, since up to about 20 rows the weights' stream is the longer of the two and
 // beyond that every padded row costs FMA time.  The few rows' blocks are a warp each, so that enough of them fit an SM to
 // keep both the weights' stream and the FMA units busy.  From 33 rows on tiles of 64 x 128, whose shared-memory loads
@@ -508,7 +514,7 @@ static int dispatch_f32(const GemmArgs& g, cudaStream_t stream) {
     const long short_tiles = (long)((g.M + SG_BM - 1) / SG_BM) * ((g.N + SG_BN - 1) / SG_BN);
     if (g.K < 64 || (g.K <= 128 && short_tiles >= 256) || (g.K <= 256 && short_tiles >= 1024)) return launch_f32_short<TO>(g, stream);
     const long big_tiles = (long)((g.M + 63) / 64) * ((g.N + 127) / 128), k_blocks = (g.K + FG_BK - 1) / FG_BK;
-    if (g.M <= 32 || big_tiles * k_blocks < 8 * 148) return launch_f32<FgShape<1, 2, 4, 8, 4, 4>, TO>(g, stream);
+    if (g.M <= 32 || big_tiles * k_blocks < 8 * fg_sms()) return launch_f32<FgShape<1, 2, 4, 8, 4, 4>, TO>(g, stream);
     return launch_f32<FgShape<2, 2, 4, 8, 8, 3>, TO>(g, stream);
 }
 
