@@ -48,7 +48,7 @@ class StepContext:
         self.side_stream = None          # a second stream blocks may fork onto (decode steps only)
 
 
-GRAPH_F32_RUN_BYTES = 128 << 20      # weights a run of the schedule streams, up to which 32-bit decode steps are captured
+GRAPH_F32_RUN_BYTES = 128 << 20      # weights of a model for each run of its schedule, up to which 32-bit decode steps are captured
 
 
 def _pad4(n: int) -> int:
@@ -83,9 +83,10 @@ class Engine:
         self.act_dtype, self.device = act_dtype, torch.device(device)
         self.vocab = model.spec.vocab
         # Decode steps (one token per sequence) replay a CUDA graph per batch shape: always in bfloat16, in 32 bits
-        # where a run of the schedule has few weights to stream.  A run's launches take the host about 100 us; a run
-        # of more than GRAPH_F32_RUN_BYTES takes the device as long, and a capture would only cost (a step of Phi-1.5
-        # in 32 bits, 200 MB a run: 3.7 ms on the device, 2.5 ms to launch; of a model of 0.2 MB a run: 0.1 and 0.5 ms).
+        # where a run of the schedule has few weights.  A run's launches take the host 60 to 100 us; with more than
+        # GRAPH_F32_RUN_BYTES (embedding and head shared out over the runs) the device takes about as long, and a capture
+        # gains little over its cost (a step of Phi-1.5 in 32 bits, 225 MB a run: 2.35 ms, 2.0 of them to launch, and
+        # 2.17 captured; of a model of 0.3 MB a run: 0.42 and 0.10 ms).
         self.use_graphs = bool(getattr(model, "capturable", False)) and (
             act_dtype == torch.bfloat16 or model.weight_bytes() <= GRAPH_F32_RUN_BYTES * max(1, len(model.spec.schedule)))
         self.graph_max_batch = 256

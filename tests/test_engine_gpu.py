@@ -419,3 +419,37 @@ def test_captured_32_bit_steps_are_the_launched_ones():
     assert none == 0 and captured == 2
     for a, b in zip(own, rep):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("size", ["ALPHA", "BETA", "GAMMA"])
+@pytest.mark.parametrize("design", ["vopedra", "gozolix", "lilupel", "darusun", "dibedra", "nakurax"])
+def test_captured_32_bit_steps_of_every_design(design, size):
+    """The same for the designs with states, mixtures, latents and several streams, across a page's edge and as the batch
+    shrinks.  A captured step cuts the context for its bucket's longest sequence, so attention's partial sums may meet in
+    another order: 2^-24 of a sum at a time, through up to seven layers."""
+    import importlib
+    import gopherllm_b200 as gl
+    models = importlib.import_module(design + "_models")
+    cfg = getattr(models, size)
+    folder = models.write_folder(cfg, models.draw(cfg, 5))
+    rng = np.random.default_rng(7)
+    lens = [60, 3, 20]
+    seqs = [[int(t) for t in rng.integers(0, cfg["vocab"], size=n + 12)] for n in lens]
+
+    def run(graphs):
+        m = gl.load(folder, dtype="float32", max_tokens=3 * 128)
+        assert m.engine.use_graphs
+        m.engine.use_graphs = graphs
+        slots = [m.open_sequence() for _ in seqs]
+        outs = [m.step([(slots[i], seqs[i][:lens[i]]) for i in range(3)])]
+        for step in range(11):
+            outs.append(m.step([(slots[i], [seqs[i][lens[i] + step]]) for i in (range(3) if step < 7 else range(2))]))
+        captured = sum(1 for g in m.engine._graphs.values() if g)
+        m.engine.check_device()
+        m.close()
+        return outs, captured
+
+    (own, none), (rep, captured) = run(False), run(True)
+    assert none == 0 and captured == 2
+    for a, b in zip(own, rep):
+        assert (a - b).abs().max() <= 2e-5 * max(1.0, a.abs().max().item())

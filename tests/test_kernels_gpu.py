@@ -477,13 +477,30 @@ def test_attention_generic(dtype, nH, nKV, hd, window):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("nH,nKV,hd", [(4, 2, 64), (2, 2, 33), (3, 1, 256)])
-@pytest.mark.parametrize("window", [0, 100])
+@pytest.mark.parametrize("nH,nKV,hd", [(4, 2, 64), (2, 2, 33), (3, 1, 256), (4, 2, 40), (4, 4, 100), (2, 1, 36)])
+@pytest.mark.parametrize("window", [0, 100, 250])
 def test_attention_generic_one_token(dtype, nH, nKV, hd, window):
     """Sequences of one token, whose pages the warps of a block share: fewer pages than warps, more, page edges, and
     beside a sequence of several tokens."""
     run_attention("generic", dtype, nH, nKV, hd, window, [0, 63, 64, 511, 512, 1100], [1] * 6)
     run_attention("generic", dtype, nH, nKV, hd, window, [200, 30, 64], [1, 5, 1])
+    run_attention("generic", dtype, nH, nKV, hd, window, [191, 192, 255, 256], [1] * 4)
+
+
+@pytest.mark.parametrize("hd", [64, 40, 33])
+def test_attention_generic_row_does_not_depend_on_the_batch(hd):
+    """A lone token's row in 32 bits, bit for bit, alone and beside longer runs, with few pages and with many."""
+    o = ops()
+    nH, nKV, ctxs = 4, 2, [10, 300, 900, 130]
+    k, v, q = rnd(4, 901, nKV, hd, seed=1), rnd(4, 901, nKV, hd, seed=2), rnd(8, nH * hd, seed=3) * hd ** -0.5
+    kc, vc, table = make_cache(k, v, [c + 5 if c == 130 else c + 1 for c in ctxs], torch.float32)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    together = torch.empty(8, nH * hd, device=DEV)
+    o.attention_generic(q, together, kc, vc, i32([0, 1, 2, 3]), i32([1, 1, 1, 5]), i32(ctxs), table, nH, nKV, hd, 5)
+    for b in range(3):
+        alone = torch.empty(1, nH * hd, device=DEV)
+        o.attention_generic(q[b:b + 1], alone, kc, vc, i32([0]), i32([1]), i32(ctxs[b:b + 1]), table[b:b + 1].contiguous(), nH, nKV, hd, 1)
+        assert torch.equal(alone[0], together[b]), b
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])

@@ -304,6 +304,22 @@ def test_replay_of_a_trace(tmp_path):
 def test_selective_scan_forms(C, N, qlens, dtype):
     """Runs that end inside a group of tokens and inside a staged chunk, one token a sequence, states of fewer lanes than a
     group, of no power of two and too many to fetch ahead, and many sequences, against the recurrence in 64-bit."""
+    check_selective_scan(C, N, qlens, dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("tokens", [48, 128])
+@pytest.mark.parametrize("C,N,qlens", [(40, 16, [50, 129, 300, 1]), (24, 40, [300, 50, 129]), (3000, 16, [128, 257])])
+def test_selective_scan_in_chunks_of_several_stages(C, N, qlens, tokens, dtype, monkeypatch):
+    """Chunks as long as those of long prompts, so that inputs fetched ahead cross a chunk's stages: ragged last stages and last
+    chunks, runs of one chunk and of many, states that are fetched ahead and states that are not."""
+    from gopherllm_b200 import ops
+    monkeypatch.setattr(ops, "SCAN_CHUNKED_FROM", 64)
+    monkeypatch.setattr(ops, "SCAN_CHUNK_TOKENS", tokens)
+    check_selective_scan(C, N, qlens, dtype)
+
+
+def check_selective_scan(C, N, qlens, dtype):
     from types import SimpleNamespace
     from gopherllm_b200 import ops
     g = torch.Generator().manual_seed(C + N)
