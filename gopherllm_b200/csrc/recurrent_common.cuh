@@ -29,3 +29,30 @@ __device__ __forceinline__ float rc_decay(float x) {
     if (x > -0.5f) return 1.0f + expm1f(x);
     return expf(x);
 }
+
+// 16 bytes of a row (4 floats or 8 bfloat16) as floats; both addresses 16-byte aligned
+__device__ __forceinline__ void mc_load16(const float* src, float* dst) {
+    *reinterpret_cast<float4*>(dst) = *reinterpret_cast<const float4*>(src);
+}
+__device__ __forceinline__ void mc_load16(const __nv_bfloat16* src, float* dst) {
+    const uint4 raw = *reinterpret_cast<const uint4*>(src);
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+    const float2 f0 = __bfloat1622float2(h[0]), f1 = __bfloat1622float2(h[1]);
+    const float2 f2 = __bfloat1622float2(h[2]), f3 = __bfloat1622float2(h[3]);
+    reinterpret_cast<float4*>(dst)[0] = make_float4(f0.x, f0.y, f1.x, f1.y);
+    reinterpret_cast<float4*>(dst)[1] = make_float4(f2.x, f2.y, f3.x, f3.y);
+}
+
+// 4 or 8 floats as 16 bytes of a row
+__device__ __forceinline__ void mc_store16(float* dst, const float* v) {
+    *reinterpret_cast<float4*>(dst) = *reinterpret_cast<const float4*>(v);
+}
+__device__ __forceinline__ void mc_store16(__nv_bfloat16* dst, const float* v) {
+    uint4 raw;
+    __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&raw);
+    h[0] = __floats2bfloat162_rn(v[0], v[1]);
+    h[1] = __floats2bfloat162_rn(v[2], v[3]);
+    h[2] = __floats2bfloat162_rn(v[4], v[5]);
+    h[3] = __floats2bfloat162_rn(v[6], v[7]);
+    *reinterpret_cast<uint4*>(dst) = raw;
+}

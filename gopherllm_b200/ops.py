@@ -1352,7 +1352,7 @@ def memory_scan(kind: int, proj: torch.Tensor, state: torch.Tensor, ctx, H: int,
                              _addr(sin) if rot_half else None, _addr(skip) if plain else None,
                              gates.shape[1] if plain and gates is not None else 0, kv_heads if plain else 0, rot_half,
                              k_scale)
-        fn = _lib("recurrent.cu").gl_memory_chunks
+        fn = _lib("memory_chunks.cu").gl_memory_chunks
         _check(_launch(fn, byref(c), c_int(dtype_code(proj.dtype)), _stream()), "memory_chunks",
                7 if gated else 5 if plain else 4)
         return out
