@@ -1212,7 +1212,7 @@ MEMORY_CHUNKS_MAX_ROWS = 128     # rows a head the chunked walk of the matrix me
 USE_MEMORY_CHUNKS = True
 # The gated and the bounded-forget memories walk a run token by token or as chunks side by side.  In 32 bits the order of
 # a state's sums follows the longest run alone and not how many sequences run beside it: chunks of SCAN_CHUNK_TOKENS from
-# SCAN_CHUNKED_FROM tokens on.  In bfloat16 also shorter runs, where chunks are expected to take clearly less time, and
+# SCAN_CHUNKED_FROM tokens on.  In bfloat16 also shorter runs, where chunks are expected to take less time, and
 # shorter chunks: the order of the (32-bit) sums then depends on the lengths of all the step's runs.
 # Token by token a launch takes as long as its longest run, or with many sequences as long as the machine needs for all
 # of them (near the line something of both); in chunks it takes some time for its passes and for every sequence, and the
@@ -1220,12 +1220,13 @@ USE_MEMORY_CHUNKS = True
 # passes' us; the same rate in chunks), fitted to runs of 200 to 2,040 tokens, 1 to 16 sequences.  us a launch, one
 # piece / chunks, of a memory of 8 x 128 x 256: 1 x 1,000 tokens 503 / 250, 1 x 500 257 / 145, 4 of 64 to 1,000 800 / 470,
 # 8 of 100 to 500 637 / 639, 16 x 500 1788 / 1813; of 32 x 32 x 64: 345 / 177, 177 / 120, 498 / 273, 342 / 279, 505 / 796.
-# MEMORY_CHUNK_GAIN: over nine memories of 1,024 to 524,288 elements and 22 batches of 1 to 17 runs of 64 to 1,000 tokens
-# chunks lost up to 14 % in 4 of the 48 cases where the expected gain was below 15 % (16 x 500 tokens of 32 x 128 x 128:
-# 2923 / 3381 us), and won 16 % to 6.8 times in the 172 where it was more.
+# Over nine memories of 1,024 to 524,288 elements and 22 batches of 1 to 17 runs of 100 to 1,000 tokens the chosen form was the
+# slower one, by up to 14 %, for runs shorter than those of the fit (1 x 150 tokens of 4 x 128 x 128: 75 / 82 us) and near the
+# line of the largest memory (16 x 500 of 32 x 128 x 128: 2923 / 3381 us), which therefore wants a clearer gain.
+MEMORY_CHUNKED_FROM = 200
+MEMORY_CHUNK_LARGE, MEMORY_CHUNK_LARGE_GAIN = 1 << 19, 1.08
 MEMORY_CHUNK_COST = {0: (0.5, 1.17e6, 55.0, 1.2e6), 1: (0.35, 1.04e6, 50.0, 0.8e6)}
 MEMORY_CHUNK_SEQUENCE = 8.0
-MEMORY_CHUNK_GAIN = 1.15
 # Chunks of 64 tokens, of 32 where the tokens are few (1 x 1,000 tokens 237 and 218 us with 64, 242 and 190 with 32; 1 x 500
 # 173 and 168, 133 and 132; 1 x 2,040 468 and 320, 474 and 340, and 469 and 399 with 128).
 MEMORY_CHUNK_TOKENS, MEMORY_CHUNK_TOKENS_FEW, MEMORY_CHUNK_FEW_TOKENS = 64, 32, 1200
@@ -1233,11 +1234,14 @@ MEMORY_CHUNK_TOKENS, MEMORY_CHUNK_TOKENS_FEW, MEMORY_CHUNK_FEW_TOKENS = 64, 32, 
 
 def memory_walks_chunks(kind: int, n_seqs: int, tokens: int, longest: int, elements: int) -> bool:
     """Whether a gated or a bounded-forget memory of ``elements`` numbers is expected to walk a step's runs (``tokens`` in
-    all) in chunks in clearly less time."""
+    all) in chunks in less time."""
+    if longest < MEMORY_CHUNKED_FROM:
+        return False
     a_token, rate, passes, chunk_rate = MEMORY_CHUNK_COST[kind]
     run, all_runs = a_token * longest, tokens * elements / rate
     chunks = passes + MEMORY_CHUNK_SEQUENCE * n_seqs + tokens * elements / chunk_rate
-    return max(run, all_runs) + 0.5 * min(run, all_runs) > MEMORY_CHUNK_GAIN * chunks
+    gain = MEMORY_CHUNK_LARGE_GAIN if elements >= MEMORY_CHUNK_LARGE else 1.0
+    return max(run, all_runs) + 0.5 * min(run, all_runs) > gain * chunks
 
 
 def memory_chunk_tokens(kind: int, exact: bool, n_seqs: int, tokens: int, longest: int, H: int, D: int, V: int) -> int:
