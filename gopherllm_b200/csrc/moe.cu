@@ -802,15 +802,16 @@ moe_expert_tc_kernel(ExpertArgs a) {
 #define MV_WARPS(gated) ((gated) ? 8 : 4)
 
 template <bool GATED>
-__global__ void __launch_bounds__(MV_WARPS(GATED) * 32)
+__global__ void __launch_bounds__(MV_WARPS(GATED) * 32, GATED ? 2 : 4)      // (16 warps an SM with both rows' pieces in registers)
 moe_expert_rows_kernel(ExpertArgs a) {
     __shared__ __align__(16) __nv_bfloat16 xs[MV_ROWS][MV_KCH];
     __shared__ int rows[MOE_TM];
     gl_grid_launch_dependents();
     gl_grid_wait();
     const int tile = blockIdx.y;
-    if (tile >= *a.n_tiles) return;
-    const int e = a.tile_expert[tile], start = a.tile_start[tile], nrows = a.tile_rows[tile];
+    // (asked for together: the arrays have an entry for every tile of the grid)
+    const int tiles = *a.n_tiles, e = a.tile_expert[tile], start = a.tile_start[tile], nrows = a.tile_rows[tile];
+    if (tile >= tiles) return;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (tid < MOE_TM) rows[tid] = tid < nrows ? (GATED ? a.order[start + tid] / a.top : start + tid) : -1;
     __syncthreads();
@@ -827,26 +828,29 @@ moe_expert_rows_kernel(ExpertArgs a) {
         for (int r = 0; r < MV_ROWS; ++r) acc0[r] = acc1[r] = 0.f;
         for (int k0 = 0; k0 < a.K; k0 += MV_KCH) {
             const int kn = min(MV_KCH, a.K - k0);
-            // A lane's first pieces of both weight rows are asked for before the tokens' rows are staged: the trip to
-            // memory runs under the staging, and after it the next pieces' under the arithmetic of this step.
+            // A lane's pieces of both weight rows, 2,048 columns of them, are asked for together and before the tokens' rows
+            // are staged: with one piece ahead a warp went to memory eight times in a row, which was the kernel's time
+            // (4 of 32 experts of 1,344 x 2,048 a token, the plan and the sum of the choices included: 1 token 33 -> 24 us, 4 74 -> 58, 16 175 -> 146).
             const uint4 none = make_uint4(0, 0, 0, 0);
-            uint4 next0 = lane * 8 < kn ? *(const uint4*)(w0 + k0 + lane * 8) : none;
-            uint4 next1 = lane * 8 < kn ? *(const uint4*)(w1 + k0 + lane * 8) : none;
+            uint4 ra[MV_KCH / 256], rb[MV_KCH / 256];
+#pragma unroll
+            for (int p = 0; p < MV_KCH / 256; ++p) {
+                const int k = p * 256 + lane * 8;
+                ra[p] = k < kn ? __ldcs((const uint4*)(w0 + k0 + k)) : none;
+                rb[p] = k < kn ? __ldcs((const uint4*)(w1 + k0 + k)) : none;
+            }
             __syncthreads();
             for (int el = tid; el < nr * (kn / 8); el += MV_WARPS(GATED) * 32) {
                 const int r = el / (kn / 8), c = (el - r * (kn / 8)) * 8;
                 *(uint4*)&xs[r][c] = *(const uint4*)(X + (size_t)rows[r0 + r] * a.K + k0 + c);
             }
             __syncthreads();
-#pragma unroll 2
-            for (int k = lane * 8; k < kn; k += 256) {
-                const uint4 ra = next0, rb = next1;
-                if (k + 256 < kn) {
-                    next0 = *(const uint4*)(w0 + k0 + k + 256);
-                    next1 = *(const uint4*)(w1 + k0 + k + 256);
-                }
-                const __nv_bfloat162* pa = (const __nv_bfloat162*)&ra;
-                const __nv_bfloat162* pb = (const __nv_bfloat162*)&rb;
+#pragma unroll
+            for (int p = 0; p < MV_KCH / 256; ++p) {
+                const int k = p * 256 + lane * 8;
+                if (k >= kn) break;
+                const __nv_bfloat162* pa = (const __nv_bfloat162*)&ra[p];
+                const __nv_bfloat162* pb = (const __nv_bfloat162*)&rb[p];
                 float wa[8], wb[8];
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
