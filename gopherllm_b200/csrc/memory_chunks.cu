@@ -24,7 +24,7 @@ struct MemoryChunkArgs {
     const void* proj;         // [T, ld] activation type
     float* out;               // [T, H*V] raw S^T q
     float* nq;                // gated: [T, H] n.q
-    float* gates;             // gated: [T, H, 4]: log input gate, log forget gate -> keep, take, e^-m, unused
+    float* gates;             // gated: [T, H, 4]: log input gate, log forget gate -> keep, take, e^-m, log keep
     float* state;             // [slots, state_stride]: S [H, D, V], gated: n [H, D], m [H]
     const float* lower;       // bounded forget: [H*D]
     float* chunk_state;       // [B, n_chunks, H, D, cols]
@@ -88,6 +88,7 @@ memory_gate_walk_kernel(MemoryChunkArgs a) {
         }
         if (ok) {
             g[0] = rc_decay(gf + m_old - m_mine);
+            g[3] = gf + m_old - m_mine;
             g[1] = expf(gi - m_mine);
             g[2] = expf(-m_mine);
         }
@@ -95,7 +96,7 @@ memory_gate_walk_kernel(MemoryChunkArgs a) {
     if (lane == 0) *m_g = m;
 }
 
-// the plain decay's keep and take of every token: gates[t, h, 0] = keep, gates[t, h, 1] = take
+// the plain decay's keep and take of every token: gates[t, h, 0] = keep, gates[t, h, 1] = take, gates[t, h, 3] = log keep
 template <typename TA>
 __global__ void __launch_bounds__(256)
 memory_decay_gates_kernel(MemoryChunkArgs a) {
@@ -104,13 +105,17 @@ memory_decay_gates_kernel(MemoryChunkArgs a) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (long long)a.T * a.H) return;
     const int t = (int)(i / a.H), h = (int)(i - (long long)t * a.H);
-    float take = 1.0f, keep = a.lower ? a.lower[h] : 1.0f;
+    float take = 1.0f, keep = a.lower ? a.lower[h] : 1.0f, log_keep = 0.f;
     if (a.gates_in) {
         take = rc_softplus(gl_load((const TA*)a.gates_in + (size_t)t * a.gates_ld + a.f_off + h) + a.dt_bias[h]);
-        keep = rc_decay(-expf(a.a_log[h]) * take);
+        log_keep = -expf(a.a_log[h]) * take;
+        keep = rc_decay(log_keep);
+    } else if (a.lower) {
+        log_keep = (float)log((double)keep);
     }
     a.gates[i * 4 + 0] = keep;
     a.gates[i * 4 + 1] = take;
+    a.gates[i * 4 + 3] = log_keep;
 }
 
 // the product of a chunk's decays per row
@@ -131,28 +136,6 @@ memory_chunk_decay_kernel(MemoryChunkArgs a) {
         else p *= l + (1.0f - l) * rc_sigmoid(gl_load((const TA*)a.proj + (size_t)(qstart + s) * a.ld + a.f_off + h * a.D + d));
     }
     a.chunk_decay[(((size_t)b * a.n_chunks + chunk) * a.H + h) * a.D + d] = p;
-}
-
-// two 32-bit multiply-adds in one instruction (the pair's halves are independent and rounded like fmaf's)
-__device__ __forceinline__ unsigned long long mc_pack(float x, float y) {
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
-    return r;
-}
-__device__ __forceinline__ unsigned long long mc_fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-    unsigned long long r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ unsigned long long mc_mul2(unsigned long long a, unsigned long long b) {
-    unsigned long long r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ float2 mc_unpack(unsigned long long v) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
 }
 
 // MODE 1: from zero, keep the last state.  MODE 2: from the chunk's start, with outputs.  NT: threads (columns) a block.
@@ -373,6 +356,546 @@ memory_chunk_carry_kernel(MemoryChunkArgs a) {
     }
 }
 
+// ---------------------------------------------------------------------------
+// The scalar-decay memories' chunks (gated kind and plain decay) as matrix products, for bfloat16 inputs.
+//
+// With one decay a (token, head), the tokens of a chunk meet in closed form.  L_t = keep_1 .. keep_t within the chunk,
+// S_0 the state the chunk starts from:
+//   o_t  = L_t S_0^T q_t + sum_{s <= t} (L_t / L_s) take_s (q_t . k_s) v_s,
+//   S_C  = L_C S_0 + sum_s (L_C / L_s) take_s k_s v_s^T,
+// products of 64 x 64 x D, 64 x D x V and D x 64 x V numbers a chunk and head instead of a walk over its tokens.
+//
+// Nothing is computed with fewer bits than in the walk.  q, k and v are bfloat16 and enter exactly; what is a 32-bit number
+// (the weighted keys, the weighted scores, the state, keys and queries after a rotation) enters as a sum of three bfloat16
+// numbers, 24 bits, and each of the three is multiplied.  The products accumulate in 32 bits; since the tensor cores cut off
+// what an addition cannot hold instead of rounding it, a product's 16 terms (its parts, smallest first) are summed from zero and
+// the sums added in registers: accumulated in place the error was three times the walk's.  L_t / L_s is e to the
+// difference of sums of logarithms; the sums are taken in 64-bit, so that a token that forgets nearly everything leaves the
+// later ones' decays as exact as they were.
+//
+// What bounds it: the tensor cores' mma.sync (about 2,200 products of 16 x 8 x 16 a chunk and head of 128 x 64), then the
+// trips of chunk states through memory.  Token by token on CUDA cores the same took six times the arithmetic instructions.
+// With 64 heads of 128 x 64, a run of 2,047 tokens: 426 -> 166 us; 16 heads of 64 x 128 with a rotation 122 -> 78; gated, 8 heads of
+// 128 x 256, runs of 64, 376, 688 and 1,000 tokens 413 -> 120.  Relative error of the results against 64 bits, walk and
+// products: 3.9e-8 and 3.4e-8, fixed decays 2.2e-7 and 1.7e-7, rotated 5.4e-8 and 5.7e-8, gated 2.5e-7 and 1.3e-7.
+//
+// A value that is infinite or NaN reaches its column from its token on and nothing before it (a zero weight times infinity
+// would be NaN in the tokens before): such values are taken out of the products and their column is NaN from there on.
+#define MT_TOKENS 64                 // tokens of a chunk, at most
+#define MT_COLS 64                   // columns of a block
+#define MT_VP (MT_COLS + 8)          // pitches in elements: rows of 16-byte pieces on different banks
+#define MT_LOG_MIN -200.f            // e^-200 is zero in 32 bits: a keep of zero keeps its logarithm finite
+
+__device__ __forceinline__ void mt_ldm4(unsigned addr, unsigned (&r)[4]) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ void mt_ldm4t(unsigned addr, unsigned (&r)[4]) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ void mt_mma(float (&d)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void mt_add(float (&d)[4], const float (&f)[4]) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) d[e] += f[e];
+}
+// two 32-bit numbers as three pairs of bfloat16: x = p0.x + p1.x + p2.x up to the last of 24 bits
+__device__ __forceinline__ void mt_split2(float x, float y, unsigned& p0, unsigned& p1, unsigned& p2) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+    const float2 hf = __bfloat1622float2(h);
+    x -= hf.x; y -= hf.y;
+    const __nv_bfloat162 m = __floats2bfloat162_rn(x, y);
+    const float2 mf = __bfloat1622float2(m);
+    const __nv_bfloat162 l = __floats2bfloat162_rn(x - mf.x, y - mf.y);
+    p0 = *(const unsigned*)&h; p1 = *(const unsigned*)&m; p2 = *(const unsigned*)&l;
+}
+__device__ __forceinline__ void mt_unpack8(const uint4& raw, float (&f)[8]) {
+    const __nv_bfloat162* h = (const __nv_bfloat162*)&raw;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { const float2 v = __bfloat1622float2(h[i]); f[2 * i] = v.x; f[2 * i + 1] = v.y; }
+}
+// eight 32-bit numbers into the three planes of a tile, 16 bytes a plane
+__device__ __forceinline__ void mt_put8(const float (&f)[8], __nv_bfloat16* dst, int plane) {
+    uint4 p[3];
+    mt_split2(f[0], f[1], p[0].x, p[1].x, p[2].x);
+    mt_split2(f[2], f[3], p[0].y, p[1].y, p[2].y);
+    mt_split2(f[4], f[5], p[0].z, p[1].z, p[2].z);
+    mt_split2(f[6], f[7], p[0].w, p[1].w, p[2].w);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) *(uint4*)(dst + (size_t)i * plane) = p[i];
+}
+
+// the first warp: the sums of the logarithms of keep up to each of a chunk's n tokens, and take (zero behind the n-th)
+__device__ __forceinline__ void mt_gates(const MemoryChunkArgs& a, int h, int t_first, int n, double* cum, float* take) {
+    if (threadIdx.x >= 32) return;
+    const int lane = threadIdx.x;
+    double x[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int s = 2 * lane + i;
+        const float* g = a.gates + ((size_t)(t_first + min(s, n - 1)) * a.H + h) * 4;
+        const float l = g[3];
+        x[i] = s < n ? (double)(l < MT_LOG_MIN ? MT_LOG_MIN : l) : 0.0;
+        take[s] = s < n ? g[1] : 0.f;
+    }
+    double sum = x[0] + x[1];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const double up = __shfl_up_sync(0xffffffffu, sum, o);
+        if (lane >= o) sum += up;
+    }
+    cum[2 * lane + 1] = sum;
+    cum[2 * lane] = sum - x[1];
+}
+
+// A block's share of the rows [0, n) of q or k (column ``off`` of proj on): all of a thread's pieces are asked for at once (load),
+// then turned by their positions where the kind does that and handed to put(row, first dim, eight 32-bit numbers); rows
+// behind the n-th are zeros.
+template <int D, bool ROT, int THREADS>
+struct MtRows {
+    static constexpr int P = D / 8, IT = MT_TOKENS * P / THREADS;
+    uint4 raw[IT], partner[ROT ? IT : 1];
+    __device__ __forceinline__ void load(const MemoryChunkArgs& a, int off, int t_first, int n) {
+        const int half = ROT ? a.rot_half / 8 : 0;                  // pieces of a half of the rotated dims
+#pragma unroll
+        for (int i = 0; i < IT; ++i) {
+            const int e = threadIdx.x + i * THREADS, s = e / P, p = e - s * P;
+            const __nv_bfloat16* row = (const __nv_bfloat16*)a.proj + (size_t)(t_first + s) * a.ld + off;
+            raw[i] = s < n ? *(const uint4*)(row + p * 8) : make_uint4(0, 0, 0, 0);
+            if constexpr (ROT) partner[i] = s < n && p < half ? *(const uint4*)(row + (p + half) * 8) : make_uint4(0, 0, 0, 0);
+        }
+    }
+    template <typename Put>
+    __device__ __forceinline__ void each(const MemoryChunkArgs& a, int t_first, int n, const Put& put) const {
+        const int half = ROT ? a.rot_half / 8 : 0;
+#pragma unroll
+        for (int i = 0; i < IT; ++i) {
+            const int e = threadIdx.x + i * THREADS, s = e / P, p = e - s * P;
+            if (ROT && p >= half && p < 2 * half) continue;         // (comes with its partner)
+            float u[8];
+            mt_unpack8(raw[i], u);
+            if (ROT && p < half) {
+                float v[8], x[8], y[8];
+                mt_unpack8(partner[i], v);
+                const size_t at = (size_t)(t_first + min(s, n - 1)) * a.rot_half + p * 8;
+                const float *cs = a.cosv + at, *sn = a.sinv + at;
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    x[k] = u[k] * cs[k] - v[k] * sn[k];
+                    y[k] = v[k] * cs[k] + u[k] * sn[k];
+                }
+                put(s, p * 8, x);
+                put(s, (p + half) * 8, y);
+            } else {
+                put(s, p * 8, u);
+            }
+        }
+    }
+    // the pieces as they are
+    __device__ __forceinline__ void copy(__nv_bfloat16* to, int pitch) const {
+#pragma unroll
+        for (int i = 0; i < IT; ++i) {
+            const int e = threadIdx.x + i * THREADS, s = e / P, p = e - s * P;
+            *(uint4*)(to + s * pitch + p * 8) = raw[i];
+        }
+    }
+};
+// the same of a block's columns of v
+template <int THREADS>
+struct MtValues {
+    static constexpr int P = MT_COLS / 8, IT = MT_TOKENS * P / THREADS;
+    uint4 raw[IT];
+    __device__ __forceinline__ void load(const MemoryChunkArgs& a, int h, int col0, int t_first, int n) {
+#pragma unroll
+        for (int i = 0; i < IT; ++i) {
+            const int e = threadIdx.x + i * THREADS, s = e / P, j = col0 + (e - s * P) * 8;
+            raw[i] = s < n && j < a.V ? *(const uint4*)((const __nv_bfloat16*)a.proj + (size_t)(t_first + s) * a.ld + a.v_off + h * a.V + j)
+                                      : make_uint4(0, 0, 0, 0);
+        }
+    }
+};
+
+// the chunk states' layout here: S [D, V], then (gated kind) n [D]
+__device__ __forceinline__ float* mt_chunk_state(const MemoryChunkArgs& a, int b, int chunk, int h) {
+    return a.chunk_state + (((size_t)b * a.n_chunks + chunk) * a.H + h) * a.D * a.cols;
+}
+
+template <int D>
+static constexpr size_t mt_states_smem() { return (size_t)(3 * MT_TOKENS * (D + 8) + MT_TOKENS * MT_VP) * 2; }
+
+// every chunk from a zero state: sum_s (L_C / L_s) take_s k_s v_s^T, and the product of its decays
+template <int D, bool ROT, bool GATED>
+__global__ void __launch_bounds__(128)
+memory_chunk_states_tc_kernel(MemoryChunkArgs a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ double cum[MT_TOKENS];
+    __shared__ float take[MT_TOKENS], weight[MT_TOKENS];
+    constexpr int KP = D + 8, PLANE = MT_TOKENS * KP;
+    __nv_bfloat16* wk = (__nv_bfloat16*)smem_raw;                   // [3][tokens][D]
+    __nv_bfloat16* vs = wk + 3 * PLANE;                             // [tokens][columns]
+    gl_grid_wait();
+    const int b = blockIdx.z / a.n_chunks, chunk = blockIdx.z - b * a.n_chunks, h = blockIdx.y;
+    const int col0 = blockIdx.x * MT_COLS, V = a.V;
+    const int qlen = a.seq_qlen[b], t_first = a.seq_qstart[b] + chunk * a.chunk_len;
+    const int n = min(a.chunk_len, qlen - chunk * a.chunk_len);
+    if (n <= 0) return;
+    const int kh = GATED ? h : h / (a.H / a.KVH);
+    MtRows<D, ROT, 128> keys;
+    MtValues<128> values;
+    keys.load(a, a.k_off + kh * D, t_first, n);
+    values.load(a, h, col0, t_first, n);
+    mt_gates(a, h, t_first, n, cum, take);
+#pragma unroll
+    for (int i = 0; i < values.IT; ++i) {
+        const int e = threadIdx.x + i * 128, s = e / values.P;
+        *(uint4*)(vs + s * MT_VP + (e - s * values.P) * 8) = values.raw[i];
+    }
+    __syncthreads();
+    if (threadIdx.x < MT_TOKENS)                                    // (the weights enter a long sum: e in 64-bit, rounded once)
+        weight[threadIdx.x] = (float)(exp(cum[n - 1] - cum[threadIdx.x]) * (double)take[threadIdx.x] * (GATED ? 1.0 : (double)a.k_scale));
+    __syncthreads();
+    keys.each(a, t_first, n, [&](int s, int d, const float (&f)[8]) {
+        float y[8];
+        const float w = weight[s];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) y[i] = s < n ? w * f[i] : 0.f;
+        mt_put8(y, wk + s * KP + d, PLANE);
+    });
+    __syncthreads();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, grp = lane >> 2, tq = lane & 3;
+    constexpr int MT = D / 64;                                      // tiles of 16 rows a warp
+    float acc[MT][8][4];
+#pragma unroll
+    for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.f;
+    const unsigned wk0 = (unsigned)__cvta_generic_to_shared(wk), vs0 = (unsigned)__cvta_generic_to_shared(vs);
+    for (int ks = 0; ks * 16 < n; ++ks) {
+        unsigned bf[4][4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            mt_ldm4t(vs0 + ((ks * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * MT_VP + j * 16 + (lane >> 4) * 8) * 2, bf[j]);
+#pragma unroll
+        for (int i = 0; i < MT; ++i) {
+            float f[8][4] = {};
+#pragma unroll
+            for (int p = 2; p >= 0; --p) {
+                unsigned af[4];
+                mt_ldm4t(wk0 + (p * PLANE + (ks * 16 + (lane & 7) + (lane >> 4) * 8) * KP + (warp * MT + i) * 16 + ((lane >> 3) & 1) * 8) * 2, af);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) mt_mma(f[j], af, bf[j >> 1][(j & 1) * 2], bf[j >> 1][(j & 1) * 2 + 1]);
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j) mt_add(acc[i][j], f[j]);
+        }
+    }
+    float* cs = mt_chunk_state(a, b, chunk, h);
+#pragma unroll
+    for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int d = (warp * MT + i) * 16 + grp, col = col0 + j * 8 + 2 * tq;
+            if (col < V) {                                          // (V is whole pieces of 8)
+                *(float2*)(cs + (size_t)d * V + col) = make_float2(acc[i][j][0], acc[i][j][1]);
+                *(float2*)(cs + (size_t)(d + 8) * V + col) = make_float2(acc[i][j][2], acc[i][j][3]);
+            }
+        }
+    if (blockIdx.x != 0) return;
+    if (GATED && threadIdx.x < D) {
+        float sum = 0.f;
+        for (int s = 0; s < n; ++s) {
+            const __nv_bfloat16* w = wk + s * KP + threadIdx.x;
+            sum += __bfloat162float(w[0]) + (__bfloat162float(w[PLANE]) + __bfloat162float(w[2 * PLANE]));
+        }
+        cs[(size_t)D * V + threadIdx.x] = sum;
+    }
+    if (threadIdx.x == 0) a.chunk_decay[(((size_t)b * a.n_chunks + chunk) * a.H + h) * D] = (float)exp(cum[n - 1]);
+}
+
+// every chunk's start state from the run's start state and what the chunks add, and the run's last state
+__global__ void __launch_bounds__(128)
+memory_chunk_carry4_kernel(MemoryChunkArgs a) {
+    gl_grid_launch_dependents();
+    gl_grid_wait();
+    const int b = blockIdx.z, h = blockIdx.y;
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) * 4, DV = a.D * a.V;
+    if (i >= a.D * a.cols) return;
+    float* srow = a.state + (size_t)a.seq_slot[b] * a.state_stride;
+    float* mine = i < DV ? srow + (size_t)h * DV + i : srow + (size_t)a.H * DV + (size_t)h * a.D + (i - DV);
+    float S[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) S[k] = mine[k];                     // (a slot's row begins anywhere)
+    const int chunks = (a.seq_qlen[b] + a.chunk_len - 1) / a.chunk_len;
+    for (int k0 = 0; k0 < chunks; k0 += 8) {
+        float4 last[8];
+        float decay[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int c = min(k0 + j, chunks - 1);
+            last[j] = *(const float4*)(mt_chunk_state(a, b, c, h) + i);
+            decay[j] = a.chunk_decay[(((size_t)b * a.n_chunks + c) * a.H + h) * a.D];
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            if (k0 + j < chunks) {
+                *(float4*)(mt_chunk_state(a, b, k0 + j, h) + i) = make_float4(S[0], S[1], S[2], S[3]);
+                S[0] = fmaf(decay[j], S[0], last[j].x); S[1] = fmaf(decay[j], S[1], last[j].y);
+                S[2] = fmaf(decay[j], S[2], last[j].z); S[3] = fmaf(decay[j], S[3], last[j].w);
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) mine[k] = S[k];
+}
+
+template <int D, bool ROT>
+static constexpr size_t mt_outputs_smem() {
+    return (size_t)((ROT ? 6 : 2) * MT_TOKENS * (D + 8) + MT_TOKENS * MT_VP + 3 * D * MT_VP) * 2;
+}
+
+// the read-outs of a chunk from its start state, 64 columns a block: eight warps, 16 tokens and 32 columns each (both of a row
+// group's warps take its scores, which are few beside the state's products)
+template <int D, bool ROT, bool GATED>
+__global__ void __launch_bounds__(256, 2)
+memory_chunk_outputs_tc_kernel(MemoryChunkArgs a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ double cum[MT_TOKENS];
+    __shared__ float take[MT_TOKENS], n0[GATED ? D : 1];
+    __shared__ int bad[MT_COLS];                                    // a column's first token whose value is not finite
+    constexpr int KP = D + 8, PLANE = MT_TOKENS * KP, TQ = ROT ? 3 : 1, SPLANE = D * MT_VP;
+    __nv_bfloat16* qs = (__nv_bfloat16*)smem_raw;                   // [TQ][tokens][D]
+    __nv_bfloat16* ks = qs + TQ * PLANE;
+    __nv_bfloat16* vs = ks + TQ * PLANE;                            // [tokens][columns]
+    __nv_bfloat16* ss = vs + MT_TOKENS * MT_VP;                     // [3][D][columns]
+    gl_grid_wait();
+    const int b = blockIdx.z / a.n_chunks, chunk = blockIdx.z - b * a.n_chunks, h = blockIdx.y;
+    const int col0 = blockIdx.x * MT_COLS, V = a.V;
+    const int qlen = a.seq_qlen[b], t_first = a.seq_qstart[b] + chunk * a.chunk_len;
+    const int n = min(a.chunk_len, qlen - chunk * a.chunk_len);
+    if (n <= 0) return;
+    const int kh = GATED ? h : h / (a.H / a.KVH);
+    const float* cs = mt_chunk_state(a, b, chunk, h);
+    // everything the block reads is asked for before any of it is used
+    MtRows<D, ROT, 256> queries, keys;
+    MtValues<256> values;
+    float4 start[D * MT_COLS / 1024];
+    queries.load(a, a.q_off + kh * D, t_first, n);
+    keys.load(a, a.k_off + kh * D, t_first, n);
+    values.load(a, h, col0, t_first, n);
+#pragma unroll
+    for (int i = 0; i < D * MT_COLS / 1024; ++i) {
+        const int e = threadIdx.x + i * 256, d = e / (MT_COLS / 4), j = col0 + (e - d * (MT_COLS / 4)) * 4;
+        start[i] = j < V ? *(const float4*)(cs + (size_t)d * V + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    if (GATED && threadIdx.x < D) n0[threadIdx.x] = cs[(size_t)D * V + threadIdx.x];
+    if (threadIdx.x < MT_COLS) bad[threadIdx.x] = MT_TOKENS;
+    mt_gates(a, h, t_first, n, cum, take);
+    if constexpr (ROT) {
+        queries.each(a, t_first, n, [&](int s, int d, const float (&f)[8]) { mt_put8(f, qs + s * KP + d, PLANE); });
+        keys.each(a, t_first, n, [&](int s, int d, const float (&f)[8]) { mt_put8(f, ks + s * KP + d, PLANE); });
+    } else {
+        queries.copy(qs, KP);
+        keys.copy(ks, KP);
+    }
+#pragma unroll
+    for (int i = 0; i < D * MT_COLS / 1024; ++i) {
+        const int e = threadIdx.x + i * 256, d = e / (MT_COLS / 4), j = (e - d * (MT_COLS / 4)) * 4;
+        uint2 p[3];
+        mt_split2(start[i].x, start[i].y, p[0].x, p[1].x, p[2].x);
+        mt_split2(start[i].z, start[i].w, p[0].y, p[1].y, p[2].y);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) *(uint2*)(ss + k * SPLANE + d * MT_VP + j) = p[k];
+    }
+    __syncthreads();                                                // (``bad`` is set before anyone lowers it)
+#pragma unroll
+    for (int i = 0; i < values.IT; ++i) {
+        const int e = threadIdx.x + i * 256, s = e / values.P, j = (e - s * values.P) * 8;
+        unsigned x[4] = {values.raw[i].x, values.raw[i].y, values.raw[i].z, values.raw[i].w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if ((x[k] & 0x7f80u) == 0x7f80u) { x[k] &= 0xffff0000u; atomicMin(&bad[j + 2 * k], s); }
+            if ((x[k] & 0x7f800000u) == 0x7f800000u) { x[k] &= 0xffffu; atomicMin(&bad[j + 2 * k + 1], s); }
+        }
+        *(uint4*)(vs + s * MT_VP + j) = make_uint4(x[0], x[1], x[2], x[3]);
+    }
+    __syncthreads();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, grp = lane >> 2, tq = lane & 3;
+    const int group = warp >> 1, r0 = group * 16, c0 = (warp & 1) * 32;      // this warp's tokens and columns
+    if (r0 >= n) return;
+    const unsigned q0 = (unsigned)__cvta_generic_to_shared(qs), k0 = (unsigned)__cvta_generic_to_shared(ks);
+    const unsigned v0 = (unsigned)__cvta_generic_to_shared(vs), s0 = (unsigned)__cvta_generic_to_shared(ss);
+    float acc[4][4], g[8][4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[j][e] = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) g[j][e] = 0.f;
+    for (int kk = 0; kk < D / 16; ++kk) {
+        unsigned af[TQ][4];
+#pragma unroll
+        for (int p = 0; p < TQ; ++p)
+            mt_ldm4(q0 + (p * PLANE + (r0 + (lane & 7) + ((lane >> 3) & 1) * 8) * KP + kk * 16 + (lane >> 4) * 8) * 2, af[p]);
+        // the state, smallest parts first (parts whose product is below the last of 24 bits are left out)
+        float f[4][4] = {};
+#pragma unroll
+        for (int p = 2; p >= 0; --p) {
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                unsigned bf[4];
+                mt_ldm4t(s0 + (p * SPLANE + (kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * MT_VP + c0 + j * 16 + (lane >> 4) * 8) * 2, bf);
+#pragma unroll
+                for (int q = TQ - 1; q >= 0; --q) {
+                    if (p + q > 2) continue;
+                    mt_mma(f[2 * j], af[q], bf[0], bf[1]);
+                    mt_mma(f[2 * j + 1], af[q], bf[2], bf[3]);
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) mt_add(acc[j], f[j]);
+        // the scores of the tokens up to this group's last
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (j > group) break;
+            float u[2][4] = {};
+#pragma unroll
+            for (int p = TQ - 1; p >= 0; --p) {
+                unsigned bf[4];
+                mt_ldm4(k0 + (p * PLANE + (j * 16 + (lane & 7) + (lane >> 4) * 8) * KP + kk * 16 + ((lane >> 3) & 1) * 8) * 2, bf);
+#pragma unroll
+                for (int q = TQ - 1; q >= 0; --q) {
+                    if (p + q > 2) continue;
+                    mt_mma(u[0], af[q], bf[0], bf[1]);
+                    mt_mma(u[1], af[q], bf[2], bf[3]);
+                }
+            }
+            mt_add(g[2 * j], u[0]);
+            mt_add(g[2 * j + 1], u[1]);
+        }
+    }
+    const int ta = r0 + grp, tb = ta + 8;                            // this lane's two tokens
+    const double ca = cum[ta], cb = cum[tb];
+    const float la = expf((float)ca) * a.q_scale, lb = expf((float)cb) * a.q_scale;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) { acc[j][0] *= la; acc[j][1] *= la; acc[j][2] *= lb; acc[j][3] *= lb; }
+    const float sc = a.q_scale * (GATED ? 1.0f : a.k_scale);
+    float na = 0.f, nb = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        if (j > 2 * group + 1) break;
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int s = j * 8 + 2 * tq + e;
+            const double c = cum[s];
+            const float f = take[s] * sc;
+            // (a choice, not a product with zero: what a later token's key is must not show)
+            g[j][e] = s <= ta ? g[j][e] * (f * expf((float)(ca - c))) : 0.f;
+            g[j][2 + e] = s <= tb ? g[j][2 + e] * (f * expf((float)(cb - c))) : 0.f;
+            na += g[j][e];
+            nb += g[j][2 + e];
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        if (i > group) break;
+        unsigned pf[3][4];
+        mt_split2(g[2 * i][0], g[2 * i][1], pf[0][0], pf[1][0], pf[2][0]);
+        mt_split2(g[2 * i][2], g[2 * i][3], pf[0][1], pf[1][1], pf[2][1]);
+        mt_split2(g[2 * i + 1][0], g[2 * i + 1][1], pf[0][2], pf[1][2], pf[2][2]);
+        mt_split2(g[2 * i + 1][2], g[2 * i + 1][3], pf[0][3], pf[1][3], pf[2][3]);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            unsigned bf[4];
+            mt_ldm4t(v0 + ((i * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * MT_VP + c0 + j * 16 + (lane >> 4) * 8) * 2, bf);
+            float u[2][4] = {};
+#pragma unroll
+            for (int p = 2; p >= 0; --p) {
+                mt_mma(u[0], pf[p], bf[0], bf[1]);
+                mt_mma(u[1], pf[p], bf[2], bf[3]);
+            }
+            mt_add(acc[2 * j], u[0]);
+            mt_add(acc[2 * j + 1], u[1]);
+        }
+    }
+    float da = 1.f, db = 1.f;
+    if (GATED) {
+        // the normaliser: n.q of the start state (a quad shares a token's dims) and of the chunk's own keys
+        float ua = 0.f, ub = 0.f;
+        for (int d = tq; d < D; d += 4) {
+            ua = fmaf(__bfloat162float(qs[ta * KP + d]), n0[d], ua);
+            ub = fmaf(__bfloat162float(qs[tb * KP + d]), n0[d], ub);
+        }
+        na = fmaf(la, ua, na);
+        nb = fmaf(lb, ub, nb);
+#pragma unroll
+        for (int o = 1; o < 4; o <<= 1) { na += __shfl_xor_sync(0xffffffffu, na, o); nb += __shfl_xor_sync(0xffffffffu, nb, o); }
+        const float* ga = a.gates + ((size_t)(t_first + min(ta, n - 1)) * a.H + h) * 4;
+        const float* gb = a.gates + ((size_t)(t_first + min(tb, n - 1)) * a.H + h) * 4;
+        da = fmaxf(fabsf(na), ga[2]) + 1e-6f;
+        db = fmaxf(fabsf(nb), gb[2]) + 1e-6f;
+    }
+    const float skip = !GATED && a.d_skip ? a.d_skip[h] : 0.f;
+    float* out = a.out + (size_t)t_first * a.H * V + (size_t)h * V + col0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int col = c0 + j * 8 + 2 * tq;
+        if (col0 + col >= V) continue;
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const int t = r ? tb : ta;
+            if (t >= n) continue;
+            float2 y = make_float2(acc[j][2 * r], acc[j][2 * r + 1]);
+            if (GATED) { y.x /= r ? db : da; y.y /= r ? db : da; }
+            if (!GATED && a.d_skip) {
+                y.x = fmaf(skip, __bfloat162float(vs[t * MT_VP + col]), y.x);
+                y.y = fmaf(skip, __bfloat162float(vs[t * MT_VP + col + 1]), y.y);
+            }
+            if (t >= bad[col]) y.x = __int_as_float(0x7fffffff);
+            if (t >= bad[col + 1]) y.y = __int_as_float(0x7fffffff);
+            *(float2*)(out + (size_t)t * a.H * V + col) = y;
+        }
+    }
+}
+
+// Whether these sizes go on the tensor cores: a chunk's tokens and a head's rows in one block's tiles, rows of whole 16-byte
+// pieces.  (Everything else walks: other head sizes, 32-bit inputs, longer chunks, rows that begin anywhere.)
+static bool mt_takes(const MemoryChunkArgs& a, int act_dtype) {
+    return act_dtype == GL_BF16 && (a.kind == 0 || a.kind == 3) && (a.D == 64 || a.D == 128) && a.V % 8 == 0 && a.chunk_len <= MT_TOKENS
+           && a.ld % 8 == 0 && a.q_off % 8 == 0 && a.k_off % 8 == 0 && a.v_off % 8 == 0 && (!a.cosv || a.rot_half % 8 == 0)
+           && !(((uintptr_t)a.proj | (uintptr_t)a.chunk_state) & 15) && !((uintptr_t)a.out & 7);
+}
+
+template <int D, bool ROT, bool GATED>
+static int mt_launch(const MemoryChunkArgs& a, cudaStream_t stream) {
+    constexpr size_t s1 = mt_states_smem<D>(), s2 = mt_outputs_smem<D, ROT>();
+    if (cudaFuncSetAttribute(memory_chunk_states_tc_kernel<D, ROT, GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s1) != cudaSuccess ||
+        cudaFuncSetAttribute(memory_chunk_outputs_tc_kernel<D, ROT, GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s2) != cudaSuccess) {
+        cudaGetLastError();
+        return GL_ERR_SMEM;
+    }
+    const dim3 grid((a.V + MT_COLS - 1) / MT_COLS, a.H, a.B * a.n_chunks);
+    int rc = gl_launch_in_order(memory_chunk_states_tc_kernel<D, ROT, GATED>, grid, dim3(128), s1, stream, a);
+    if (rc != 0) return rc;
+    rc = gl_launch(memory_chunk_carry4_kernel, dim3((a.D * a.cols / 4 + 127) / 128, a.H, a.B), dim3(128), 0, stream, 1, a);
+    if (rc != 0) return rc;
+    return gl_launch_in_order(memory_chunk_outputs_tc_kernel<D, ROT, GATED>, grid, dim3(256), s2, stream, a);
+}
+
+static int mt_chunks(const MemoryChunkArgs& a, cudaStream_t stream) {
+    const bool rot = a.kind == 3 && a.cosv;
+    if (a.kind == 0) return a.D == 64 ? mt_launch<64, false, true>(a, stream) : mt_launch<128, false, true>(a, stream);
+    if (a.D == 64) return rot ? mt_launch<64, true, false>(a, stream) : mt_launch<64, false, false>(a, stream);
+    return rot ? mt_launch<128, true, false>(a, stream) : mt_launch<128, false, false>(a, stream);
+}
+// ---------------------------------------------------------------------------
+
 // the gated kind's outputs divided by max(|n.q|, e^-m) + 1e-6, all tokens at once
 __global__ void __launch_bounds__(256)
 memory_divide_kernel(MemoryChunkArgs a) {
@@ -400,6 +923,9 @@ static int launch_memory_chunks_nt(const MemoryChunkArgs& a, cudaStream_t stream
     if (KIND == 0) {
         rc = gl_launch(memory_gate_walk_kernel, dim3(a.B * a.H), dim3(32), 0, stream, 1, a);
         if (rc != 0) return rc;
+    }
+    if constexpr (sizeof(TA) == 2 && (KIND == 0 || KIND == 3)) {
+        if (mt_takes(a, GL_BF16)) return mt_chunks(a, stream);
     }
     rc = gl_launch(memory_chunk_decay_kernel<TA, KIND>, dim3((a.D + 127) / 128, a.H, a.B * a.n_chunks), dim3(128), 0, stream, 1, a);
     if (rc != 0) return rc;
@@ -442,7 +968,12 @@ static int dispatch_memory_chunks_kind(const MemoryChunkArgs& a, cudaStream_t st
     return dispatch_memory_chunks<TA, 3>(a, stream);
 }
 
-// (launches 4 kernels for the bounded-forget kind, 5 for the plain decay, 7 for the gated one)
+// kernels that gl_memory_chunks launches
+GL_API int gl_memory_chunks_launches(const MemoryChunkArgs* args, int act_dtype) {
+    const int gates = args->kind == 0 ? 2 : args->kind == 3 ? 1 : 0;
+    return gates + (mt_takes(*args, act_dtype) ? 3 : args->kind == 0 ? 5 : 4);
+}
+
 GL_API int gl_memory_chunks(const MemoryChunkArgs* args, int act_dtype, cudaStream_t stream) {
     const MemoryChunkArgs& a = *args;
     if (a.B <= 0 || a.T <= 0) return GL_OK;

@@ -56,3 +56,25 @@ __device__ __forceinline__ void mc_store16(__nv_bfloat16* dst, const float* v) {
     h[3] = __floats2bfloat162_rn(v[6], v[7]);
     *reinterpret_cast<uint4*>(dst) = raw;
 }
+
+// two 32-bit multiply-adds in one instruction (the pair's halves are independent and rounded like fmaf's)
+__device__ __forceinline__ unsigned long long mc_pack(float x, float y) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ unsigned long long mc_fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ unsigned long long mc_mul2(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ float2 mc_unpack(unsigned long long v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}

@@ -1356,9 +1356,8 @@ def memory_scan(kind: int, proj: torch.Tensor, state: torch.Tensor, ctx, H: int,
                              _addr(sin) if rot_half else None, _addr(skip) if plain else None,
                              gates.shape[1] if plain and gates is not None else 0, kv_heads if plain else 0, rot_half,
                              k_scale)
-        fn = _lib("memory_chunks.cu").gl_memory_chunks
-        _check(_launch(fn, byref(c), c_int(dtype_code(proj.dtype)), _stream()), "memory_chunks",
-               7 if gated else 5 if plain else 4)
+        lib, code = _lib("memory_chunks.cu"), c_int(dtype_code(proj.dtype))
+        _check(_launch(lib.gl_memory_chunks, byref(c), code, _stream()), "memory_chunks", lib.gl_memory_chunks_launches(byref(c), code))
         return out
     # the gated kind's new normaliser and maximum, moved into the state rows by a second kernel
     nm = empty((ctx.n_seqs, H, D + 1), torch.float32, proj.device) if kind == MEMORY_GATED else None
