@@ -1498,6 +1498,28 @@ SCAN_MAX_STATE = 256
 # and a carry between them): a token-by-token walk leaves most of the machine idle when the sequences are few.
 SCAN_CHUNK_TOKENS = 128     # (a prompt of 2,048 tokens: 11.3 / 11.4 / 13.0 / 15.5 ms with chunks of 64 / 128 / 256 / 512)
 SCAN_CHUNKED_FROM = 1024       # (512 tokens in 4 chunks took 8 % longer than walked in one piece)
+# States of up to SCAN_CHUNK_STATE numbers have walks of their own over chunks, a thread a channel.  In 32 bits when chunks are
+# taken stays a matter of the longest run alone; in bfloat16 they are taken from SCAN_SHORT_CHUNKED_FROM tokens on, and shorter,
+# so that few sequences fill the machine.
+# (us a launch with 4,096 channels of 16, in one piece / chunks of 32 / 64 / 128: 1 x 150 tokens 37 / 43 / 62 / 113, 1 x 200 47 / 46 /
+# 62 / 113, 1 x 500 113 / 76 / 80 / 114, 1 x 1,000 221 / 123 / 135 / 148, 1 x 2,040 449 / 237 / 229 / 256, 4 x 150 98 / 89 / 90 /
+# 122, 16 x 300 619 / 545 / 545 / 526.)
+SCAN_CHUNK_STATE = 16
+SCAN_SHORT_CHUNKED_FROM = 192
+SCAN_SHORT_CHUNK_TOKENS, SCAN_SHORT_CHUNK_TOKENS_FEW, SCAN_SHORT_FEW_TOKENS = 64, 32, 1000
+
+
+def scan_chunk_tokens(C: int, N: int, exact: bool, n_seqs: int, tokens: int, longest: int) -> int:
+    """Tokens a chunk of a selective scan's walk over runs of ``tokens`` in all, 0: in one piece.  ``exact``: 32-bit inputs."""
+    if longest >= SCAN_CHUNKED_FROM and (exact or N > SCAN_CHUNK_STATE):
+        return SCAN_CHUNK_TOKENS
+    if exact or N > SCAN_CHUNK_STATE or longest < SCAN_SHORT_CHUNKED_FROM:
+        return 0
+    n = SCAN_SHORT_CHUNK_TOKENS if tokens > SCAN_SHORT_FEW_TOKENS else SCAN_SHORT_CHUNK_TOKENS_FEW
+    # every (sequence, chunk) keeps a whole state (and there are at most 65,535 chunks): many long sequences take longer ones
+    while n < 1024 and (n_seqs * -(-longest // n) * C * N * 4 > MEMORY_CHUNKS_MAX_BYTES or -(-longest // n) > 65535):
+        n *= 2
+    return n
 
 
 def selective_scan(x: torch.Tensor, dtp: torch.Tensor, bc: torch.Tensor, z: torch.Tensor, z_off: int,
@@ -1522,12 +1544,13 @@ def selective_scan(x: torch.Tensor, dtp: torch.Tensor, bc: torch.Tensor, z: torc
                            ctx.seq_slot.data_ptr(), ctx.seq_qstart.data_ptr(), ctx.seq_qlen.data_ptr(),
                            ctx.n_seqs, C, N, z.shape[1], z_off, state.shape[1], None, None, 0, 0, 1 if ctx.max_qlen == 1 else 0)
     kernels = 1
-    if ctx.max_qlen >= SCAN_CHUNKED_FROM:
-        chunks = -(-ctx.max_qlen // SCAN_CHUNK_TOKENS)
+    tokens = scan_chunk_tokens(C, N, x.dtype == torch.float32, ctx.n_seqs, T, ctx.max_qlen)
+    if tokens:
+        chunks = -(-ctx.max_qlen // tokens)
         chunk_state = empty((ctx.n_seqs, chunks, C, N), torch.float32, x.device)
         chunk_dt = empty((ctx.n_seqs, chunks, C), torch.float32, x.device)
         a.chunk_state, a.chunk_dt = chunk_state.data_ptr(), chunk_dt.data_ptr()
-        a.chunk_len, a.n_chunks, kernels = SCAN_CHUNK_TOKENS, chunks, 3
+        a.chunk_len, a.n_chunks, kernels = tokens, chunks, 3
     fn = _lib("selective_scan.cu").gl_selective_scan
     _check(_launch(fn, byref(a), c_int(dtype_code(x.dtype)), _stream()), "selective_scan", kernels)
     return out

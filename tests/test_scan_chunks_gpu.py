@@ -1,0 +1,44 @@
+"""The selective scan's walks over chunks, a thread a channel: states of one to sixteen numbers, channels that leave a block part
+empty, chunks and stages that end anywhere, against the recurrence in 64 bits."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from test_vopedra_gpu import check_selective_scan
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("tokens", [1, 30, 64, 100])
+@pytest.mark.parametrize("C,N", [(1, 16), (130, 5), (128, 1), (257, 12)])
+def test_chunks_of_any_length(C, N, tokens, dtype, monkeypatch):
+    from gopherllm_b200 import ops
+    monkeypatch.setattr(ops, "scan_chunk_tokens", lambda *a: tokens)
+    check_selective_scan(C, N, [64, 1, 131, 65], dtype)
+
+
+def test_endless_and_harsh_steps_in_chunks(monkeypatch):
+    """An infinite step forgets the state and writes infinity from its token on, in its channel alone; steps so large that a
+    state is gone at once leave what is left exact."""
+    from gopherllm_b200 import ops
+    monkeypatch.setattr(ops, "scan_chunk_tokens", lambda *a: 32)
+    C, N, T = 40, 16, 100
+    g = torch.Generator().manual_seed(2)
+    up = lambda *s: torch.rand(*s, generator=g) + 0.1  # noqa: E731
+    x, bc, z, dtp, a_log, d_skip, state = up(T, C), up(T, 2 * N), up(T, C), 100.0 * up(T, C), up(C, N), up(C), up(1, C * N)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+    ctx = SimpleNamespace(seq_slot=i32([0]), seq_qstart=i32([0]), seq_qlen=i32([T]), n_seqs=1, max_qlen=T, n_tokens=T)
+    run = lambda d: ops.selective_scan(x.cuda(), d.cuda(), bc.cuda(), z.cuda(), 0, a_log.cuda(), d_skip.cuda(), state.cuda(), ctx).cpu()  # noqa: E731
+    got = run(dtp).double()
+    dt, S = dtp.double(), state.double().view(C, N)          # (softplus of numbers above 20 is the number)
+    for t in range(T):
+        step = torch.nn.functional.softplus(dt[t])
+        S = torch.exp(-step[:, None] * torch.exp(a_log.double())) * S + (step * x[t].double())[:, None] * bc[t, :N].double()
+        want = (S @ bc[t, N:].double() + d_skip.double() * x[t].double()) * torch.nn.functional.silu(z[t].double())
+        assert ((got[t] - want).abs() <= 2e-5 * want.abs().max()).all(), t
+    ended = dtp / 100.0
+    ended[45, ::3] = float("inf")
+    got = run(ended)
+    assert torch.isfinite(got[:45]).all() and torch.isfinite(got[:, 1::3]).all() and (got[45:, ::3] == float("inf")).all()
