@@ -28,6 +28,9 @@ static_assert(GL_VALUE_DIM % 16 == 0 && GL_VALUE_DIM >= 16 && GL_VALUE_DIM <= 25
 #define AP_ROW (AP_HD * 2 + 16)       // padded row: 8 consecutive rows fall in distinct banks
 #define AP_VROW (AP_VD * 2 + 16)
 #define AP_TILE (64 * AP_ROW)
+#ifndef AP_VALUE_HEADS                // value heads a block takes at most: their results are AP_VD / 2 registers each
+#define AP_VALUE_HEADS (AP_VD <= 64 ? 4 : AP_VD <= 128 ? 2 : 1)
+#endif
 #define AP_VTILE (64 * AP_VROW)
 
 struct PairsArgs {
@@ -103,6 +106,13 @@ __device__ __forceinline__ void ap_load_rows(unsigned dst, const __nv_bfloat16* 
     }
 }
 
+// VG: value heads of a block (of a mixer with nVal of them a query head).  The scores and the softmax of a query head are the same
+// whatever the values, so a block takes as many value heads as its registers hold: with one, a page's scores, exponentials
+// and key tile were computed and fetched once for every value head.
+// 32 query heads and 8 value heads of 64 with a table, the mixing behind them included: runs of 64, 376, 688 and 1,000 tokens 399 us
+// with one value head a block, 404 with two (two blocks an SM instead of three for it), 315 with four; 2,047 tokens 778 and 602;
+// 8 x 40 34 and 29.  The same numbers whichever.
+template <int VG>
 __global__ void __launch_bounds__(AP_THREADS)
 attn_pairs_tc_kernel(PairsArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -110,13 +120,13 @@ attn_pairs_tc_kernel(PairsArgs a) {
     // memory is two key stages and two value stages, so that two or three blocks fit an SM at long key rows)
     const unsigned sK[2] = {ap_smem(smem), ap_smem(smem) + AP_TILE};
     const unsigned sQ = sK[1];
-    const unsigned sV[2] = {sK[0] + 2 * AP_TILE, sK[0] + 2 * AP_TILE + AP_VTILE};
+    const unsigned sV[2] = {sK[0] + 2 * AP_TILE, sK[0] + 2 * AP_TILE + VG * AP_VTILE};
     gl_grid_wait();                                            // (a long kernel: the next one is not launched early)
     const int b = blockIdx.z;
-    const int h = blockIdx.y / a.nVal;                         // query head
+    const int h = blockIdx.y / (a.nVal / VG);                  // query head
     const int g = h / (a.nH / a.nKV);                          // its key head
     const int nvh = a.nVH > 0 ? a.nVH : a.nKV;
-    const int vh = a.nVal > 1 ? blockIdx.y - h * a.nVal : h / (a.nH / nvh);   // the pair's value head
+    const int vh = a.nVal > 1 ? (blockIdx.y - h * (a.nVal / VG)) * VG : h / (a.nH / nvh);   // the pairs' first value head
     const int qlen = a.seq_qlen[b];
     const int n_qtiles = (qlen + AP_BM - 1) / AP_BM;
     const int qt = n_qtiles - 1 - (int)blockIdx.x;           // longest rows first
@@ -141,8 +151,12 @@ attn_pairs_tc_kernel(PairsArgs a) {
     auto k_page = [&](int p) {
         return a.seq_base ? K + (first_row + (size_t)p * GL_PAGE) * k_row + (size_t)g * AP_HD : K + (size_t)pg[p] * page_stride + head_off;
     };
-    auto v_page = [&](int p) {
-        return a.seq_base ? V + (first_row + (size_t)p * GL_PAGE) * v_row + (size_t)vh * AP_VD : V + (size_t)pg[p] * vpage_stride + vhead_off;
+    auto load_values = [&](int st, int p, int nv) {
+#pragma unroll
+        for (int i = 0; i < VG; ++i)
+            ap_load_rows<AP_VD>(sV[st] + i * AP_VTILE,
+                                a.seq_base ? V + (first_row + (size_t)p * GL_PAGE) * v_row + (size_t)(vh + i) * AP_VD
+                                           : V + (size_t)pg[p] * vpage_stride + vhead_off + (size_t)i * GL_PAGE * vs, v_row, nv);
     };
     const size_t q_row = a.q_ld > 0 ? (size_t)a.q_ld : (size_t)a.nH * AP_HD;
 
@@ -151,7 +165,7 @@ attn_pairs_tc_kernel(PairsArgs a) {
     {
         const int nv = min(GL_PAGE, total - page_begin * GL_PAGE);
         ap_load_rows<AP_HD>(sK[0], k_page(page_begin), k_row, nv);
-        if (!a.v_in_k) ap_load_rows<AP_VD>(sV[0], v_page(page_begin), v_row, nv);
+        if (!a.v_in_k) load_values(0, page_begin, nv);
     }
     ap_commit();
     ap_wait<0>();
@@ -165,9 +179,9 @@ attn_pairs_tc_kernel(PairsArgs a) {
         ap_ldm4(sQ + r * AP_ROW + c * 16, qf[kk][0], qf[kk][1], qf[kk][2], qf[kk][3]);
     }
     __syncthreads();
-    float o[AP_NT][4];
+    float o[VG * AP_NT][4];
 #pragma unroll
-    for (int i = 0; i < AP_NT; ++i)
+    for (int i = 0; i < VG * AP_NT; ++i)
 #pragma unroll
         for (int e = 0; e < 4; ++e) o[i][e] = 0.f;
     float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
@@ -185,7 +199,7 @@ attn_pairs_tc_kernel(PairsArgs a) {
         if (p + 1 < page_end) {
             const int nv = min(GL_PAGE, total - (p + 1) * GL_PAGE);
             ap_load_rows<AP_HD>(sK[st ^ 1], k_page(p + 1), k_row, nv);
-            if (!a.v_in_k) ap_load_rows<AP_VD>(sV[st ^ 1], v_page(p + 1), v_row, nv);
+            if (!a.v_in_k) load_values(st ^ 1, p + 1, nv);
         }
         ap_commit();
         ap_wait<1>();
@@ -267,7 +281,7 @@ attn_pairs_tc_kernel(PairsArgs a) {
                 l_run[1] += s[j][2] + s[j][3];
             }
 #pragma unroll
-            for (int i = 0; i < AP_NT; ++i) {
+            for (int i = 0; i < VG * AP_NT; ++i) {
                 o[i][0] *= corr[0]; o[i][1] *= corr[0];
                 o[i][2] *= corr[1]; o[i][3] *= corr[1];
             }
@@ -279,11 +293,11 @@ attn_pairs_tc_kernel(PairsArgs a) {
                 pa[2] = ap_pack(s[2 * kk + 1][0], s[2 * kk + 1][1]);
                 pa[3] = ap_pack(s[2 * kk + 1][2], s[2 * kk + 1][3]);
 #pragma unroll
-                for (int dn = 0; dn < AP_NT; dn += 2) {
+                for (int dn = 0; dn < VG * AP_NT; dn += 2) {
                     unsigned b0, b1, b2, b3;
                     const int r = kk * 16 + ((lane >> 3) & 1) * 8 + (lane & 7);
-                    const int c = dn + (lane >> 4);
-                    ap_ldm4t((a.v_in_k ? sK[st] + r * AP_ROW : sV[st] + r * AP_VROW) + c * 16, b0, b1, b2, b3);
+                    const int c = dn % AP_NT + (lane >> 4);
+                    ap_ldm4t((a.v_in_k ? sK[st] + r * AP_ROW : sV[st] + (dn / AP_NT) * AP_VTILE + r * AP_VROW) + c * 16, b0, b1, b2, b3);
                     ap_mma(o[dn], pa, b0, b1);
                     ap_mma(o[dn + 1], pa, b2, b3);
                 }
@@ -308,8 +322,7 @@ attn_pairs_tc_kernel(PairsArgs a) {
         inv_lo = sc_lo / (l_run[0] * sc_lo + expf(sink - top_lo));
         inv_hi = sc_hi / (l_run[1] * sc_hi + expf(sink - top_hi));
     }
-    const int slot = a.nVal > 1 ? vh : 0;
-    if (a.out && a.nVal == 1) {
+    if (VG == 1 && a.out && a.nVal == 1) {
         __nv_bfloat16* O = (__nv_bfloat16*)a.out;
 #pragma unroll
         for (int i = 0; i < AP_NT; ++i) {
@@ -324,8 +337,8 @@ attn_pairs_tc_kernel(PairsArgs a) {
         return;
     }
 #pragma unroll
-    for (int i = 0; i < AP_NT; ++i) {
-        const int d = i * 8 + 2 * t;
+    for (int i = 0; i < VG * AP_NT; ++i) {
+        const int d = (i % AP_NT) * 8 + 2 * t, slot = a.nVal > 1 ? vh + i / AP_NT : 0;
         if (r_lo < rows)
             *(float2*)(a.pairs + (((size_t)(qstart + q0 + r_lo) * a.nH + h) * a.nVal + slot) * AP_VD + d) =
                 make_float2(o[i][0] * inv_lo, o[i][1] * inv_lo);
@@ -565,6 +578,21 @@ GL_API int gl_attention_rows_decode_tc(const RowsDecodeArgs* args, cudaStream_t 
 
 GL_API int gl_attention_pairs_tc_dims() { return AP_HD * 1000 + AP_VD; }
 
+template <int VG>
+static int launch_pairs(const PairsArgs& a, cudaStream_t stream) {
+    const size_t smem = 2 * (size_t)AP_TILE + (a.v_in_k ? 0 : 2 * VG * (size_t)AP_VTILE);
+    static size_t configured = 0;
+    if (smem > configured) {
+        if (cudaFuncSetAttribute(attn_pairs_tc_kernel<VG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+            cudaGetLastError();
+            return GL_ERR_SMEM;
+        }
+        configured = smem;
+    }
+    dim3 grid((a.max_qlen + AP_BM - 1) / AP_BM, a.nH * (a.nVal / VG), a.B);
+    return gl_launch(attn_pairs_tc_kernel<VG>, grid, dim3(AP_THREADS), smem, stream, 1, a) == 0 ? GL_OK : GL_ERR_LAUNCH;
+}
+
 GL_API int gl_attention_pairs_tc(const PairsArgs* args, cudaStream_t stream) {
     const PairsArgs& a = *args;
     if (a.B <= 0 || a.max_qlen <= 0) return GL_OK;
@@ -574,15 +602,8 @@ GL_API int gl_attention_pairs_tc(const PairsArgs* args, cudaStream_t stream) {
     if (a.v_in_k && (AP_VD > AP_HD || a.nVal != 1 || (a.nVH > 0 && a.nVH != a.nKV))) return GL_ERR_SHAPE;
     if (a.q_ld % 8 || (a.seq_base && (a.kv_ld <= 0 || a.kv_ld % 8 || a.v_in_k))) return GL_ERR_SHAPE;
     if (a.B > 65535 || a.nH * a.nVal > 65535) return GL_ERR_SHAPE;
-    const size_t smem = 2 * (size_t)AP_TILE + (a.v_in_k ? 0 : 2 * (size_t)AP_VTILE);
-    static size_t configured = 0;
-    if (smem > configured) {
-        if (cudaFuncSetAttribute(attn_pairs_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-            cudaGetLastError();
-            return GL_ERR_SMEM;
-        }
-        configured = smem;
-    }
-    dim3 grid((a.max_qlen + AP_BM - 1) / AP_BM, a.nH * a.nVal, a.B);
-    return gl_launch(attn_pairs_tc_kernel, grid, dim3(AP_THREADS), smem, stream, 1, a) == 0 ? GL_OK : GL_ERR_LAUNCH;
+    // as many value heads a block as a power of two up to AP_VALUE_HEADS divides
+    if (a.nVal % 4 == 0 && AP_VALUE_HEADS >= 4) return launch_pairs<AP_VALUE_HEADS >= 4 ? 4 : 1>(a, stream);
+    if (a.nVal % 2 == 0 && AP_VALUE_HEADS >= 2) return launch_pairs<AP_VALUE_HEADS >= 2 ? 2 : 1>(a, stream);
+    return launch_pairs<1>(a, stream);
 }
