@@ -153,6 +153,56 @@ GL_API int gl_scale_softcap(float* x, long long n, float scale, float cap, cudaS
 }
 
 // ---------------------------------------------------------------------------
+// Rows of whole 16-byte pieces for the row kernels below: a thread holds NV4 pieces of its block's row in registers, so a row is
+// read once, every load of a row is in flight before the first is used, and a norm's own vectors, which no kernel writes,
+// are asked for before the kernel waits for the one before it.  What bounds these kernels is that chain of trips (few rows:
+// launch, row, sum, weights, store, one after the other) or HBM (many rows); element by element, with the weights fetched
+// behind the statistics, they took both twice.
+// ---------------------------------------------------------------------------
+template <int NV4>
+__device__ __forceinline__ void row_pieces(float4 (&v)[NV4], const float* src, int n4) {
+#pragma unroll
+    for (int i = 0; i < NV4; ++i) {
+        const int k = threadIdx.x + i * blockDim.x;
+        v[i] = k < n4 ? __ldcg((const float4*)src + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+}
+// a vector no kernel writes: its loads may be issued ahead of the wait
+template <int NV4>
+__device__ __forceinline__ void row_weights(float4 (&v)[NV4], const float* __restrict__ w, int n4) {
+#pragma unroll
+    for (int i = 0; i < NV4; ++i) {
+        const int k = threadIdx.x + i * blockDim.x;
+        v[i] = k < n4 ? ((const float4*)w)[k] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+}
+template <int NV4>
+__device__ __forceinline__ float row_squares(const float4 (&v)[NV4]) {
+    float q = 0.f;
+#pragma unroll
+    for (int i = 0; i < NV4; ++i) q += (v[i].x * v[i].x + v[i].y * v[i].y) + (v[i].z * v[i].z + v[i].w * v[i].w);
+    return q;
+}
+__device__ __forceinline__ void row_put(float* row, int k, const float4& y) { ((float4*)row)[k] = y; }
+__device__ __forceinline__ void row_put(__nv_bfloat16* row, int k, const float4& y) {
+    __nv_bfloat162 p0 = __floats2bfloat162_rn(y.x, y.y), p1 = __floats2bfloat162_rn(y.z, y.w);
+    uint2 pk;
+    pk.x = *(unsigned*)&p0; pk.y = *(unsigned*)&p1;
+    ((uint2*)row)[k] = pk;
+}
+// Pieces a thread and threads a block, or false: rows that are no whole pieces, or longer than 8,192.  Few rows are spread
+// over more threads (the chain is short then), many rows over fewer (a block has more in flight and less to wait for).
+static bool row_shape(int R, int D, uintptr_t addresses, int& nv, int& threads) {
+    if (D % 4 || D > 8192 || (addresses & 15)) return false;
+    const int n4 = D / 4;
+    if (R < 64) nv = n4 <= 256 ? 1 : n4 <= 512 ? 2 : n4 <= 1024 ? 4 : 8;
+    else nv = n4 <= 64 ? 1 : n4 <= 128 ? 2 : n4 <= 1024 ? 4 : 8;
+    threads = ((n4 + nv - 1) / nv + 31) / 32 * 32;
+    return true;
+}
+#define ROW_BY_PIECES(CALL) (nv == 1 ? CALL(1) : nv == 2 ? CALL(2) : nv == 4 ? CALL(4) : CALL(8))
+
+// ---------------------------------------------------------------------------
 // Normalisation of selected rows of a 32-bit matrix.
 //   layernorm: mean, biased variance over the row, y = (x-mean)*rsqrt(var+eps)*g + b
 //              (bert.go:748-776; the reference takes 1/sqrt in 64-bit, so does this)
@@ -246,82 +296,70 @@ __global__ void norm_kernel(const float* x, const int* __restrict__ rows,
     }
 }
 
-// One warp per row, for many rows: the row lives in registers as NV4 float4 per lane, the
-// statistics need warp shuffles only, loads and stores are 16 bytes (D a multiple of 4).
+// A block per row, for many rows: the row lives in registers as NV4 float4 per thread, loads and stores are 16 bytes (D a
+// multiple of 4).  What bounds it is HBM.  With a warp per row a warp held 20 pieces a lane, an SM eight such warps, and a block
+// of eight rows started and ended together: 2,048 rows of 2,560 17.1 us, 12,411 rows 81 us (2.4 TB/s); a row spread over five
+// warps leaves an SM a dozen blocks at different places of their rows: 11.2 and 58 us (what the kernel adds to a prompt's layer).
 template <typename TO, int NV4>
 __global__ void __launch_bounds__(256)
-norm_warp_kernel(const float* x, const int* __restrict__ rows, const float* __restrict__ gamma,
-                 const float* __restrict__ beta, TO* __restrict__ out, int R, int D, float eps, int rms) {
+norm_rows_kernel(const float* x, const int* __restrict__ rows, const float* __restrict__ gamma,
+                 const float* __restrict__ beta, TO* __restrict__ out, int D, float eps, int rms) {
+    __shared__ float red[16];
     gl_grid_launch_dependents();
+    const int n4 = D >> 2, warps = blockDim.x >> 5;
+    float4 g[NV4], b[NV4], v[NV4];
+    row_weights(g, gamma, n4);
+    if (beta) row_weights(b, beta, n4);
     gl_grid_wait();
-    const int lane = threadIdx.x & 31;
-    const int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (r >= R) return;
-    const float4* xr = (const float4*)(x + (size_t)(rows ? rows[r] : r) * D);
-    const int n4 = D >> 2;
-    float4 v[NV4];
-    float s = 0.f;
+    row_pieces(v, x + (size_t)(rows ? rows[blockIdx.x] : blockIdx.x) * D, n4);
+    float mean = 0.f;
+    if (!rms) {
+        float s = 0.f;
 #pragma unroll
-    for (int i = 0; i < NV4; ++i) {
-        const int k = lane + 32 * i;
-        v[i] = k < n4 ? xr[k] : make_float4(0.f, 0.f, 0.f, 0.f);
-        s += (v[i].x + v[i].y) + (v[i].z + v[i].w);
+        for (int i = 0; i < NV4; ++i) s += (v[i].x + v[i].y) + (v[i].z + v[i].w);
+        s = gl_warp_sum(s);
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+        __syncthreads();
+        for (int i = 0; i < warps; ++i) mean += red[i];                    // same order in every thread
+        mean /= (float)D;
     }
-    const float mean = rms ? 0.f : gl_warp_sum(s) / (float)D;
     float q = 0.f;
 #pragma unroll
     for (int i = 0; i < NV4; ++i) {
-        if (lane + 32 * i < n4) {
-            const float a = v[i].x - mean, b = v[i].y - mean, c = v[i].z - mean, d = v[i].w - mean;
-            q += (a * a + b * b) + (c * c + d * d);
+        if ((int)(threadIdx.x + i * blockDim.x) < n4) {
+            const float a = v[i].x - mean, c = v[i].y - mean, d = v[i].z - mean, e = v[i].w - mean;
+            q += (a * a + c * c) + (d * d + e * e);
         }
     }
-    const float var = gl_warp_sum(q) / (float)D;
-    float inv = 0.f;
-    if (lane == 0) inv = (float)(1.0 / sqrt((double)(var + eps)));
-    inv = __shfl_sync(0xffffffffu, inv, 0);
-    const float4* g4 = (const float4*)gamma;
-    const float4* b4 = (const float4*)beta;
+    q = gl_warp_sum(q);
+    if ((threadIdx.x & 31) == 0) red[8 + (threadIdx.x >> 5)] = q;
+    __syncthreads();
+    float var = 0.f;
+    for (int i = 0; i < warps; ++i) var += red[8 + i];
+    var /= (float)D;
+    const float inv = (float)(1.0 / sqrt((double)(var + eps)));            // in 64-bit, as the reference takes it (bert.go:764)
 #pragma unroll
     for (int i = 0; i < NV4; ++i) {
-        const int k = lane + 32 * i;
-        if (k < n4) {
-            const float4 g = g4[k];
-            float4 y;
-            y.x = (v[i].x - mean) * inv * g.x; y.y = (v[i].y - mean) * inv * g.y;
-            y.z = (v[i].z - mean) * inv * g.z; y.w = (v[i].w - mean) * inv * g.w;
-            if (beta) { const float4 b = b4[k]; y.x += b.x; y.y += b.y; y.z += b.z; y.w += b.w; }
-            if constexpr (sizeof(TO) == 4) {
-                ((float4*)(out + (size_t)r * D))[k] = y;
-            } else {
-                __nv_bfloat162 p0 = __floats2bfloat162_rn(y.x, y.y), p1 = __floats2bfloat162_rn(y.z, y.w);
-                uint2 pk;
-                pk.x = *(unsigned*)&p0; pk.y = *(unsigned*)&p1;
-                ((uint2*)(out + (size_t)r * D))[k] = pk;
-            }
-        }
+        const int k = threadIdx.x + i * blockDim.x;
+        if (k >= n4) break;
+        float4 y = make_float4((v[i].x - mean) * inv * g[i].x, (v[i].y - mean) * inv * g[i].y,
+                               (v[i].z - mean) * inv * g[i].z, (v[i].w - mean) * inv * g[i].w);
+        if (beta) { y.x += b[i].x; y.y += b[i].y; y.z += b[i].z; y.w += b[i].w; }
+        row_put(out + (size_t)blockIdx.x * D, k, y);
     }
-}
-
-template <typename TO, int NV4>
-static int launch_norm_warp(const float* x, const int* rows, const float* gamma, const float* beta, TO* out,
-                            int R, int D, float eps, int rms, cudaStream_t stream) {
-    return gl_launch(norm_warp_kernel<TO, NV4>, dim3((R + 7) / 8), dim3(256), 0, stream, 1, x, rows, gamma, beta, out, R, D, eps, rms);
 }
 
 template <typename TO>
 static int launch_norm(const float* x, const int* rows, const float* gamma, const float* beta, TO* out,
                        int R, int D, float eps, int rms, cudaStream_t stream) {
-    const bool vec = D % 4 == 0 && !(((uintptr_t)x | (uintptr_t)out | (uintptr_t)gamma | (uintptr_t)beta) & 15);
     // (the 32-bit path keeps one kernel for every row count, so that a row's result never depends
     // on how many rows come with it)
-    if (sizeof(TO) == 2 && R >= 256 && vec && D <= 4096) {
-        const int n = (D / 4 + 31) / 32;
-        if (n <= 4) return launch_norm_warp<TO, 4>(x, rows, gamma, beta, out, R, D, eps, rms, stream);
-        if (n <= 8) return launch_norm_warp<TO, 8>(x, rows, gamma, beta, out, R, D, eps, rms, stream);
-        if (n <= 16) return launch_norm_warp<TO, 16>(x, rows, gamma, beta, out, R, D, eps, rms, stream);
-        if (n <= 24) return launch_norm_warp<TO, 24>(x, rows, gamma, beta, out, R, D, eps, rms, stream);
-        return launch_norm_warp<TO, 32>(x, rows, gamma, beta, out, R, D, eps, rms, stream);
+    int nv, row_threads;
+    if (sizeof(TO) == 2 && R >= 256 && D <= 4096
+        && row_shape(R, D, (uintptr_t)x | (uintptr_t)out | (uintptr_t)gamma | (uintptr_t)beta, nv, row_threads)) {
+#define CALL(N) gl_launch(norm_rows_kernel<TO, N>, dim3(R), dim3(row_threads), 0, stream, 1, x, rows, gamma, beta, out, D, eps, rms)
+        return ROW_BY_PIECES(CALL);
+#undef CALL
     }
     const int threads = D >= 2048 ? 512 : (D >= 512 ? 256 : 128);
     const int per = (D + threads - 1) / threads;
@@ -675,56 +713,6 @@ GL_API int gl_enter_pass(float* x, const float* base, const float* table, int T,
     const long long want = (n + 255) / 256;
     return gl_launch(enter_pass_kernel, dim3((unsigned)(want > 8192 ? 8192 : want)), dim3(256), 0, stream, 1, x, base, table, n, D, row);
 }
-
-// ---------------------------------------------------------------------------
-// Rows of whole 16-byte pieces for the row kernels below: a thread holds NV4 pieces of its block's row in registers, so a row is
-// read once, every load of a row is in flight before the first is used, and a norm's own vectors, which no kernel writes,
-// are asked for before the kernel waits for the one before it.  What bounds these kernels is that chain of trips (few rows:
-// launch, row, sum, weights, store, one after the other) or HBM (many rows); element by element, with the weights fetched
-// behind the statistics, they took both twice.
-// ---------------------------------------------------------------------------
-template <int NV4>
-__device__ __forceinline__ void row_pieces(float4 (&v)[NV4], const float* src, int n4) {
-#pragma unroll
-    for (int i = 0; i < NV4; ++i) {
-        const int k = threadIdx.x + i * blockDim.x;
-        v[i] = k < n4 ? __ldcg((const float4*)src + k) : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-}
-// a vector no kernel writes: its loads may be issued ahead of the wait
-template <int NV4>
-__device__ __forceinline__ void row_weights(float4 (&v)[NV4], const float* __restrict__ w, int n4) {
-#pragma unroll
-    for (int i = 0; i < NV4; ++i) {
-        const int k = threadIdx.x + i * blockDim.x;
-        v[i] = k < n4 ? ((const float4*)w)[k] : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-}
-template <int NV4>
-__device__ __forceinline__ float row_squares(const float4 (&v)[NV4]) {
-    float q = 0.f;
-#pragma unroll
-    for (int i = 0; i < NV4; ++i) q += (v[i].x * v[i].x + v[i].y * v[i].y) + (v[i].z * v[i].z + v[i].w * v[i].w);
-    return q;
-}
-__device__ __forceinline__ void row_put(float* row, int k, const float4& y) { ((float4*)row)[k] = y; }
-__device__ __forceinline__ void row_put(__nv_bfloat16* row, int k, const float4& y) {
-    __nv_bfloat162 p0 = __floats2bfloat162_rn(y.x, y.y), p1 = __floats2bfloat162_rn(y.z, y.w);
-    uint2 pk;
-    pk.x = *(unsigned*)&p0; pk.y = *(unsigned*)&p1;
-    ((uint2*)row)[k] = pk;
-}
-// Pieces a thread and threads a block, or false: rows that are no whole pieces, or longer than 8,192.  Few rows are spread
-// over more threads (the chain is short then), many rows over fewer (a block has more in flight and less to wait for).
-static bool row_shape(int R, int D, uintptr_t addresses, int& nv, int& threads) {
-    if (D % 4 || D > 8192 || (addresses & 15)) return false;
-    const int n4 = D / 4;
-    if (R < 64) nv = n4 <= 256 ? 1 : n4 <= 512 ? 2 : n4 <= 1024 ? 4 : 8;
-    else nv = n4 <= 64 ? 1 : n4 <= 128 ? 2 : n4 <= 1024 ? 4 : 8;
-    threads = ((n4 + nv - 1) / nv + 31) / 32 * 32;
-    return true;
-}
-#define ROW_BY_PIECES(CALL) (nv == 1 ? CALL(1) : nv == 2 ? CALL(2) : nv == 4 ? CALL(4) : CALL(8))
 
 // ---------------------------------------------------------------------------
 // A branch's output normalised over the width and added: 
