@@ -376,6 +376,7 @@ __global__ void __launch_bounds__(AP_THREADS)
 attn_rows_decode_tc_kernel(RowsDecodeArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     constexpr int QT = 16 * AP_ROW;
+    __shared__ float pf[4][16];
     const unsigned sQ = ap_smem(smem);
     const unsigned sK[2] = {sQ + QT, sQ + QT + AP_TILE};
     const unsigned sV[2] = {sQ + QT + 2 * AP_TILE, sQ + QT + 2 * AP_TILE + AP_VTILE};
@@ -529,26 +530,38 @@ attn_rows_decode_tc_kernel(RowsDecodeArgs a) {
         pm[(warp * 16 + grp + 8) * 2 + 1] = l_run[1];
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < a.rows * AP_VD; i += AP_THREADS) {
-        const int r = i / AP_VD, d = i - r * AP_VD;
+    // each warp's factor on a row, once a row and not once an element of it (with the exponentials in the loop below a block of 16
+    // rows of 256 spent as long on them as on its page)
+    if (threadIdx.x < 64) {
+        const int w = threadIdx.x >> 4, r = threadIdx.x & 15;
         float mm = -INFINITY;
 #pragma unroll
-        for (int w = 0; w < 4; ++w) mm = fmaxf(mm, pm[(w * 16 + r) * 2]);
-        float y = 0.f, l = 0.f;
+        for (int v = 0; v < 4; ++v) mm = fmaxf(mm, pm[(v * 16 + r) * 2]);
+        const float mw = pm[(w * 16 + r) * 2];
+        pf[w][r] = mw > -INFINITY ? expf(mw - mm) : 0.f;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < a.rows * (AP_VD / 4); i += AP_THREADS) {
+        const int r = i / (AP_VD / 4), d = (i - r * (AP_VD / 4)) * 4;
+        float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
         for (int w = 0; w < 4; ++w) {
-            const float mw = pm[(w * 16 + r) * 2];
-            if (mw > -INFINITY) {
-                const float f = expf(mw - mm);
-                y = fmaf(po[((size_t)w * 16 + r) * AP_VD + d], f, y);
-                l = fmaf(pm[(w * 16 + r) * 2 + 1], f, l);
-            }
+            if (!(pm[(w * 16 + r) * 2] > -INFINITY)) continue;
+            const float f = pf[w][r];
+            const float4 v = *(const float4*)(po + ((size_t)w * 16 + r) * AP_VD + d);
+            y.x = fmaf(v.x, f, y.x); y.y = fmaf(v.y, f, y.y); y.z = fmaf(v.z, f, y.z); y.w = fmaf(v.w, f, y.w);
         }
-        a.parts[(((size_t)b * a.nH + head0 + r) * a.splits + split) * AP_VD + d] = y;
+        const size_t at = ((size_t)b * a.nH + head0 + r) * a.splits + split;
+        *(float4*)(a.parts + at * AP_VD + d) = y;
         if (d == 0) {
-            float* dst = a.ml + (((size_t)b * a.nH + head0 + r) * a.splits + split) * 2;
-            dst[0] = mm;
-            dst[1] = l;
+            float mm = -INFINITY, l = 0.f;
+#pragma unroll
+            for (int w = 0; w < 4; ++w) {
+                mm = fmaxf(mm, pm[(w * 16 + r) * 2]);
+                if (pm[(w * 16 + r) * 2] > -INFINITY) l = fmaf(pm[(w * 16 + r) * 2 + 1], pf[w][r], l);
+            }
+            a.ml[at * 2] = mm;
+            a.ml[at * 2 + 1] = l;
         }
     }
 }
