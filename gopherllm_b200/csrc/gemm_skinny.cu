@@ -63,8 +63,11 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], unsigned a0, unsigned a1
 // byte offset of 16-byte chunk c of row r in a tile of 128-byte rows
 __device__ __forceinline__ int swz(int r, int c) { return r * 128 + ((c ^ (r & 7)) << 4); }
 
+// Blocks an SM, stated (what shared memory allows): left to itself the compiler gave the kernel 40 to 56 registers, with spills for up
+// to 8 tokens, and loaded a stage's fragments in turn with its products.  With 64 to 100 they are on their way together: a step of
+// Phi-2 with one sequence of 2,040 positions 1.437 -> 1.387 ms, with 8 2.282 -> 2.164; 12 requests of Phi-1.5 24.9 -> 23.9 ms.
 template <int MT, int STAGES, typename TO>
-__global__ void __launch_bounds__(SK_THREADS)
+__global__ void __launch_bounds__(SK_THREADS, MT <= 2 ? 4 : 3)
 gemm_skinny_kernel(GemmArgs g, int k_per_block, const __grid_constant__ CUtensorMap map_w,
                    const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w2,
                    const __grid_constant__ CUtensorMap map_a2) {
@@ -218,10 +221,10 @@ static constexpr size_t skinny_smem() {
     // stages + barriers + room to align the start; the reduction tile reuses the stages
     return (size_t)STAGES * (SK_ROWS * 128 + MT * 8 * 128) + 8 * STAGES + 1024;
 }
-static_assert(4 * (SK_ROWS * 128 + 8 * 8 * 128) >= 8 * 8 * (SK_ROWS + 1) * 4, "reduction tile fits the stages");
 
 template <int MT, int STAGES, typename TO>
 static int launch_skinny(const GemmArgs& g, int S, cudaStream_t stream) {
+    static_assert(STAGES * (SK_ROWS * 128 + MT * 8 * 128) >= MT * 8 * (SK_ROWS + 1) * 4, "reduction tile fits the stages");
     constexpr size_t smem = skinny_smem<MT, STAGES>();
     static bool configured = false;
     if (!configured) {
@@ -253,20 +256,27 @@ static int launch_skinny(const GemmArgs& g, int S, cudaStream_t stream) {
     return GL_OK;
 }
 
-// blocks of one SM that fit by shared memory, for each M bucket
+// Eights of tokens a kernel is built for.  From 17 tokens on the products themselves, not the weights' stream, set the pace (a
+// k-step of a warp is as many mma.sync as there are eights), so each count has its own kernel: 37 tokens on the one for 64 paid
+// for 27 that are not there (a request of 37 tokens and 12 more, Phi-1.5: 11.13 -> 10.35 ms with the registers above).
+#define SK_BY_TOKENS(M, CALL) \
+    ((M) <= 8 ? CALL(1, 6) : (M) <= 16 ? CALL(2, 6) : (M) <= 24 ? CALL(3, 5) : (M) <= 32 ? CALL(4, 5) \
+     : (M) <= 40 ? CALL(5, 5) : (M) <= 48 ? CALL(6, 4) : (M) <= 56 ? CALL(7, 4) : CALL(8, 4))
+
+// blocks of one SM that fit by shared memory
 static int blocks_per_sm(int M) {
-    const size_t smem = M <= 8 ? skinny_smem<1, 6>() : M <= 16 ? skinny_smem<2, 6>()
-                      : M <= 32 ? skinny_smem<4, 5>() : skinny_smem<8, 4>();
+#define CALL(MT, STAGES) skinny_smem<MT, STAGES>()
+    const size_t smem = SK_BY_TOKENS(M, CALL);
+#undef CALL
     const int n = (int)((227 * 1024) / (smem + 1024));
     return n < 1 ? 1 : (n > 8 ? 8 : n);
 }
 
 template <typename TO>
 static int dispatch_m(const GemmArgs& g, int S, cudaStream_t stream) {
-    if (g.M <= 8) return launch_skinny<1, 6, TO>(g, S, stream);
-    if (g.M <= 16) return launch_skinny<2, 6, TO>(g, S, stream);
-    if (g.M <= 32) return launch_skinny<4, 5, TO>(g, S, stream);
-    return launch_skinny<8, 4, TO>(g, S, stream);
+#define CALL(MT, STAGES) launch_skinny<MT, STAGES, TO>(g, S, stream)
+    return SK_BY_TOKENS(g.M, CALL);
+#undef CALL
 }
 
 // 1 if a bounded wait of this library ever ran out (the result of that launch is invalid)
