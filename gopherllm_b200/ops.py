@@ -1244,10 +1244,32 @@ def memory_walks_chunks(kind: int, n_seqs: int, tokens: int, longest: int, eleme
     return max(run, all_runs) + 0.5 * min(run, all_runs) > gain * chunks
 
 
-def memory_chunk_tokens(kind: int, exact: bool, n_seqs: int, tokens: int, longest: int, H: int, D: int, V: int) -> int:
-    """Tokens a chunk of a memory's walk over runs of ``tokens`` in all, 0: token by token.  ``exact``: 32-bit inputs."""
+# Chunks that are products on the tensor cores (csrc/memory_chunks.cu) pay from 48 tokens on, with four sequences or more from 24
+# on, in chunks of 64 (of 32 up to 128 tokens in all).  us a launch, token by token / chunks of 32 / of 64: gated, 8 heads of 128 x 256:
+# 1 x 33 22.9 / 22.4 / 22.0, 1 x 64 36.8 / 22.3 / 24.6, 1 x 160 82 / 27 / 29, 4 x 33 58 / 30 / 26, 16 x 32 128 / 50 / 50, 16 x 300 1063 / 454 /
+# 297; plain decay, 64 heads of 128 x 64: 1 x 33 28 / 20 / 20, 4 x 100 150 / 63 / 53, 16 x 12 70 / 75 / 74, 16 x 300 1420 / 805 / 520; 16 heads
+# of 64 x 128 with a rotation: 1 x 33 19.4 / 19.3 / 20.4, 1 x 64 30 / 19 / 22, 16 x 12 27 / 34 / 34, 16 x 32 53 / 38 / 39.
+MEMORY_PRODUCTS_FROM, MEMORY_PRODUCTS_FROM_MANY, MEMORY_PRODUCTS_MANY = 48, 24, 4
+MEMORY_PRODUCTS_FEW_TOKENS = 128
+
+
+def memory_takes_products(kind: int, dtype, ld: int, D: int, V: int, offsets, rot_half: int) -> bool:
+    """Whether a memory's chunks go on the tensor cores (the launcher's own rule, but for addresses)."""
+    return (dtype == torch.bfloat16 and kind in (MEMORY_GATED, MEMORY_DECAY) and D in (64, 128) and V % 8 == 0 and ld % 8 == 0
+            and rot_half % 8 == 0 and all(o % 8 == 0 for o in offsets))
+
+
+def memory_chunk_tokens(kind: int, exact: bool, n_seqs: int, tokens: int, longest: int, H: int, D: int, V: int,
+                        products: bool = False) -> int:
+    """Tokens a chunk of a memory's walk over runs of ``tokens`` in all, 0: token by token.  ``exact``: 32-bit inputs;
+    ``products``: chunks are products on the tensor cores."""
     if not USE_MEMORY_CHUNKS or kind not in (MEMORY_GATED, MEMORY_BOUNDED_FORGET, MEMORY_DECAY) or D > MEMORY_CHUNKS_MAX_ROWS:
         return 0
+    if products and longest >= (MEMORY_PRODUCTS_FROM_MANY if n_seqs >= MEMORY_PRODUCTS_MANY else MEMORY_PRODUCTS_FROM):
+        n = MEMORY_CHUNK_TOKENS if tokens > MEMORY_PRODUCTS_FEW_TOKENS else MEMORY_CHUNK_TOKENS_FEW
+        chunks = n_seqs * -(-longest // n)
+        if chunks * H * D * V * 4 <= MEMORY_CHUNKS_MAX_BYTES and chunks <= 65535:
+            return n
     if kind == MEMORY_DECAY:
         if longest < DECAY_CHUNKED_FROM:
             return 0
@@ -1337,7 +1359,8 @@ def memory_scan(kind: int, proj: torch.Tensor, state: torch.Tensor, ctx, H: int,
         _need(lower, "lower", torch.float32, (H * D,))
     out = empty((T, H * V), torch.float32, proj.device)
     gated, plain = kind == MEMORY_GATED, kind == MEMORY_DECAY
-    chunk_tokens = memory_chunk_tokens(kind, proj.dtype == torch.float32, ctx.n_seqs, T, ctx.max_qlen, H, D, V)
+    products = memory_takes_products(kind, proj.dtype, ld, D, V, (q_off, k_off, v_off), rot_half)
+    chunk_tokens = memory_chunk_tokens(kind, proj.dtype == torch.float32, ctx.n_seqs, T, ctx.max_qlen, H, D, V, products)
     if chunk_tokens:
         chunks = -(-ctx.max_qlen // chunk_tokens)
         # a long run: chunks of tokens side by side, a lane a column (two walks and a carry between them)
