@@ -296,17 +296,83 @@ __global__ void norm_kernel(const float* x, const int* __restrict__ rows,
     }
 }
 
-// A block per row, for many rows: the row lives in registers as NV4 float4 per thread, loads and stores are 16 bytes (D a
-// multiple of 4).  What bounds it is HBM.  With a warp per row a warp held 20 pieces a lane, an SM eight such warps, and a block
-// of eight rows started and ended together: 2,048 rows of 2,560 17.1 us, 12,411 rows 81 us (2.4 TB/s); a row spread over five
-// warps leaves an SM a dozen blocks at different places of their rows: 11.2 and 58 us (what the kernel adds to a prompt's layer).
+// y + b, each sum rounded by itself (left to the compiler, some sizes' kernels joined it with the product before)
+__device__ __forceinline__ float4 row_add(const float4& y, const float4& b) {
+    return make_float4(__fadd_rn(y.x, b.x), __fadd_rn(y.y, b.y), __fadd_rn(y.z, b.z), __fadd_rn(y.w, b.w));
+}
+
+// One warp per row, for many rows: the row lives in registers as NV4 float4 per lane, the
+// statistics need warp shuffles only, loads and stores are 16 bytes (D a multiple of 4).
+// What bounds it is HBM: 12,411 rows of 2,560 38 us (5.0 TB/s), of 512 7.9 (a block per row, below: 48 and 13).
+template <typename TO, int NV4>
+__global__ void __launch_bounds__(256)
+norm_warp_kernel(const float* x, const int* __restrict__ rows, const float* __restrict__ gamma,
+                 const float* __restrict__ beta, TO* __restrict__ out, int R, int D, float eps, int rms) {
+    gl_grid_launch_dependents();
+    gl_grid_wait();
+    const int lane = threadIdx.x & 31;
+    const int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (r >= R) return;
+    const float4* xr = (const float4*)(x + (size_t)(rows ? rows[r] : r) * D);
+    const int n4 = D >> 2;
+    float4 v[NV4];
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < NV4; ++i) {
+        const int k = lane + 32 * i;
+        v[i] = k < n4 ? xr[k] : make_float4(0.f, 0.f, 0.f, 0.f);
+        s += (v[i].x + v[i].y) + (v[i].z + v[i].w);
+    }
+    const float mean = rms ? 0.f : gl_warp_sum(s) / (float)D;
+    float q = 0.f;
+#pragma unroll
+    for (int i = 0; i < NV4; ++i) {
+        if (lane + 32 * i < n4) {
+            const float a = v[i].x - mean, b = v[i].y - mean, c = v[i].z - mean, d = v[i].w - mean;
+            q += (a * a + b * b) + (c * c + d * d);
+        }
+    }
+    const float var = gl_warp_sum(q) / (float)D;
+    float inv = 0.f;
+    if (lane == 0) inv = (float)(1.0 / sqrt((double)(var + eps)));
+    inv = __shfl_sync(0xffffffffu, inv, 0);
+    const float4* g4 = (const float4*)gamma;
+    const float4* b4 = (const float4*)beta;
+#pragma unroll
+    for (int i = 0; i < NV4; ++i) {
+        const int k = lane + 32 * i;
+        if (k < n4) {
+            const float4 g = g4[k];
+            float4 y;
+            y.x = (v[i].x - mean) * inv * g.x; y.y = (v[i].y - mean) * inv * g.y;
+            y.z = (v[i].z - mean) * inv * g.z; y.w = (v[i].w - mean) * inv * g.w;
+            if (beta) y = row_add(y, b4[k]);
+            row_put(out + (size_t)r * D, k, y);
+        }
+    }
+}
+
+// The sum over a row of its pieces' sums, which the block's threads left in shared memory: lane l of every warp adds pieces l, l + 32,
+// ... in turn, then the lanes are added.  The order is the width's alone, whatever the block's shape.
+__device__ __forceinline__ float row_sum(const float* piece, int n4) {
+    float s = 0.f;
+#pragma unroll 4
+    for (int k = threadIdx.x & 31; k < n4; k += 32) s += piece[k];
+    return gl_warp_sum(s);
+}
+
+// A block per row, for some hundred to a few thousand rows: a thread holds NV4 pieces of the row, so that an SM has a dozen blocks at
+// different places of their rows.  The numbers are the kernel's above, to the last bit, so the form may follow the number of rows.
+// (Summed thread by thread and warp by warp instead, a prompt's logits moved by half a percent, by which the rounding of a few bfloat16
+// numbers shows after thirty layers.)  Inputs from HBM, us, a warp and a block per row: 256 x 2,560 7.6 and 3.3, 2,048 x 2,048 7.7 and
+// 7.2, 2,048 x 2,560 9.3 and 9.4, 4,096 x 2,560 17.7 and 16.9, 2,048 x 4,096 23.3 and 15.9, 2,048 x 1,024 5.0 and 4.1.
 template <typename TO, int NV4>
 __global__ void __launch_bounds__(256)
 norm_rows_kernel(const float* x, const int* __restrict__ rows, const float* __restrict__ gamma,
                  const float* __restrict__ beta, TO* __restrict__ out, int D, float eps, int rms) {
-    __shared__ float red[16];
+    extern __shared__ float pieces[];                                      // [2][n4]: the sums' and the squares'
     gl_grid_launch_dependents();
-    const int n4 = D >> 2, warps = blockDim.x >> 5;
+    const int n4 = D >> 2;
     float4 g[NV4], b[NV4], v[NV4];
     row_weights(g, gamma, n4);
     if (beta) row_weights(b, beta, n4);
@@ -314,29 +380,24 @@ norm_rows_kernel(const float* x, const int* __restrict__ rows, const float* __re
     row_pieces(v, x + (size_t)(rows ? rows[blockIdx.x] : blockIdx.x) * D, n4);
     float mean = 0.f;
     if (!rms) {
-        float s = 0.f;
 #pragma unroll
-        for (int i = 0; i < NV4; ++i) s += (v[i].x + v[i].y) + (v[i].z + v[i].w);
-        s = gl_warp_sum(s);
-        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+        for (int i = 0; i < NV4; ++i) {
+            const int k = threadIdx.x + i * blockDim.x;
+            if (k < n4) pieces[k] = (v[i].x + v[i].y) + (v[i].z + v[i].w);
+        }
         __syncthreads();
-        for (int i = 0; i < warps; ++i) mean += red[i];                    // same order in every thread
-        mean /= (float)D;
+        mean = row_sum(pieces, n4) / (float)D;
     }
-    float q = 0.f;
 #pragma unroll
     for (int i = 0; i < NV4; ++i) {
-        if ((int)(threadIdx.x + i * blockDim.x) < n4) {
+        const int k = threadIdx.x + i * blockDim.x;
+        if (k < n4) {
             const float a = v[i].x - mean, c = v[i].y - mean, d = v[i].z - mean, e = v[i].w - mean;
-            q += (a * a + c * c) + (d * d + e * e);
+            pieces[n4 + k] = (a * a + c * c) + (d * d + e * e);
         }
     }
-    q = gl_warp_sum(q);
-    if ((threadIdx.x & 31) == 0) red[8 + (threadIdx.x >> 5)] = q;
     __syncthreads();
-    float var = 0.f;
-    for (int i = 0; i < warps; ++i) var += red[8 + i];
-    var /= (float)D;
+    const float var = row_sum(pieces + n4, n4) / (float)D;
     const float inv = (float)(1.0 / sqrt((double)(var + eps)));            // in 64-bit, as the reference takes it (bert.go:764)
 #pragma unroll
     for (int i = 0; i < NV4; ++i) {
@@ -344,9 +405,15 @@ norm_rows_kernel(const float* x, const int* __restrict__ rows, const float* __re
         if (k >= n4) break;
         float4 y = make_float4((v[i].x - mean) * inv * g[i].x, (v[i].y - mean) * inv * g[i].y,
                                (v[i].z - mean) * inv * g[i].z, (v[i].w - mean) * inv * g[i].w);
-        if (beta) { y.x += b[i].x; y.y += b[i].y; y.z += b[i].z; y.w += b[i].w; }
+        if (beta) y = row_add(y, b[i]);
         row_put(out + (size_t)blockIdx.x * D, k, y);
     }
+}
+
+template <typename TO, int NV4>
+static int launch_norm_warp(const float* x, const int* rows, const float* gamma, const float* beta, TO* out,
+                            int R, int D, float eps, int rms, cudaStream_t stream) {
+    return gl_launch(norm_warp_kernel<TO, NV4>, dim3((R + 7) / 8), dim3(256), 0, stream, 1, x, rows, gamma, beta, out, R, D, eps, rms);
 }
 
 template <typename TO>
@@ -354,12 +421,24 @@ static int launch_norm(const float* x, const int* rows, const float* gamma, cons
                        int R, int D, float eps, int rms, cudaStream_t stream) {
     // (the 32-bit path keeps one kernel for every row count, so that a row's result never depends
     // on how many rows come with it)
-    int nv, row_threads;
-    if (sizeof(TO) == 2 && R >= 256 && D <= 4096
-        && row_shape(R, D, (uintptr_t)x | (uintptr_t)out | (uintptr_t)gamma | (uintptr_t)beta, nv, row_threads)) {
-#define CALL(N) gl_launch(norm_rows_kernel<TO, N>, dim3(R), dim3(row_threads), 0, stream, 1, x, rows, gamma, beta, out, D, eps, rms)
-        return ROW_BY_PIECES(CALL);
+    if constexpr (sizeof(TO) == 2) {
+        int nv, row_threads;
+        if (R >= 256 && D <= 4096 && row_shape(R, D, (uintptr_t)x | (uintptr_t)out | (uintptr_t)gamma | (uintptr_t)beta, nv, row_threads)) {
+            // A block a row up to 4,096 rows, of up to 1,024 columns up to 2,048; above, its threads' share of a row no longer pays for its
+            // start (a warp and a block per row, us: 3,000 x 512 4.1 and 4.8, 4,096 x 1,024 5.8 and 6.7, 8,192 x 2,560 29.5 and 32.8).
+            if (R <= (D > 1024 ? 4096 : 2048)) {
+                const size_t smem = 2 * (size_t)(D / 4) * sizeof(float);
+#define CALL(N) gl_launch(norm_rows_kernel<TO, N>, dim3(R), dim3(row_threads), smem, stream, 1, x, rows, gamma, beta, out, D, eps, rms)
+                return nv == 1 ? CALL(1) : nv == 2 ? CALL(2) : CALL(4);        // (up to 4,096 columns)
 #undef CALL
+            }
+            const int n = (D / 4 + 31) / 32;
+            if (n <= 4) return launch_norm_warp<TO, 4>(x, rows, gamma, beta, out, R, D, eps, rms, stream);
+            if (n <= 8) return launch_norm_warp<TO, 8>(x, rows, gamma, beta, out, R, D, eps, rms, stream);
+            if (n <= 16) return launch_norm_warp<TO, 16>(x, rows, gamma, beta, out, R, D, eps, rms, stream);
+            if (n <= 24) return launch_norm_warp<TO, 24>(x, rows, gamma, beta, out, R, D, eps, rms, stream);
+            return launch_norm_warp<TO, 32>(x, rows, gamma, beta, out, R, D, eps, rms, stream);
+        }
     }
     const int threads = D >= 2048 ? 512 : (D >= 512 ? 256 : 128);
     const int per = (D + threads - 1) / threads;
