@@ -176,12 +176,57 @@ __device__ __forceinline__ void row_weights(float4 (&v)[NV4], const float* __res
         v[i] = k < n4 ? ((const float4*)w)[k] : make_float4(0.f, 0.f, 0.f, 0.f);
     }
 }
-template <int NV4>
-__device__ __forceinline__ float row_squares(const float4 (&v)[NV4]) {
+// M warp sums at once, M a power of two up to 8: sum i is left in the lanes whose top log2(M) bits, the highest first, spell i's bits
+// from the lowest on.  Each is the number gl_warp_sum gives; a step hands over half of what is left.
+template <int M>
+__device__ __forceinline__ float row_warp_sums(float (&q)[M]) {
+    const int lane = threadIdx.x & 31;
+    int o = 16;
+#pragma unroll
+    for (int m = M; m > 1; m >>= 1, o >>= 1)
+#pragma unroll
+        for (int i = 0; i < m / 2; ++i) {
+            const bool up = lane & o;
+            const float keep = up ? q[2 * i + 1] : q[2 * i], give = up ? q[2 * i] : q[2 * i + 1];
+            q[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+    float s = q[0];
+#pragma unroll
+    for (; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
+}
+// The squares of a row, summed in an order that is the width's alone: that of a block of G times as many threads with a G-th of the
+// pieces each.  Thread t of that block is thread t mod blockDim of this one, which keeps the sums of its G threads apart.
+template <int G, int NV4>
+__device__ __forceinline__ void row_squares(const float4 (&v)[NV4], float* q) {
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+        q[g] = 0.f;
+#pragma unroll
+        for (int i = g; i < NV4; i += G) q[g] += fmaf(v[i].x, v[i].x, v[i].y * v[i].y) + fmaf(v[i].z, v[i].z, v[i].w * v[i].w);
+    }
+}
+// a sum a warp of that block into red; with M = 2 G the second row's are behind red + 8
+template <int G, int M>
+__device__ __forceinline__ void row_put_sums(float (&q)[M], float* red) {
+    const float s = row_warp_sums(q);
+    constexpr int LANES = 32 / M;
+    const int lane = threadIdx.x & 31;
+    if (lane % LANES) return;
+    const int top = lane / LANES, i = M == 8 ? (top >> 2) | (top & 2) | (top & 1) << 2 : M == 4 ? top >> 1 | (top & 1) << 1 : top;
+    red[i / G * 8 + i % G * (int)(blockDim.x >> 5) + (threadIdx.x >> 5)] = s;
+}
+template <int G>
+__device__ __forceinline__ float row_total(const float* red) {
+    const int n = G * (int)(blockDim.x >> 5);
     float q = 0.f;
 #pragma unroll
-    for (int i = 0; i < NV4; ++i) q += (v[i].x * v[i].x + v[i].y * v[i].y) + (v[i].z * v[i].z + v[i].w * v[i].w);
+    for (int i = 0; i < 8; ++i) if (i < n) q += red[i];
     return q;
+}
+// y + v * inv * g (spelled out: the compiler joins products with sums in one size's kernel and not in another's)
+__device__ __forceinline__ float4 row_scaled(const float4& v, float inv, const float4& g, const float4& y) {
+    return make_float4(fmaf(v.x * inv, g.x, y.x), fmaf(v.y * inv, g.y, y.y), fmaf(v.z * inv, g.z, y.z), fmaf(v.w * inv, g.w, y.w));
 }
 __device__ __forceinline__ void row_put(float* row, int k, const float4& y) { ((float4*)row)[k] = y; }
 __device__ __forceinline__ void row_put(__nv_bfloat16* row, int k, const float4& y) {
@@ -190,17 +235,22 @@ __device__ __forceinline__ void row_put(__nv_bfloat16* row, int k, const float4&
     pk.x = *(unsigned*)&p0; pk.y = *(unsigned*)&p1;
     ((uint2*)row)[k] = pk;
 }
-// Pieces a thread and threads a block, or false: rows that are no whole pieces, or longer than 8,192.  Few rows are spread
-// over more threads (the chain is short then), many rows over fewer (a block has more in flight and less to wait for).
-static bool row_shape(int R, int D, uintptr_t addresses, int& nv, int& threads) {
+// Pieces a thread, how many threads of the widest block a thread stands for (row_squares) and threads a block, or false: rows that are
+// no whole pieces, or longer than 8,192.  Many rows are taken by few threads with up to four pieces (a block has more in flight and
+// less to wait for), fewer than 64 by the widest block (the chain is short then): the same numbers from either.
+struct RowShape { int nv, g, threads; };
+static bool row_shape(int R, int D, uintptr_t addresses, RowShape& s) {
     if (D % 4 || D > 8192 || (addresses & 15)) return false;
     const int n4 = D / 4;
-    if (R < 64) nv = n4 <= 256 ? 1 : n4 <= 512 ? 2 : n4 <= 1024 ? 4 : 8;
-    else nv = n4 <= 64 ? 1 : n4 <= 128 ? 2 : n4 <= 1024 ? 4 : 8;
-    threads = ((n4 + nv - 1) / nv + 31) / 32 * 32;
+    s.nv = n4 <= 64 ? 1 : n4 <= 128 ? 2 : n4 <= 1024 ? 4 : 8;
+    s.g = n4 <= 64 ? 1 : n4 <= 128 ? 2 : n4 <= 256 ? 4 : n4 <= 512 ? 2 : 1;
+    s.threads = ((n4 + s.nv - 1) / s.nv + 31) / 32 * 32;
+    if (R < 64) { s.nv /= s.g; s.threads *= s.g; s.g = 1; }
     return true;
 }
-#define ROW_BY_PIECES(CALL) (nv == 1 ? CALL(1) : nv == 2 ? CALL(2) : nv == 4 ? CALL(4) : CALL(8))
+#define ROW_BY_PIECES(S, CALL) \
+    (S.nv == 1 ? CALL(1, 1) : S.nv == 2 ? (S.g == 1 ? CALL(2, 1) : CALL(2, 2)) \
+     : S.nv == 4 ? (S.g == 1 ? CALL(4, 1) : S.g == 2 ? CALL(4, 2) : CALL(4, 4)) : CALL(8, 1))
 
 // ---------------------------------------------------------------------------
 // Normalisation of selected rows of a 32-bit matrix.
@@ -422,14 +472,14 @@ static int launch_norm(const float* x, const int* rows, const float* gamma, cons
     // (the 32-bit path keeps one kernel for every row count, so that a row's result never depends
     // on how many rows come with it)
     if constexpr (sizeof(TO) == 2) {
-        int nv, row_threads;
-        if (R >= 256 && D <= 4096 && row_shape(R, D, (uintptr_t)x | (uintptr_t)out | (uintptr_t)gamma | (uintptr_t)beta, nv, row_threads)) {
+        RowShape shape;
+        if (R >= 256 && D <= 4096 && row_shape(R, D, (uintptr_t)x | (uintptr_t)out | (uintptr_t)gamma | (uintptr_t)beta, shape)) {
             // A block a row up to 4,096 rows, of up to 1,024 columns up to 2,048; above, its threads' share of a row no longer pays for its
             // start (a warp and a block per row, us: 3,000 x 512 4.1 and 4.8, 4,096 x 1,024 5.8 and 6.7, 8,192 x 2,560 29.5 and 32.8).
             if (R <= (D > 1024 ? 4096 : 2048)) {
                 const size_t smem = 2 * (size_t)(D / 4) * sizeof(float);
-#define CALL(N) gl_launch(norm_rows_kernel<TO, N>, dim3(R), dim3(row_threads), smem, stream, 1, x, rows, gamma, beta, out, D, eps, rms)
-                return nv == 1 ? CALL(1) : nv == 2 ? CALL(2) : CALL(4);        // (up to 4,096 columns)
+#define CALL(N) gl_launch(norm_rows_kernel<TO, N>, dim3(R), dim3(shape.threads), smem, stream, 1, x, rows, gamma, beta, out, D, eps, rms)
+                return shape.nv == 1 ? CALL(1) : shape.nv == 2 ? CALL(2) : CALL(4);        // (up to 4,096 columns)
 #undef CALL
             }
             const int n = (D / 4 + 31) / 32;
@@ -837,7 +887,7 @@ rms_scale_add_kernel(const float* a, const float* __restrict__ w, const float* a
 
 // the same by pieces; one branch: a2 and w2 are absent.  2,128 rows of 2,048, two branches and one add: 21.1 -> 11.0 us; 4 rows,
 // launch after launch: 4.3 -> 1.7 us.
-template <int NV4>
+template <int NV4, int G>
 __global__ void __launch_bounds__(256)
 rms_scale_add_rows_kernel(const float* a, const float* __restrict__ w, const float* a2, const float* __restrict__ w2,
                           const float* add0, const float* add1, const float* add2, float* out, int D, float eps, float alpha) {
@@ -863,23 +913,25 @@ rms_scale_add_rows_kernel(const float* a, const float* __restrict__ w, const flo
 #pragma unroll
         for (int i = 0; i < NV4; ++i) { sum[i].x += t[i].x; sum[i].y += t[i].y; sum[i].z += t[i].z; sum[i].w += t[i].w; }
     }
-    float q = gl_warp_sum(row_squares(v)), q2 = a2 ? gl_warp_sum(row_squares(u)) : 0.f;
-    if ((threadIdx.x & 31) == 0) { red[threadIdx.x >> 5] = q; red[8 + (threadIdx.x >> 5)] = q2; }
+    if (a2) {
+        float q[2 * G];
+        row_squares<G>(v, q);
+        row_squares<G>(u, q + G);
+        row_put_sums<G>(q, red);
+    } else {
+        float q[G];
+        row_squares<G>(v, q);
+        row_put_sums<G>(q, red);
+    }
     __syncthreads();
-    q = q2 = 0.f;
-    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) { q += red[i]; q2 += red[8 + i]; }      // same order in every thread
+    const float q = row_total<G>(red), q2 = a2 ? row_total<G>(red + 8) : 0.f;
     const float inv = alpha / sqrtf(q / (float)D + eps), inv2 = alpha / sqrtf(q2 / (float)D + eps);
 #pragma unroll
     for (int i = 0; i < NV4; ++i) {
         const int k = threadIdx.x + i * blockDim.x;
         if (k >= n4) break;
-        float4 y = make_float4(v[i].x * inv * g[i].x, v[i].y * inv * g[i].y, v[i].z * inv * g[i].z, v[i].w * inv * g[i].w);
-        if (a2) {
-            y.x += u[i].x * inv2 * g2[i].x; y.y += u[i].y * inv2 * g2[i].y;
-            y.z += u[i].z * inv2 * g2[i].z; y.w += u[i].w * inv2 * g2[i].w;
-        }
-        y.x += sum[i].x; y.y += sum[i].y; y.z += sum[i].z; y.w += sum[i].w;
-        row_put(out + base, k, y);
+        const float4 y = row_scaled(v[i], inv, g[i], sum[i]);
+        row_put(out + base, k, a2 ? row_scaled(u[i], inv2, g2[i], y) : y);
     }
 }
 
@@ -889,14 +941,14 @@ GL_API int gl_rms_scale_add(const float* a, const float* w, const float* a2, con
                             float* out, int R, int D, float eps, float alpha, cudaStream_t stream) {
     if (R <= 0) return GL_OK;
     if (D <= 0 || (a2 && !w2)) return GL_ERR_SHAPE;
-    int nv, threads;
+    RowShape shape;
     if (row_shape(R, D, (uintptr_t)a | (uintptr_t)w | (uintptr_t)a2 | (uintptr_t)w2 | (uintptr_t)add0 | (uintptr_t)add1
-                        | (uintptr_t)add2 | (uintptr_t)out, nv, threads)) {
-#define CALL(N) gl_launch(rms_scale_add_rows_kernel<N>, dim3((unsigned)R), dim3(threads), 0, stream, 1, a, w, a2, w2, add0, add1, add2, out, D, eps, alpha)
-        return ROW_BY_PIECES(CALL);
+                        | (uintptr_t)add2 | (uintptr_t)out, shape)) {
+#define CALL(N, G) gl_launch(rms_scale_add_rows_kernel<N, G>, dim3((unsigned)R), dim3(shape.threads), 0, stream, 1, a, w, a2, w2, add0, add1, add2, out, D, eps, alpha)
+        return ROW_BY_PIECES(shape, CALL);
 #undef CALL
     }
-    threads = D >= 2048 ? 256 : (D >= 512 ? 128 : 64);
+    const int threads = D >= 2048 ? 256 : (D >= 512 ? 128 : 64);
     return gl_launch(rms_scale_add_kernel, dim3((unsigned)R), dim3(threads), 0, stream, 1, a, w, a2, w2, add0, add1, add2, out, R, D, eps, alpha);
 }
 
@@ -945,7 +997,7 @@ rms_norm_pair_kernel(const float* x, const float* __restrict__ g1, const float* 
 }
 
 // the same by pieces, a block a row.  2,128 rows of 2,048: 29.5 -> 6.1 us; 4 rows: 3.2 -> 1.4 us.
-template <typename TO, int NV4>
+template <typename TO, int NV4, int G>
 __global__ void __launch_bounds__(256)
 rms_norm_pair_rows_kernel(const float* x, const float* __restrict__ g1, const float* __restrict__ g2,
                           TO* __restrict__ out1, TO* __restrict__ out2, int D, float eps) {
@@ -958,11 +1010,11 @@ rms_norm_pair_rows_kernel(const float* x, const float* __restrict__ g1, const fl
     row_weights(b, g2, n4);
     gl_grid_wait();
     row_pieces(v, x + base, n4);
-    float q = gl_warp_sum(row_squares(v));
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = q;
+    float part[G];
+    row_squares<G>(v, part);
+    row_put_sums<G>(part, red);
     __syncthreads();
-    q = 0.f;
-    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) q += red[i];          // same order in every thread
+    const float q = row_total<G>(red);
     const float inv = (float)(1.0 / sqrt((double)(q / (float)D + eps)));   // in 64-bit, as the single norm takes it
 #pragma unroll
     for (int i = 0; i < NV4; ++i) {
@@ -976,9 +1028,9 @@ rms_norm_pair_rows_kernel(const float* x, const float* __restrict__ g1, const fl
 
 template <typename TO>
 static int launch_rms_norm_pair_rows(const float* x, const float* g1, const float* g2, TO* out1, TO* out2, int R, int D, float eps,
-                                     int nv, int threads, cudaStream_t stream) {
-#define CALL(N) gl_launch(rms_norm_pair_rows_kernel<TO, N>, dim3((unsigned)R), dim3(threads), 0, stream, 1, x, g1, g2, out1, out2, D, eps)
-    return ROW_BY_PIECES(CALL);
+                                     const RowShape& shape, cudaStream_t stream) {
+#define CALL(N, G) gl_launch(rms_norm_pair_rows_kernel<TO, N, G>, dim3((unsigned)R), dim3(shape.threads), 0, stream, 1, x, g1, g2, out1, out2, D, eps)
+    return ROW_BY_PIECES(shape, CALL);
 #undef CALL
 }
 
@@ -986,11 +1038,11 @@ GL_API int gl_rms_norm_pair(const float* x, const float* g1, const float* g2, vo
                             int R, int D, float eps, cudaStream_t stream) {
     if (R <= 0) return GL_OK;
     if (D <= 0) return GL_ERR_SHAPE;
-    int nv, threads;
-    if (row_shape(R, D, (uintptr_t)x | (uintptr_t)g1 | (uintptr_t)g2 | (uintptr_t)out1 | (uintptr_t)out2, nv, threads)) {
-        if (out_dtype == GL_F32) return launch_rms_norm_pair_rows(x, g1, g2, (float*)out1, (float*)out2, R, D, eps, nv, threads, stream);
+    RowShape shape;
+    if (row_shape(R, D, (uintptr_t)x | (uintptr_t)g1 | (uintptr_t)g2 | (uintptr_t)out1 | (uintptr_t)out2, shape)) {
+        if (out_dtype == GL_F32) return launch_rms_norm_pair_rows(x, g1, g2, (float*)out1, (float*)out2, R, D, eps, shape, stream);
         if (out_dtype == GL_BF16)
-            return launch_rms_norm_pair_rows(x, g1, g2, (__nv_bfloat16*)out1, (__nv_bfloat16*)out2, R, D, eps, nv, threads, stream);
+            return launch_rms_norm_pair_rows(x, g1, g2, (__nv_bfloat16*)out1, (__nv_bfloat16*)out2, R, D, eps, shape, stream);
         return GL_ERR_DTYPE;
     }
     if (R >= 64) {
@@ -999,7 +1051,7 @@ GL_API int gl_rms_norm_pair(const float* x, const float* g1, const float* g2, vo
         if (out_dtype == GL_BF16) return gl_launch(rms_norm_pair_kernel<__nv_bfloat16, 1>, grid, dim3(256), 0, stream, 1, x, g1, g2, (__nv_bfloat16*)out1, (__nv_bfloat16*)out2, R, D, eps);
         return GL_ERR_DTYPE;
     }
-    threads = D >= 2048 ? 256 : (D >= 512 ? 128 : 64);
+    const int threads = D >= 2048 ? 256 : (D >= 512 ? 128 : 64);
     if (out_dtype == GL_F32) return gl_launch(rms_norm_pair_kernel<float, 0>, dim3((unsigned)R), dim3(threads), 0, stream, 1, x, g1, g2, (float*)out1, (float*)out2, R, D, eps);
     if (out_dtype == GL_BF16) return gl_launch(rms_norm_pair_kernel<__nv_bfloat16, 0>, dim3((unsigned)R), dim3(threads), 0, stream, 1, x, g1, g2, (__nv_bfloat16*)out1, (__nv_bfloat16*)out2, R, D, eps);
     return GL_ERR_DTYPE;
@@ -1063,7 +1115,7 @@ post_norm_add_kernel(const float* a, const float* b, const float* __restrict__ w
 }
 
 // the same by pieces.  2,128 rows of 2,048: 21.1 -> 9.8 us; 1 row: 3.9 -> 1.5 us.
-template <int NV4>
+template <int NV4, int G>
 __global__ void __launch_bounds__(256)
 post_norm_add_rows_kernel(const float* a, const float* b, const float* __restrict__ w, const float* add, float* out,
                           __nv_bfloat16* rounded, int D, float eps, float sa, float sb) {
@@ -1085,18 +1137,17 @@ post_norm_add_rows_kernel(const float* a, const float* b, const float* __restric
         for (int i = 0; i < NV4; ++i) v[i] = make_float4(sa * v[i].x, sa * v[i].y, sa * v[i].z, sa * v[i].w);
     }
     row_pieces(u, add + base, n4);
-    float q = gl_warp_sum(row_squares(v));
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = q;
+    float part[G];
+    row_squares<G>(v, part);
+    row_put_sums<G>(part, red);
     __syncthreads();
-    q = 0.f;
-    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) q += red[i];          // same order in every thread
+    const float q = row_total<G>(red);
     const float inv = 1.0f / sqrtf(q / (float)D + eps);
 #pragma unroll
     for (int i = 0; i < NV4; ++i) {
         const int k = threadIdx.x + i * blockDim.x;
         if (k >= n4) break;
-        const float4 y = make_float4(u[i].x + v[i].x * inv * g[i].x, u[i].y + v[i].y * inv * g[i].y,
-                                     u[i].z + v[i].z * inv * g[i].z, u[i].w + v[i].w * inv * g[i].w);
+        const float4 y = row_scaled(v[i], inv, g[i], u[i]);
         row_put(out + base, k, y);
         if (rounded) row_put(rounded + base, k, y);
     }
@@ -1108,13 +1159,13 @@ GL_API int gl_post_norm_add(const float* a, const float* b, const float* w, cons
     if (D <= 0 || !a || !w || !add || !out) return GL_ERR_SHAPE;
     const size_t smem = (size_t)D * sizeof(float);
     if (smem > 48 * 1024) return GL_ERR_SMEM;
-    int nv, threads;
-    if (row_shape(R, D, (uintptr_t)a | (uintptr_t)b | (uintptr_t)w | (uintptr_t)add | (uintptr_t)out | (uintptr_t)rounded, nv, threads)) {
-#define CALL(N) gl_launch(post_norm_add_rows_kernel<N>, dim3((unsigned)R), dim3(threads), 0, stream, 1, a, b, w, add, out, (__nv_bfloat16*)rounded, D, eps, sa, sb)
-        return ROW_BY_PIECES(CALL);
+    RowShape shape;
+    if (row_shape(R, D, (uintptr_t)a | (uintptr_t)b | (uintptr_t)w | (uintptr_t)add | (uintptr_t)out | (uintptr_t)rounded, shape)) {
+#define CALL(N, G) gl_launch(post_norm_add_rows_kernel<N, G>, dim3((unsigned)R), dim3(shape.threads), 0, stream, 1, a, b, w, add, out, (__nv_bfloat16*)rounded, D, eps, sa, sb)
+        return ROW_BY_PIECES(shape, CALL);
 #undef CALL
     }
-    threads = D >= 2048 ? 256 : (D >= 512 ? 128 : 64);
+    const int threads = D >= 2048 ? 256 : (D >= 512 ? 128 : 64);
     return gl_launch(post_norm_add_kernel, dim3((unsigned)R), dim3(threads), smem, stream, 1, a, b, w, add, out,
                      (__nv_bfloat16*)rounded, D, eps, sa, sb);
 }
