@@ -446,8 +446,10 @@ __device__ __forceinline__ void mt_gates(const MemoryChunkArgs& a, int h, int t_
         const double up = __shfl_up_sync(0xffffffffu, sum, o);
         if (lane >= o) sum += up;
     }
+    // (from the tokens before alone: taken as the sum up to the next token less that token's, it would be NaN where that one is)
+    const double before = __shfl_up_sync(0xffffffffu, sum, 1);
+    cum[2 * lane] = (lane > 0 ? before : 0.0) + x[0];
     cum[2 * lane + 1] = sum;
-    cum[2 * lane] = sum - x[1];
 }
 
 // A block's share of the rows [0, n) of q or k (column ``off`` of proj on): all of a thread's pieces are asked for at once (load),

@@ -123,3 +123,28 @@ def test_a_value_that_is_no_number_stays_behind_its_token(kind, H, D, V, KVH, ha
         lost = torch.zeros_like(S, dtype=torch.bool)
         lost[2, 1, :, col] = True
         assert not torch.isfinite(S[lost]).any() and torch.equal(S[~lost], S0[~lost])
+
+
+@pytest.mark.parametrize("what", ["gate", "second gate", "key", "query"])
+@pytest.mark.parametrize("place", [74, 75])                  # an even and an odd place of a chunk: a lane holds two tokens' gates
+@pytest.mark.parametrize("kind,H,D,V,KVH,half", SIZES)
+def test_a_gate_or_key_that_is_no_number_stays_behind_its_token(kind, H, D, V, KVH, half, place, what, monkeypatch):
+    """A NaN in a gate or a key shows in its heads' rows from its token on, one in a query in its own row, in its sequence alone; every
+    other row is the same bit for bit."""
+    from gopherllm_b200 import ops
+    if kind == 3 and what == "second gate":
+        pytest.skip("the plain decay has one gate")
+    monkeypatch.setattr(ops, "memory_chunk_tokens", lambda *a: 64)
+    qlens = [70, 130, 64]
+    proj, call, _ = make(kind, H, D, V, KVH, half, qlens, 5)
+    whole, _ = call()
+    at, end, KD, off = qlens[0] + place, qlens[0] + qlens[1], KVH * D, 2 * KVH * D + H * V
+    heads = [H - 1] if "gate" in what else list(range((KVH - 1) * (H // KVH), H))
+    p = proj.clone()
+    p[at, {"gate": off + H - 1, "second gate": off + 2 * H - 1, "key": 2 * KD - 1, "query": KD - 1}[what]] = float("nan")
+    got, _ = call(p)
+    hit = torch.zeros(sum(qlens), H, V, dtype=torch.bool)
+    for h in heads:
+        hit[at:at + 1 if what == "query" else end, h] = True
+    hit = hit.view(sum(qlens), H * V)
+    assert not torch.isfinite(got[hit]).any() and torch.equal(got[~hit], whole[~hit])
