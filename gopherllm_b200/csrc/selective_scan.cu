@@ -275,7 +275,7 @@ selective_carry_kernel(SelectiveScanArgs a) {
 __device__ __forceinline__ unsigned long long ss_decay2(unsigned long long x2) {
     const auto both = [](float v) { return mc_pack(v, v); };
     const float2 x = mc_unpack(x2);
-    const bool gone0 = x.x < -87.f, gone1 = x.y < -87.f;            // (a NaN stays)
+    const bool gone0 = x.x < -87.f, gone1 = x.y < -87.f;
     const unsigned long long y = mc_pack(gone0 ? -87.f : x.x, gone1 ? -87.f : x.y);
     const unsigned long long t = mc_fma2(y, both(1.44269504f), both(12582912.f));       // k in the low bits
     const unsigned long long k = mc_fma2(t, both(1.f), both(-12582912.f));
@@ -290,7 +290,8 @@ __device__ __forceinline__ unsigned long long ss_decay2(unsigned long long x2) {
     const float2 e = mc_unpack(p), n = mc_unpack(t);
     const float r0 = __int_as_float(__float_as_int(e.x) + (__float_as_int(n.x) << 23));
     const float r1 = __int_as_float(__float_as_int(e.y) + (__float_as_int(n.y) << 23));
-    return mc_pack(gone0 ? 0.f : r0, gone1 ? 0.f : r1);
+    // (a NaN is handed on: the bits put together above are no NaN's)
+    return mc_pack(gone0 ? 0.f : x.x != x.x ? x.x : r0, gone1 ? 0.f : x.y != x.y ? x.y : r1);
 }
 
 // MODE 1: a chunk from a zero state, no outputs.  MODE 2: a chunk from its start.

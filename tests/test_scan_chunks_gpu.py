@@ -42,3 +42,42 @@ def test_endless_and_harsh_steps_in_chunks(monkeypatch):
     ended[45, ::3] = float("inf")
     got = run(ended)
     assert torch.isfinite(got[:45]).all() and torch.isfinite(got[:, 1::3]).all() and (got[45:, ::3] == float("inf")).all()
+
+
+def scan_call(C, N, T, seed=2):
+    """Positive inputs of one run, and the call with some of them replaced."""
+    from gopherllm_b200 import ops
+    g = torch.Generator().manual_seed(seed)
+    up = lambda *s: torch.rand(*s, generator=g) + 0.1  # noqa: E731
+    inputs = dict(x=up(T, C), bc=up(T, 2 * N), z=up(T, C), dtp=up(T, C), a_log=up(C, N) - 1.0, d_skip=up(C))
+    state = up(1, C * N)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+    ctx = SimpleNamespace(seq_slot=i32([0]), seq_qstart=i32([0]), seq_qlen=i32([T]), n_seqs=1, max_qlen=T, n_tokens=T)
+
+    def run(**other):
+        t = {k: v.cuda() for k, v in {**inputs, **other}.items()}
+        kept = state.cuda()
+        out = ops.selective_scan(t["x"], t["dtp"], t["bc"], t["z"], 0, t["a_log"], t["d_skip"], kept, ctx)
+        return out.cpu(), kept.cpu()
+    return inputs, run
+
+
+@pytest.mark.parametrize("N", [16, 5])
+def test_a_decay_that_is_no_number(N, monkeypatch):
+    """A rate that is NaN, and an infinite one at a step of zero: the channel is NaN from there on, as in the walk in one piece."""
+    from gopherllm_b200 import ops
+    C, T, at = 40, 100, 45
+    inputs, run = scan_call(C, N, T)
+    rate, step = inputs["a_log"].clone(), inputs["dtp"].clone()
+    rate[3, N // 2], rate[7, N - 1] = float("nan"), float("inf")
+    step[at, 7] = -200.0                              # (softplus of it is zero)
+    both = []
+    for tokens in (0, 32):
+        monkeypatch.setattr(ops, "scan_chunk_tokens", lambda *a: tokens)
+        both.append(run(a_log=rate, dtp=step))
+    for piece, chunks in zip(*both):
+        assert torch.equal(piece.isnan(), chunks.isnan())
+        assert torch.allclose(piece, chunks, rtol=1e-5, atol=1e-6, equal_nan=True)
+    out = both[1][0]
+    assert out[:, 3].isnan().all() and out[at:, 7].isnan().all() and torch.isfinite(out[:at, 7]).all()
+    assert torch.isfinite(out[:, [c for c in range(C) if c not in (3, 7)]]).all()
