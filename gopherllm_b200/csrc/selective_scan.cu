@@ -294,8 +294,8 @@ __device__ __forceinline__ unsigned long long ss_decay2(unsigned long long x2) {
     return mc_pack(gone0 ? 0.f : x.x != x.x ? x.x : r0, gone1 ? 0.f : x.y != x.y ? x.y : r1);
 }
 
-// MODE 1: a chunk from a zero state, no outputs.  MODE 2: a chunk from its start.
-template <typename TA, int MODE>
+// MODE 1: a chunk from a zero state, no outputs.  MODE 2: a chunk from its start.  FULL: N == SC_STATE.
+template <typename TA, int MODE, bool FULL>
 __global__ void __launch_bounds__(RC_THREADS, 4)
 selective_chunk_kernel(SelectiveScanArgs a) {
     __shared__ __align__(16) float bcs[SC_TOKENS][2 * SC_STATE];    // B, then C
@@ -353,14 +353,16 @@ selective_chunk_kernel(SelectiveScanArgs a) {
                 if (g0 + u >= ns) break;
                 const float dt = rc_softplus(d[u]), dx = dt * x[u];
                 if (MODE == 1) dt_sum += dt;
-                const unsigned long long dt2 = mc_pack(dt, dt), dx2 = mc_pack(dx, dx);
+                const unsigned long long dt2 = mc_pack(dt, dt);
+                // (nothing enters a state that does not exist: an infinite input times its B of zero would be NaN)
+                auto dx2 = [&](int i) { return mc_pack(FULL || 2 * i < N ? dx : 0.f, FULL || 2 * i + 1 < N ? dx : 0.f); };
                 unsigned long long y2 = mc_pack(0.f, 0.f);
                 const ulonglong2* row = (const ulonglong2*)bcs[g0 + u];
 #pragma unroll
                 for (int i = 0; i < SC_STATE / 2; i += 2) {
                     const ulonglong2 B = row[i / 2];
-                    S[i] = mc_fma2(ss_decay2(mc_mul2(dt2, A[i])), S[i], mc_mul2(dx2, B.x));
-                    S[i + 1] = mc_fma2(ss_decay2(mc_mul2(dt2, A[i + 1])), S[i + 1], mc_mul2(dx2, B.y));
+                    S[i] = mc_fma2(ss_decay2(mc_mul2(dt2, A[i])), S[i], mc_mul2(dx2(i), B.x));
+                    S[i + 1] = mc_fma2(ss_decay2(mc_mul2(dt2, A[i + 1])), S[i + 1], mc_mul2(dx2(i + 1), B.y));
                     if (MODE == 2) {
                         const ulonglong2 Cn = row[SC_STATE / 4 + i / 2];
                         y2 = mc_fma2(S[i], Cn.x, y2);
@@ -390,12 +392,15 @@ selective_chunk_kernel(SelectiveScanArgs a) {
 template <typename TA>
 static int launch_selective_chunks(const SelectiveScanArgs& a, cudaStream_t stream) {
     const dim3 grid((a.C + RC_THREADS - 1) / RC_THREADS, a.B, a.n_chunks);
-    int rc = gl_launch_in_order(selective_chunk_kernel<TA, 1>, grid, dim3(RC_THREADS), 0, stream, a);
+    const bool full = a.N == SC_STATE;
+    int rc = full ? gl_launch_in_order(selective_chunk_kernel<TA, 1, true>, grid, dim3(RC_THREADS), 0, stream, a)
+                  : gl_launch_in_order(selective_chunk_kernel<TA, 1, false>, grid, dim3(RC_THREADS), 0, stream, a);
     if (rc != 0) return rc;
     const long long n = (long long)a.C * a.N;
     rc = gl_launch(selective_carry_kernel, dim3((unsigned)((n + 127) / 128), a.B), dim3(128), 0, stream, 1, a);
     if (rc != 0) return rc;
-    return gl_launch_in_order(selective_chunk_kernel<TA, 2>, grid, dim3(RC_THREADS), 0, stream, a);
+    return full ? gl_launch_in_order(selective_chunk_kernel<TA, 2, true>, grid, dim3(RC_THREADS), 0, stream, a)
+                : gl_launch_in_order(selective_chunk_kernel<TA, 2, false>, grid, dim3(RC_THREADS), 0, stream, a);
 }
 
 template <typename TA, int NPT>

@@ -62,6 +62,23 @@ def scan_call(C, N, T, seed=2):
     return inputs, run
 
 
+# states that fill the registers and that leave some of them unused
+@pytest.mark.parametrize("N", [16, 13, 12, 5, 1])
+def test_endless_steps_and_inputs_in_states_of_any_size(N, monkeypatch):
+    """An infinite step, and an infinite input, write infinity from their token on in their channel alone."""
+    from gopherllm_b200 import ops
+    monkeypatch.setattr(ops, "scan_chunk_tokens", lambda *a: 32)
+    C, T, at = 40, 100, 45
+    inputs, run = scan_call(C, N, T)
+    whole, _ = run()
+    for name in ("dtp", "x"):
+        t = inputs[name].clone()
+        t[at, ::3] = float("inf")
+        got, kept = run(**{name: t})
+        assert torch.equal(got[:at], whole[:at]) and torch.equal(got[:, 1::3], whole[:, 1::3]), name
+        assert (got[at:, ::3] == float("inf")).all() and (kept.view(C, N)[::3] == float("inf")).all(), name
+
+
 @pytest.mark.parametrize("N", [16, 5])
 def test_a_decay_that_is_no_number(N, monkeypatch):
     """A rate that is NaN, and an infinite one at a step of zero: the channel is NaN from there on, as in the walk in one piece."""
