@@ -11,15 +11,12 @@
 // (model.go:2707-2710); nothing else masks.
 //
 // A sequence that brings one token has one query row for a block of eight warps: there, from
-// AG_SHARE_FROM pages on, the warps share the row's half pages (half page i with warp i mod 8, straight
-// from the cache, no tiles), and their softmaxes are merged in the warps' order.  What bounds
-// such a row is the chain of trips to memory, half a page after the other: 4 sequences of 16 to 300
-// positions, 32 heads of 64 in 32 bits, took 57 us a launch with one warp walking all pages, 17.5 with
-// whole pages shared and their values asked for behind their keys, now 9.2; 1 x 2,000 385, 92 and 33;
-// 16 heads of 100 in bfloat16, 64 x 300, 200, 114 and 117 (keys read two
-// bytes at a time: 268).  On fewer pages the tiles' wide loads are ahead (1 x 10 positions, 8
-// heads of 40: 12 us with tiles, 16 without; 1 x 100 23 and 29; 16 x 128 29 and 31).  The form
-// depends on the sequence's own run alone, so a row still does not depend on the batch around it.
+// AG_SHARE_FROM pages on, the warps share the row's pages or half pages (ag_one_token), and their softmaxes are merged in the
+// warps' order.  What bounds such a row is the chain of trips to memory, half a page after the other.  us a launch, one warp
+// walking all pages / whole pages shared, values asked for behind their keys / now, 32 bits: 4 sequences of 16 to 300 positions, 32
+// heads of 64 57 / 17.5 / 9; 1 x 2,000 385 / 92 / 28; 16 heads of 100, 64 x 300 - / 186 / 124, 16 x 2,000 - / 314 / 163.
+// On fewer pages the tiles' wide loads are ahead (1 x 10 positions, 8 heads of 40: 12 us with tiles, 16 without; 1 x 100 23 and
+// 29; 16 x 128 29 and 31).  The form depends on the sequence's own run alone, so a row still does not depend on the batch around it.
 #include <type_traits>
 
 #include "common.cuh"
@@ -87,10 +84,12 @@ __device__ __forceinline__ float ag_dot(const float* q, const __nv_bfloat16* k, 
     return s;
 }
 
-// The row of a sequence that brings one token, its keys lo..p shared out among the block's warps by half pages, straight from
-// the cache.  q0: the scaled query in shared memory; part: shared memory for the warps' sums.  A half page's values are asked
-// for together with its keys (where a lane's share of them, 32 numbers a dim, fits its registers), so that it costs one trip to
-// memory and not one for the keys and four for the values.
+// The row of a sequence that brings one token, its keys lo..p shared out among the block's warps, straight from the cache: by half
+// pages where that spares the longest warp a half page (one to four pages more than whole rounds of eight), by whole pages where it
+// does not (five: ten half pages are two rounds of eight warps, as five pages are; 64 x 300 positions, 8 heads of 256 in 32 bits, 306 us
+// by halves, 266 by pages).  q0: the scaled query in shared memory; part: shared memory for the warps' sums.  A half page's values
+// are asked for together with its keys (where a lane's share of them, 32 numbers a dim, fits its registers), so that it costs one
+// trip to memory and not one for the keys and four for the values.
 template <typename TA, typename TC, int NACC, bool AHEAD>
 __device__ __forceinline__ void ag_one_token(const AttnArgs& a, const float* q0, float* part, int b, int h, int p, int lo) {
     const int hd = a.hd, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = h / (a.nH / a.nKV);
@@ -100,7 +99,11 @@ __device__ __forceinline__ void ag_one_token(const AttnArgs& a, const float* q0,
     for (int i = 0; i < NACC; ++i) acc[i] = 0.f;
     float m = -INFINITY, l = 0.f;
     int seen = 0x7fffffff, lost = -1;      // the first key of the first half page taken, and of the last one left out for a NaN
-    for (int j0 = (lo / 32 + warp) * 32; j0 <= p; j0 += AG_ROWS * 32) {
+    const int span = ((p / GL_PAGE - lo / GL_PAGE) & (AG_ROWS - 1)) < AG_ROWS / 2 ? 32 : GL_PAGE;      // keys a warp takes at a time
+    for (int j1 = (lo / span + warp) * span; j1 <= p; j1 += AG_ROWS * span)
+#pragma unroll 1
+    for (int j0 = j1; j0 < j1 + span && j0 <= p; j0 += 32) {
+        if (j0 + 31 < lo) continue;
         const int page = gl_checked(pg[gl_checked(j0 / GL_PAGE, a.max_pages, GL_BAD_POSITION)], a.n_pages > 0 ? a.n_pages : 0x7fffffff, GL_BAD_PAGE);
         const size_t at = (((size_t)page * a.nKV + g) * GL_PAGE + j0 % GL_PAGE) * hd;
         const TC* kp = (const TC*)a.k_cache + at;
@@ -282,8 +285,8 @@ template <typename TA, typename TC, int NACC>
 __global__ void __launch_bounds__(AG_ROWS * 32)
 attn_generic_kernel(AttnArgs a) { ag_rows<TA, TC, NACC>(a); }
 
-// Heads of more than 96: as many blocks an SM as shared memory allows (a prompt of 1,000 tokens, 16 heads of 100 in bfloat16: 742 us
-// with the compiler's choice of registers, 627 so; the smaller heads lose by any limit, up to half of their rate).
+// Heads of more than 96 (of them those that are no whole 16-byte pieces come here): as many blocks an SM as shared memory allows (a prompt
+// of 1,000 tokens, 16 heads of 100 in bfloat16, 742 us with the compiler's choice of registers, 627 so; smaller heads lose by any limit).
 template <typename TA, typename TC, int NACC>
 __global__ void __launch_bounds__(AG_ROWS * 32, NACC <= 4 ? 4 : NACC <= 6 ? 3 : 2)
 attn_generic_wide_kernel(AttnArgs a) { ag_rows<TA, TC, NACC>(a); }
@@ -293,7 +296,7 @@ attn_generic_wide_kernel(AttnArgs a) { ag_rows<TA, TC, NACC>(a); }
 // their dims, half pages one after the other, values in ascending order of their keys), so it is the same number from either.
 // What bounds it: shared-memory loads and multiply-adds about evenly.  hd: a multiple of 4.
 template <typename TA, typename TC, int NACC, int R>
-__global__ void __launch_bounds__(AG_ROWS * 32, R > 1 || NACC <= 3 ? 2 : NACC <= 4 ? 4 : NACC <= 6 ? 3 : 2)
+__global__ void __launch_bounds__(AG_ROWS * 32, R == 1 && NACC == 4 ? 3 : 2)
 attn_generic_rows_kernel(AttnArgs a) {
     extern __shared__ __align__(16) float smem[];
     const int hd = a.hd, ks = hd + 4;       // (eight rows' 16-byte pieces fall on different banks)
@@ -437,22 +440,36 @@ static int launch_generic_rows(const AttnArgs& a, cudaStream_t stream) {
         cudaGetLastError();
         return GL_ERR_SMEM;
     }
-    return gl_launch(kern, dim3((a.max_qlen + AG_ROWS * R - 1) / (AG_ROWS * R), a.nH, a.B), dim3(AG_ROWS * 32), smem, stream, 1, a) == 0
-               ? GL_OK : GL_ERR_LAUNCH;
+    const dim3 grid((a.max_qlen + AG_ROWS * R - 1) / (AG_ROWS * R), a.nH, a.B), block(AG_ROWS * 32);
+    // One token a sequence is not launched early: its blocks, few and long, would pile up on whichever SMs have room beside the kernel
+    // before (32 bits, early and in order: 8 x 701 positions, 16 heads of 100 61 and 28 us, 8 of 256 107 and 60; 1 x 20, 32 of 64 3.6 and 4.0).
+    const int rc = a.max_qlen == 1 ? gl_launch_in_order(kern, grid, block, smem, stream, a) : gl_launch(kern, grid, block, smem, stream, 1, a);
+    return rc == 0 ? GL_OK : GL_ERR_LAUNCH;
+}
+
+// Rows a warp of attn_generic_rows_kernel, 0: ag_rows.  It takes heads of whole 16-byte pieces: as many rows, up to four, as leave the
+// SMs a block each (two thirds of them with two).
+// One, two and four rows a warp, 32 bits, us: 4 runs of 16 to 300 tokens, 32 heads of 64 118 / 85 / 77; 2,000 tokens 2273 / 1540 /
+// 1233; 8 heads, 300 tokens 28 / 26 / 34, 100 tokens 9.8 / 10.0 / 13.9; 4 heads of 256, 500 tokens 120 / 97 / 134, 60 tokens 12 /
+// 16 / 22.  (A row a warp, its numbers read one at a time: 144, 2523 and 326 for the first, second and fifth.)
+// One token of each of many sequences in bfloat16, heads of up to 96: ag_rows, whose blocks are more to an SM (64 x 300 positions, rows and
+// ag_rows, us: 32 heads of 64 114 and 85, of 80 183 and 121; 8 x 700 18 and 21).
+static int ag_rows_a_warp(const AttnArgs& a, int cache_bytes) {
+    if (a.hd % 4 || (((uintptr_t)a.k_cache | (uintptr_t)a.v_cache) & (4 * cache_bytes - 1))) return 0;
+    const int sms = ag_sm_count();
+    if (a.max_qlen == 1 && cache_bytes == 2 && a.hd <= 96 && (long long)a.nH * a.B > 2 * sms) return 0;
+    const auto blocks = [&](int rows) { return (long long)((a.max_qlen + rows - 1) / rows) * a.nH * a.B; };
+    if (a.max_qlen > AG_ROWS && blocks(4 * AG_ROWS) >= sms) return 4;
+    if (a.max_qlen > AG_ROWS && 3 * blocks(2 * AG_ROWS) >= 2 * sms) return 2;
+    return 1;
 }
 
 template <typename TA, typename TC, int NACC>
 static int launch_generic(const AttnArgs& a, cudaStream_t stream) {
-    // Heads of whole 16-byte pieces: as many rows a warp, up to four, as leave the SMs a block each (two thirds of them with two).
-    // One, two and four rows a warp, 32 bits, us: 4 runs of 16 to 300 tokens, 32 heads of 64 118 / 85 / 77; 2,000 tokens 2273 / 1540 /
-    // 1233; 8 heads, 300 tokens 28 / 26 / 34, 100 tokens 9.8 / 10.0 / 13.9; 4 heads of 256, 500 tokens 120 / 97 / 134, 60 tokens 12 /
-    // 16 / 22.  (A row a warp, its numbers read one at a time: 144, 2523 and 326 for the first, second and fifth.)
-    if (a.hd % 4 == 0 && !(((uintptr_t)a.k_cache | (uintptr_t)a.v_cache) & (4 * sizeof(TC) - 1))) {
-        const auto blocks = [&](int rows) { return (long long)((a.max_qlen + rows - 1) / rows) * a.nH * a.B; };
-        const int sms = ag_sm_count();
-        if (a.max_qlen > AG_ROWS && blocks(4 * AG_ROWS) >= sms) return launch_generic_rows<TA, TC, NACC, 4>(a, stream);
-        if (a.max_qlen > AG_ROWS && 3 * blocks(2 * AG_ROWS) >= 2 * sms) return launch_generic_rows<TA, TC, NACC, 2>(a, stream);
-        return launch_generic_rows<TA, TC, NACC, 1>(a, stream);
+    switch (ag_rows_a_warp(a, sizeof(TC))) {
+        case 4: return launch_generic_rows<TA, TC, NACC, 4>(a, stream);
+        case 2: return launch_generic_rows<TA, TC, NACC, 2>(a, stream);
+        case 1: return launch_generic_rows<TA, TC, NACC, 1>(a, stream);
     }
     const size_t smem = ((size_t)GL_PAGE * (a.hd + 1) + (size_t)GL_PAGE * a.hd + (size_t)AG_ROWS * a.hd) * sizeof(float);
     void (*kern)(AttnArgs);
@@ -483,6 +500,9 @@ static int dispatch_generic(const AttnArgs& a, cudaStream_t stream) {
         default: return GL_ERR_SHAPE;
     }
 }
+
+// which form a call takes: rows a warp of the kernel for heads of whole 16-byte pieces, or 0
+GL_API int gl_attention_generic_rows(const AttnArgs* args, int cache_dtype) { return ag_rows_a_warp(*args, cache_dtype == GL_BF16 ? 2 : 4); }
 
 GL_API int gl_attention_generic(const AttnArgs* args, int act_dtype, int cache_dtype, cudaStream_t stream) {
     const AttnArgs& a = *args;
