@@ -1251,6 +1251,24 @@ def memory_walks_chunks(kind: int, n_seqs: int, tokens: int, longest: int, eleme
 # of 64 x 128 with a rotation: 1 x 33 19.4 / 19.3 / 20.4, 1 x 64 30 / 19 / 22, 16 x 12 27 / 34 / 34, 16 x 32 53 / 38 / 39.
 MEMORY_PRODUCTS_FROM, MEMORY_PRODUCTS_FROM_MANY, MEMORY_PRODUCTS_MANY = 48, 24, 4
 MEMORY_PRODUCTS_FEW_TOKENS = 128
+# In chunks every run pays for at least one chunk's state going through memory, token by token for its tokens alone: single tokens
+# beside a prompt cost more in chunks the more there are (us a launch, token by token / chunks of 64, a run of 24, 128, 500 tokens
+# beside 63 single ones: gated, 8 heads of 128 x 256 107 / 253, 125 / 275, 368 / 344; plain decay, 64 heads of 128 x 64 144 / 497,
+# 176 / 517, 342 / 594; 16 heads of 64 x 128 30 / 80, 68 / 87, 256 / 119).  Chunks are taken where these estimates say they pay, fitted to
+# 48 such batches (1 to 64 runs of 12 to 1,000 tokens beside 3 to 63 single ones, states of 16,384 to 524,288 numbers: in none of them the
+# chosen form took longer than token by token, in one 3 us longer than the other's 23, and in two 7 % longer).
+MEMORY_PRODUCTS_RATE = {0: 1.17e6, 3: 2.1e6}      # numbers of a state times tokens a us, token by token with the machine full
+
+
+def memory_products_pay(kind: int, n_seqs: int, tokens: int, longest: int, elements: int, chunk: int) -> bool:
+    """Whether a memory of ``elements`` numbers is expected to take less time as products in chunks of ``chunk`` tokens than
+    token by token."""
+    run = (0.33 + 0.2 * elements / 2 ** 19) * longest                    # us: a run's tokens one after the other,
+    all_runs = tokens * elements / MEMORY_PRODUCTS_RATE[kind] + n_seqs * 8 * elements / 3e6      # all tokens, and the states in and out
+    chunks = min(n_seqs * -(-longest // chunk), tokens // chunk + n_seqs)
+    moved = elements * (4 * chunks + 2 * n_seqs) * 4e-6                  # MB: a chunk's state written and read twice; 200 of them stay in L2
+    products = 20.0 + min(moved, 200.0) / 3.7 + max(moved - 200.0, 0.0) / 1.2
+    return 8.0 + max(run, all_runs) + 0.1 * min(run, all_runs) > 1.05 * products
 
 
 def memory_takes_products(kind: int, dtype, ld: int, D: int, V: int, offsets, rot_half: int) -> bool:
@@ -1267,6 +1285,8 @@ def memory_chunk_tokens(kind: int, exact: bool, n_seqs: int, tokens: int, longes
         return 0
     if products and longest >= (MEMORY_PRODUCTS_FROM_MANY if n_seqs >= MEMORY_PRODUCTS_MANY else MEMORY_PRODUCTS_FROM):
         n = MEMORY_CHUNK_TOKENS if tokens > MEMORY_PRODUCTS_FEW_TOKENS else MEMORY_CHUNK_TOKENS_FEW
+        if not memory_products_pay(kind, n_seqs, tokens, longest, H * D * V, n):
+            return 0
         chunks = n_seqs * -(-longest // n)
         if chunks * H * D * V * 4 <= MEMORY_CHUNKS_MAX_BYTES and chunks <= 65535:
             return n
@@ -1318,8 +1338,8 @@ def memory_scan(kind: int, proj: torch.Tensor, state: torch.Tensor, ctx, H: int,
     times q_scale and k_scale.  Either ``decay`` [H] (keep = decay[h], take = 1) or ``gates`` with ``a_log`` and
     ``dt_bias`` [H]: dt = softplus(gates[t, f_off + h] + dt_bias[h]), keep = exp(-exp(a_log[h]) dt), take = dt.
     Long runs of the gated, the bounded-forget and the plain-decay kind (heads of up to MEMORY_CHUNKS_MAX_ROWS rows)
-    are walked as chunks side by side: in 32 bits (and of the plain decay) by the step's longest run alone, in bfloat16 by
-    the lengths of all its runs."""
+    are walked as chunks side by side, or, in bfloat16 with heads of 64 or 128 rows and one decay a token, are products of
+    chunks: in 32 bits by the step's longest run alone, in bfloat16 by the lengths of all its runs."""
     _need(proj, "proj")
     rot_half = 0
     if kind == MEMORY_DECAY:

@@ -17,3 +17,13 @@ def test_rule():
     assert many > 64 and 64 * -(-2000 // many) * 8 * 128 * 256 * 4 <= 2 * ops.MEMORY_CHUNKS_MAX_BYTES
     # without products as before
     assert ops.memory_chunk_tokens(0, False, 1, 100, 100, 8, 128, 256) == 0 and ops.memory_chunk_tokens(3, False, 1, 100, 100, 8, 128, 64) == 0
+
+
+def test_single_tokens_beside_a_run():
+    """Runs of one token pay for a whole chunk: a prompt beside many of them is walked token by token, one beside few is not."""
+    from gopherllm_b200 import ops
+    gated = lambda n, lone: ops.memory_chunk_tokens(0, False, 1 + lone, n + lone, n, 8, 128, 256, True)  # noqa: E731
+    decay = lambda n, lone: ops.memory_chunk_tokens(3, False, 1 + lone, n + lone, n, 64, 128, 64, True)  # noqa: E731
+    assert gated(24, 63) == gated(48, 15) == gated(128, 63) == gated(256, 63) == 0 and gated(128, 15) == gated(1000, 63) == 64
+    assert decay(24, 15) == decay(128, 63) == decay(256, 63) == decay(500, 63) == 0 and decay(256, 15) == decay(300, 0) == 64
+    assert ops.memory_chunk_tokens(0, False, 16, 4800, 300, 8, 128, 256, True) == 64
