@@ -659,10 +659,15 @@ static constexpr size_t mt_outputs_smem() {
     return (size_t)((ROT ? 6 : 2) * MT_TOKENS * (D + 8) + MT_TOKENS * MT_VP + 3 * D * MT_VP) * 2;
 }
 
+// blocks an SM, stated by shared memory: with 128 rows and a rotation one fits, and held to the registers of two it spilled (16 heads
+// of 128 x 128, 2,047 tokens: 181 -> 163 us a launch of all kernels)
+template <int D, bool ROT>
+static constexpr int mt_outputs_blocks() { return 2 * (mt_outputs_smem<D, ROT>() + 4096) <= 227 * 1024 ? 2 : 1; }
+
 // the read-outs of a chunk from its start state, 64 columns a block: eight warps, 16 tokens and 32 columns each (both of a row
 // group's warps take its scores, which are few beside the state's products)
 template <int D, bool ROT, bool GATED>
-__global__ void __launch_bounds__(256, 2)
+__global__ void __launch_bounds__(256, mt_outputs_blocks<D, ROT>())
 memory_chunk_outputs_tc_kernel(MemoryChunkArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ double cum[MT_TOKENS];

@@ -93,14 +93,26 @@ def test_products_and_the_walk(kind, H, D, V, KVH, half, fixed, harsh, chunk, mo
     if kind == 0 and (fixed or harsh):
         pytest.skip("the gated kind has gates of its own")
     monkeypatch.setattr(ops, "memory_chunk_tokens", lambda *a: chunk)
+    launches, check = [], ops._check
+    monkeypatch.setattr(ops, "_check", lambda code, what, kernels=1: (launches.append(kernels), check(code, what, kernels)))
     qlens = [1, 17, 63, 64, 65, 200]
-    proj, call, exact = make(kind, H, D, V, KVH, half, qlens, H + D + V, fixed=fixed, harsh=harsh)
-    want = exact()
-    for got, ref, what in zip(call(), want, ("results", "states")):
-        # a few roundings of 2^-24 of the largest partial sum a token, and of its decays
-        bound = 2 ** -22 * max(qlens) * max(1.0, float(ref.abs().max()))
-        err = float((got.double() - ref).abs().max())
-        assert err <= bound, (what, err, bound)
+    errors = {}
+    for more, form in ((0, "products"), (1, "walk")):            # (rows that begin anywhere are walked)
+        proj, call, exact = make(kind, H, D, V, KVH, half, qlens, H + D + V, ld_more=more, fixed=fixed, harsh=harsh)
+        assert ops.memory_takes_products(kind, proj.dtype, proj.shape[1], D, V, (0, KVH * D, 2 * KVH * D), half) == (form == "products")
+        launches.clear()
+        both = call()
+        assert launches == [(2 if kind == 0 else 1) + (3 if form == "products" else 5 if kind == 0 else 4)], (form, launches)
+        for got, ref, what in zip(both, exact(), ("results", "states")):
+            # a few roundings of 2^-24 of the largest partial sum a token, and of its decays
+            bound = 2 ** -22 * max(qlens) * max(1.0, float(ref.abs().max()))
+            err = float((got.double() - ref).abs().max())
+            assert err <= bound, (form, what, err, bound)
+            errors[form, what] = float((got.double() - ref).norm() / ref.norm())
+    # factors of 24 bits: no further from 64-bit than the walk, but for roundings that fall the other way; factors of two bfloat16
+    # parts, 16 bits, would be off by some 2^-18 each
+    for what in ("results", "states"):
+        assert errors["products", what] <= min(2.0 * errors["walk", what] + 2 ** -24, 1e-6), errors
 
 
 @pytest.mark.parametrize("kind,H,D,V,KVH,half", SIZES)
