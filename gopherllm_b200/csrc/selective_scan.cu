@@ -52,6 +52,7 @@ struct SelectiveScanArgs {
     float* chunk_dt;          // [B, n_chunks, C]
     int chunk_len, n_chunks;
     int one_token;            // every run is one token
+    int by_channel;           // chunks are walked a thread a channel (N <= SC_STATE)
 };
 
 // MODE 0: a run in one piece.  MODE 1: a chunk from a zero state, no outputs.  MODE 2: a chunk from its start.
@@ -435,7 +436,7 @@ static int selective_scan_blocks(const SelectiveScanArgs& a, int npt) {
 
 template <typename TA>
 static int dispatch_selective_scan(const SelectiveScanArgs& a, cudaStream_t stream) {
-    if (a.n_chunks > 1 && a.N <= SC_STATE) return launch_selective_chunks<TA>(a, stream);
+    if (a.n_chunks > 1 && a.by_channel) return a.N <= SC_STATE ? launch_selective_chunks<TA>(a, stream) : GL_ERR_SHAPE;
     static int sms = 0;
     if (!sms) {
         int dev = 0;

@@ -1533,7 +1533,7 @@ class _SelectiveScanArgs(Structure):
                 ("seq_slot", c_void_p), ("seq_qstart", c_void_p), ("seq_qlen", c_void_p),
                 ("B", c_int), ("C", c_int), ("N", c_int), ("z_ld", c_int), ("z_off", c_int), ("state_stride", c_int),
                 ("chunk_state", c_void_p), ("chunk_dt", c_void_p), ("chunk_len", c_int), ("n_chunks", c_int),
-                ("one_token", c_int)]
+                ("one_token", c_int), ("by_channel", c_int)]
 
 
 SCAN_MAX_STATE = 256
@@ -1541,24 +1541,33 @@ SCAN_MAX_STATE = 256
 # and a carry between them): a token-by-token walk leaves most of the machine idle when the sequences are few.
 SCAN_CHUNK_TOKENS = 128     # (a prompt of 2,048 tokens: 11.3 / 11.4 / 13.0 / 15.5 ms with chunks of 64 / 128 / 256 / 512)
 SCAN_CHUNKED_FROM = 1024       # (512 tokens in 4 chunks took 8 % longer than walked in one piece)
-# States of up to SCAN_CHUNK_STATE numbers have walks of their own over chunks, a thread a channel.  In 32 bits when chunks are
-# taken stays a matter of the longest run alone; in bfloat16 they are taken from SCAN_SHORT_CHUNKED_FROM tokens on, and shorter,
-# so that few sequences fill the machine.
-# (us a launch with 4,096 channels of 16, in one piece / chunks of 32 / 64 / 128: 1 x 150 tokens 37 / 43 / 62 / 113, 1 x 200 47 / 46 /
-# 62 / 113, 1 x 500 113 / 76 / 80 / 114, 1 x 1,000 221 / 123 / 135 / 148, 1 x 2,040 449 / 237 / 229 / 256, 4 x 150 98 / 89 / 90 /
-# 122, 16 x 300 619 / 545 / 545 / 526.)
-SCAN_CHUNK_STATE = 16
-SCAN_SHORT_CHUNKED_FROM = 192
-SCAN_SHORT_CHUNK_TOKENS, SCAN_SHORT_CHUNK_TOKENS_FEW, SCAN_SHORT_FEW_TOKENS = 64, 32, 1000
+# States of more than 8 and up to SCAN_CHANNEL_STATE numbers have walks of their own over chunks, a thread a channel: the time of
+# sixteen numbers whatever the state, and of a thread a channel and chunk however few there are.  us a launch, lanes and a thread a
+# channel, chunks of 128 tokens in 32 bits: 4,096 channels of 16, 2,040 tokens 502 / 258, 2,048 of 12 259 / 161, 1,024 of 16, 1,100 tokens
+# 104 / 103, 512 of 16 61 / 103, 64 of 16 40 / 102, 2,048 of 4 84 / 121.  In 32 bits the form follows the model's sizes alone.
+SCAN_CHANNEL_STATE, SCAN_CHANNEL_FROM = 16, 16384
+
+
+def scan_by_channel(C: int, N: int, exact: bool) -> bool:
+    """Whether chunks of a selective scan are walked a thread a channel.  ``exact``: 32-bit inputs."""
+    return 8 < N <= SCAN_CHANNEL_STATE and (not exact or C * N >= SCAN_CHANNEL_FROM)
+
+
+# With them chunks pay, in bfloat16, from SCAN_SHORT_CHUNKED_FROM tokens on, of 64 tokens or, for few tokens and channels, of 32, so that
+# few sequences fill the machine (in 32 bits when chunks are taken stays a matter of the longest run alone).  us a launch with 4,096
+# channels of 16, in one piece / chunks of 32 / of 64: 1 x 200 tokens 47 / 46 / 62, 1 x 500 113 / 76 / 80, 1 x 1,000 221 / 123 / 135,
+# 1 x 2,040 449 / 237 / 229, 16 x 300 619 / 545 / 545; of 64 channels, 1 x 2,040 49 in lanes, 65 with chunks of 64.
+# Single tokens beside a run have their states go through memory for a chunk of their own (200 + 63 of them 116 in one piece, 175 in chunks,
+# 500 + 63 275 and 210): chunks are left where the states of all runs are many for the length of the longest.
+SCAN_SHORT_CHUNKED_FROM, SCAN_SHORT_STATES = 256, 12000
+SCAN_SHORT_CHUNK_TOKENS, SCAN_SHORT_CHUNK_TOKENS_FEW, SCAN_SHORT_FEW = 64, 32, 4_100_000
 
 
 def scan_chunk_tokens(C: int, N: int, exact: bool, n_seqs: int, tokens: int, longest: int) -> int:
     """Tokens a chunk of a selective scan's walk over runs of ``tokens`` in all, 0: in one piece.  ``exact``: 32-bit inputs."""
-    if longest >= SCAN_CHUNKED_FROM and (exact or N > SCAN_CHUNK_STATE):
-        return SCAN_CHUNK_TOKENS
-    if exact or N > SCAN_CHUNK_STATE or longest < SCAN_SHORT_CHUNKED_FROM:
-        return 0
-    n = SCAN_SHORT_CHUNK_TOKENS if tokens > SCAN_SHORT_FEW_TOKENS else SCAN_SHORT_CHUNK_TOKENS_FEW
+    if (exact or not scan_by_channel(C, N, exact) or longest < SCAN_SHORT_CHUNKED_FROM or n_seqs * C * N > SCAN_SHORT_STATES * longest):
+        return SCAN_CHUNK_TOKENS if longest >= SCAN_CHUNKED_FROM else 0
+    n = SCAN_SHORT_CHUNK_TOKENS if tokens * C > SCAN_SHORT_FEW else SCAN_SHORT_CHUNK_TOKENS_FEW
     # every (sequence, chunk) keeps a whole state (and there are at most 65,535 chunks): many long sequences take longer ones
     while n < 1024 and (n_seqs * -(-longest // n) * C * N * 4 > MEMORY_CHUNKS_MAX_BYTES or -(-longest // n) > 65535):
         n *= 2
@@ -1585,11 +1594,12 @@ def selective_scan(x: torch.Tensor, dtp: torch.Tensor, bc: torch.Tensor, z: torc
     a = _SelectiveScanArgs(x.data_ptr(), dtp.data_ptr(), bc.data_ptr(), z.data_ptr(), out.data_ptr(),
                            a_log.data_ptr(), d_skip.data_ptr(), state.data_ptr(),
                            ctx.seq_slot.data_ptr(), ctx.seq_qstart.data_ptr(), ctx.seq_qlen.data_ptr(),
-                           ctx.n_seqs, C, N, z.shape[1], z_off, state.shape[1], None, None, 0, 0, 1 if ctx.max_qlen == 1 else 0)
+                           ctx.n_seqs, C, N, z.shape[1], z_off, state.shape[1], None, None, 0, 0, 1 if ctx.max_qlen == 1 else 0,
+                           1 if scan_by_channel(C, N, x.dtype == torch.float32) else 0)
     kernels = 1
     tokens = scan_chunk_tokens(C, N, x.dtype == torch.float32, ctx.n_seqs, T, ctx.max_qlen)
-    if tokens:
-        chunks = -(-ctx.max_qlen // tokens)
+    chunks = -(-ctx.max_qlen // tokens) if tokens else 1
+    if chunks > 1:
         chunk_state = empty((ctx.n_seqs, chunks, C, N), torch.float32, x.device)
         chunk_dt = empty((ctx.n_seqs, chunks, C), torch.float32, x.device)
         a.chunk_state, a.chunk_dt = chunk_state.data_ptr(), chunk_dt.data_ptr()

@@ -16,6 +16,7 @@ pytestmark = pytest.mark.gpu
 def test_chunks_of_any_length(C, N, tokens, dtype, monkeypatch):
     from gopherllm_b200 import ops
     monkeypatch.setattr(ops, "scan_chunk_tokens", lambda *a: tokens)
+    monkeypatch.setattr(ops, "scan_by_channel", lambda *a: True)
     check_selective_scan(C, N, [64, 1, 131, 65], dtype)
 
 
@@ -24,6 +25,7 @@ def test_endless_and_harsh_steps_in_chunks(monkeypatch):
     state is gone at once leave what is left exact."""
     from gopherllm_b200 import ops
     monkeypatch.setattr(ops, "scan_chunk_tokens", lambda *a: 32)
+    monkeypatch.setattr(ops, "scan_by_channel", lambda *a: True)
     C, N, T = 40, 16, 100
     g = torch.Generator().manual_seed(2)
     up = lambda *s: torch.rand(*s, generator=g) + 0.1  # noqa: E731
@@ -68,6 +70,7 @@ def test_endless_steps_and_inputs_in_states_of_any_size(N, monkeypatch):
     """An infinite step, and an infinite input, write infinity from their token on in their channel alone."""
     from gopherllm_b200 import ops
     monkeypatch.setattr(ops, "scan_chunk_tokens", lambda *a: 32)
+    monkeypatch.setattr(ops, "scan_by_channel", lambda *a: True)
     C, T, at = 40, 100, 45
     inputs, run = scan_call(C, N, T)
     whole, _ = run()
@@ -88,6 +91,7 @@ def test_a_decay_that_is_no_number(N, monkeypatch):
     rate, step = inputs["a_log"].clone(), inputs["dtp"].clone()
     rate[3, N // 2], rate[7, N - 1] = float("nan"), float("inf")
     step[at, 7] = -200.0                              # (softplus of it is zero)
+    monkeypatch.setattr(ops, "scan_by_channel", lambda *a: True)
     both = []
     for tokens in (0, 32):
         monkeypatch.setattr(ops, "scan_chunk_tokens", lambda *a: tokens)

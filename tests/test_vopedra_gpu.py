@@ -224,6 +224,9 @@ def test_long_runs_walked_as_chunks(dtype, monkeypatch):
     from gopherllm_b200 import ops
     monkeypatch.setattr(ops, "SCAN_CHUNK_TOKENS", 16)
     monkeypatch.setattr(ops, "SCAN_CHUNKED_FROM", 32)
+    monkeypatch.setattr(ops, "SCAN_SHORT_CHUNKED_FROM", 32)             # (states of more than 8 numbers in bfloat16 have lines of their own)
+    monkeypatch.setattr(ops, "SCAN_SHORT_CHUNK_TOKENS", 16)
+    monkeypatch.setattr(ops, "SCAN_SHORT_CHUNK_TOKENS_FEW", 16)
     for cfg_name in ("ALPHA", "BETA"):
         cfg = getattr(vm, cfg_name)
         folder = folder_for(cfg_name, cfg, 5, long_memory=True)
@@ -316,7 +319,14 @@ def test_selective_scan_in_chunks_of_several_stages(C, N, qlens, tokens, dtype, 
     from gopherllm_b200 import ops
     monkeypatch.setattr(ops, "SCAN_CHUNKED_FROM", 64)
     monkeypatch.setattr(ops, "SCAN_CHUNK_TOKENS", tokens)
-    check_selective_scan(C, N, qlens, dtype)
+    monkeypatch.setattr(ops, "SCAN_SHORT_CHUNKED_FROM", 64)
+    monkeypatch.setattr(ops, "SCAN_SHORT_CHUNK_TOKENS", tokens)
+    monkeypatch.setattr(ops, "SCAN_SHORT_CHUNK_TOKENS_FEW", tokens)
+    monkeypatch.setattr(ops, "SCAN_SHORT_STATES", 1 << 30)
+    assert ops.scan_chunk_tokens(C, N, dtype == torch.float32, len(qlens), sum(qlens), max(qlens)) == tokens
+    for by_channel in (False, True) if N <= ops.SCAN_CHANNEL_STATE else (False,):       # both walks over chunks, whichever these sizes take
+        monkeypatch.setattr(ops, "scan_by_channel", lambda *a: by_channel)
+        check_selective_scan(C, N, qlens, dtype)
 
 
 def check_selective_scan(C, N, qlens, dtype):
