@@ -28,9 +28,8 @@ static_assert(GL_VALUE_DIM % 16 == 0 && GL_VALUE_DIM >= 16 && GL_VALUE_DIM <= 25
 #define AP_ROW (AP_HD * 2 + 16)       // padded row: 8 consecutive rows fall in distinct banks
 #define AP_VROW (AP_VD * 2 + 16)
 #define AP_TILE (64 * AP_ROW)
-#ifndef AP_VALUE_HEADS                // value heads a block takes at most: their results are AP_VD / 2 registers each
-#define AP_VALUE_HEADS (AP_VD <= 64 ? 4 : AP_VD <= 128 ? 2 : 1)
-#endif
+// value heads a block takes at most: their results are AP_VD / 2 registers each, beside a query's AP_HD / 4
+#define AP_VALUE_HEADS (AP_HD > 128 ? (AP_VD <= 64 ? 2 : 1) : AP_VD <= 64 ? 4 : AP_VD <= 128 ? 2 : 1)
 #define AP_VTILE (64 * AP_VROW)
 
 struct PairsArgs {
@@ -59,6 +58,7 @@ struct PairsArgs {
     const int* seq_base;      // [B] or null: keys and values are not in pages but rows of matrices kv_ld numbers apart, sequence
                               // b's position 0 in row seq_base[b], a head's numbers side by side from column head * size on
     int kv_ld, q_ld;          // q_ld > 0: numbers between two rows of q
+    int T;                    // rows of q (0: not known)
 };
 
 __device__ __forceinline__ unsigned ap_smem(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -107,11 +107,8 @@ __device__ __forceinline__ void ap_load_rows(unsigned dst, const __nv_bfloat16* 
 }
 
 // VG: value heads of a block (of a mixer with nVal of them a query head).  The scores and the softmax of a query head are the same
-// whatever the values, so a block takes as many value heads as its registers hold: with one, a page's scores, exponentials
-// and key tile were computed and fetched once for every value head.
-// 32 query heads and 8 value heads of 64 with a table, the mixing behind them included: runs of 64, 376, 688 and 1,000 tokens 399 us
-// with one value head a block, 404 with two (two blocks an SM instead of three for it), 315 with four; 2,047 tokens 778 and 602;
-// 8 x 40 34 and 29.  The same numbers whichever.
+// whatever the values, so a block may take several: with one, a page's scores, exponentials and key tile are computed and fetched
+// once for every value head.  The same numbers whichever; value_heads_a_block says when several pay.
 template <int VG>
 __global__ void __launch_bounds__(AP_THREADS)
 attn_pairs_tc_kernel(PairsArgs a) {
@@ -606,6 +603,32 @@ static int launch_pairs(const PairsArgs& a, cudaStream_t stream) {
     return gl_launch(attn_pairs_tc_kernel<VG>, grid, dim3(AP_THREADS), smem, stream, 1, a) == 0 ? GL_OK : GL_ERR_LAUNCH;
 }
 
+// Several value heads a block leave fewer and longer blocks, with more registers: they pay where the machine is full all the same.
+// blocks: with one value head each.  us, one / two / four value heads a block, the mixing behind them included (keys / values, query
+// heads on value heads: tokens):
+//   64 / 64, 32 on 8:  300 (1,280 blocks) 47 / 48 / 45, 2,047 863 / 862 / 634;  16 on 4: 300 (320) 21 / 25 / 30, 2,047 (2,048) 243 / 256 / 214
+//   32 / 32, 24 on 6:  300 (720) 27 / 24, 2,047 345 / 272;  8 on 2: 2,047 (512) 70 / 79;  128 / 64, 24 on 6: 2,047 649 / 595
+//   128 / 128, 32 on 8: 300 86 / 74, 2,047 1,859 / 1,376;  8 on 2: 300 (80) 24 / 31;  64 / 128, 24 on 6: 300 (720) 47 / 49
+//   256 / 64, 32 on 8: 40 (256) 15.1 / 15.3 / 18.4, 2,047 1,960 / 1,031 / 1,705;  256 / 128, 32 on 8: 2,047 1,928 / 3,181 (both spill)
+static int value_heads_a_block(const PairsArgs& a) {
+    static int sms = 0;                    // (the same whichever thread finds it first)
+    if (!sms) {
+        int dev = 0, n = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        sms = n > 0 ? n : 148;
+    }
+    long long tiles = (long long)((a.max_qlen + AP_BM - 1) / AP_BM) * a.B;          // (unequal runs have fewer)
+    if (a.T > 0 && tiles > a.T / AP_BM + a.B) tiles = a.T / AP_BM + a.B;
+    const long long blocks = tiles * a.nH * a.nVal;
+    if (AP_VALUE_HEADS >= 4 && a.nVal % 4 == 0 && blocks >= 8 * sms) return 4;
+    // (two of 64 behind keys of up to 64 are no gain: 24 on 6, 2,047 tokens 500 / 506)
+    if (AP_VALUE_HEADS < 2 || a.nVal % 2 || (AP_HD <= 64 && AP_VD > 48 && AP_VD <= 64)) return 1;
+    return blocks >= (AP_HD > 128 ? 1 : AP_VD > 64 ? 6 : 4) * sms ? 2 : 1;
+}
+
+GL_API int gl_attention_pairs_tc_heads(const PairsArgs* args) { return value_heads_a_block(*args); }
+
 GL_API int gl_attention_pairs_tc(const PairsArgs* args, cudaStream_t stream) {
     const PairsArgs& a = *args;
     if (a.B <= 0 || a.max_qlen <= 0) return GL_OK;
@@ -615,8 +638,8 @@ GL_API int gl_attention_pairs_tc(const PairsArgs* args, cudaStream_t stream) {
     if (a.v_in_k && (AP_VD > AP_HD || a.nVal != 1 || (a.nVH > 0 && a.nVH != a.nKV))) return GL_ERR_SHAPE;
     if (a.q_ld % 8 || (a.seq_base && (a.kv_ld <= 0 || a.kv_ld % 8 || a.v_in_k))) return GL_ERR_SHAPE;
     if (a.B > 65535 || a.nH * a.nVal > 65535) return GL_ERR_SHAPE;
-    // as many value heads a block as a power of two up to AP_VALUE_HEADS divides
-    if (a.nVal % 4 == 0 && AP_VALUE_HEADS >= 4) return launch_pairs<AP_VALUE_HEADS >= 4 ? 4 : 1>(a, stream);
-    if (a.nVal % 2 == 0 && AP_VALUE_HEADS >= 2) return launch_pairs<AP_VALUE_HEADS >= 2 ? 2 : 1>(a, stream);
+    const int heads = value_heads_a_block(a);
+    if (heads == 4) return launch_pairs<AP_VALUE_HEADS >= 4 ? 4 : 1>(a, stream);
+    if (heads == 2) return launch_pairs<AP_VALUE_HEADS >= 2 ? 2 : 1>(a, stream);
     return launch_pairs<1>(a, stream);
 }
