@@ -624,7 +624,7 @@ static int value_heads_a_block(const PairsArgs& a) {
     if (AP_VALUE_HEADS >= 4 && a.nVal % 4 == 0 && blocks >= 8 * sms) return 4;
     // (two of 64 behind keys of up to 64 are no gain: 24 on 6, 2,047 tokens 500 / 506)
     if (AP_VALUE_HEADS < 2 || a.nVal % 2 || (AP_HD <= 64 && AP_VD > 48 && AP_VD <= 64)) return 1;
-    return blocks >= (AP_HD > 128 ? 1 : AP_VD > 64 ? 6 : 4) * sms ? 2 : 1;
+    return blocks > (AP_HD > 128 ? 1 : AP_VD > 64 ? 6 : 4) * sms ? 2 : 1;
 }
 
 GL_API int gl_attention_pairs_tc_heads(const PairsArgs* args) { return value_heads_a_block(*args); }
