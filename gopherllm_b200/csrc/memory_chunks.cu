@@ -373,14 +373,17 @@ memory_chunk_carry_kernel(MemoryChunkArgs a) {
 // difference of sums of logarithms; the sums are taken in 64-bit, so that a token that forgets nearly everything leaves the
 // later ones' decays as exact as they were.
 //
-// What bounds it: the tensor cores' mma.sync (about 2,200 products of 16 x 8 x 16 a chunk and head of 128 x 64), then the
-// trips of chunk states through memory.  Token by token on CUDA cores the same took six times the arithmetic instructions.
+// What bounds it: the phases of a block one after the other (fetch, split, products, store) with two or three blocks an SM to fill
+// in: the tensor pipe is active 30 % of the time for the chunks' own states and 23 % for the read-outs, DRAM 11 and 14 %, a fifth of the
+// warps' places taken.  Token by token on CUDA cores the same took six times the
+// arithmetic instructions.
 // With 64 heads of 128 x 64, a run of 2,047 tokens: 426 -> 166 us; 16 heads of 64 x 128 with a rotation 122 -> 78; gated, 8 heads of
 // 128 x 256, runs of 64, 376, 688 and 1,000 tokens 413 -> 120.  Relative error of the results against 64 bits, walk and
 // products: 3.9e-8 and 3.4e-8, fixed decays 2.2e-7 and 1.7e-7, rotated 5.4e-8 and 5.7e-8, gated 2.5e-7 and 1.3e-7.
 //
-// A value that is infinite or NaN reaches its column from its token on and nothing before it (a zero weight times infinity
-// would be NaN in the tokens before): such values are taken out of the products and their column is NaN from there on.
+// What is infinite or NaN reaches nothing before its token: a value shows in its column from its token on (a zero weight times
+// infinity would be NaN in the tokens before: such values are taken out of the products and their column is NaN from there
+// on, also where the walk has infinity), a gate or a key in its head from its token on, a query in its row.
 #define MT_TOKENS 64                 // tokens of a chunk, at most
 #define MT_COLS 64                   // columns of a block
 #define MT_VP (MT_COLS + 8)          // pitches in elements: rows of 16-byte pieces on different banks

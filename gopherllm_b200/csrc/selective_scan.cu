@@ -262,7 +262,7 @@ selective_carry_kernel(SelectiveScanArgs a) {
 // The walks over chunks for states of up to SC_STATE numbers: a thread a channel, all of its states in registers, two to an
 // instruction.  Chunks give the machine its threads, so a channel need not be spread over lanes: nothing is exchanged between
 // lanes, the step size and the gate are taken once a channel, and a token's sixteen states are sixteen chains side by side.
-// What bounds it: the FMA units (fifteen of a state's twenty operations a walk).
+// What bounds it: the FMA pipe (fifteen of a state's twenty operations a walk), active 57 % of the time, and the ALU's (48 %).
 // 4,096 channels of 16 states in bfloat16, against eight lanes a channel: runs of 64, 376, 688 and 1,000 tokens in one piece
 // 407 us, in chunks of 64 256; one of 1,000 221 and 123 (chunks of 32); one of 2,040 in chunks of 128 459, now 229 (of 64).
 // ---------------------------------------------------------------------------
@@ -270,7 +270,8 @@ selective_carry_kernel(SelectiveScanArgs a) {
 #define SC_TOKENS 64        // tokens whose B and C are staged at a time
 #define SC_GROUP 4          // tokens whose step size, input and gate are on their way while as many are walked
 
-// e^x of two numbers that are never positive: x = k ln 2 + f with the logarithm in two parts (Cody and Waite), |f| < 0.347, and
+// e^x of two numbers that are never positive: x = k ln 2 + f with the logarithm in two parts (Cody and Waite: the high part has
+// 15 bits, so that k, of up to 7 bits, times it is exact, and the low part is what is left of ln 2), |f| < 0.347, and
 // the series of e^f to f^7 (the next term is below 2^-27).  Near zero k is 0 and f is x itself, so a slow decay is rounded once.
 // Below -87 (where k would leave the exponent) it is zero.
 __device__ __forceinline__ unsigned long long ss_decay2(unsigned long long x2) {
