@@ -996,15 +996,19 @@ rms_norm_pair_kernel(const float* x, const float* __restrict__ g1, const float* 
     }
 }
 
-// the same by pieces, a block a row.  2,128 rows of 2,048: 29.5 -> 6.1 us; 4 rows: 3.2 -> 1.4 us.
+// the same by pieces, a block a row, or of many narrow rows several (blockDim.y).  2,128 rows of 2,048: 29.5 -> 6.1 us; 4 rows: 3.2 ->
+// 1.4 us.  12,411 rows of 64, 128 and 256 took 4.4, 4.9 and 6.8 us element by element with a warp a row, 13.5 us with a
+// block each; with four or eight a block 3.6, 3.7 and 5.7.
 template <typename TO, int NV4, int G>
 __global__ void __launch_bounds__(256)
 rms_norm_pair_rows_kernel(const float* x, const float* __restrict__ g1, const float* __restrict__ g2,
-                          TO* __restrict__ out1, TO* __restrict__ out2, int D, float eps) {
-    __shared__ float red[8];
+                          TO* __restrict__ out1, TO* __restrict__ out2, int R, int D, float eps) {
+    __shared__ float sums[8][8];
+    float* red = sums[threadIdx.y];
     gl_grid_launch_dependents();
     const int n4 = D >> 2;
-    const size_t base = (size_t)blockIdx.x * D;
+    const int row = blockIdx.x * blockDim.y + threadIdx.y;
+    const size_t base = (size_t)min(row, R - 1) * D;               // (all of a block's threads meet at the sums)
     float4 a[NV4], b[NV4], v[NV4];
     row_weights(a, g1, n4);
     row_weights(b, g2, n4);
@@ -1019,7 +1023,7 @@ rms_norm_pair_rows_kernel(const float* x, const float* __restrict__ g1, const fl
 #pragma unroll
     for (int i = 0; i < NV4; ++i) {
         const int k = threadIdx.x + i * blockDim.x;
-        if (k >= n4) break;
+        if (k >= n4 || row >= R) break;
         const float4 y = make_float4(v[i].x * inv, v[i].y * inv, v[i].z * inv, v[i].w * inv);
         row_put(out1 + base, k, make_float4(y.x * a[i].x, y.y * a[i].y, y.z * a[i].z, y.w * a[i].w));
         row_put(out2 + base, k, make_float4(y.x * b[i].x, y.y * b[i].y, y.z * b[i].z, y.w * b[i].w));
@@ -1029,7 +1033,9 @@ rms_norm_pair_rows_kernel(const float* x, const float* __restrict__ g1, const fl
 template <typename TO>
 static int launch_rms_norm_pair_rows(const float* x, const float* g1, const float* g2, TO* out1, TO* out2, int R, int D, float eps,
                                      const RowShape& shape, cudaStream_t stream) {
-#define CALL(N, G) gl_launch(rms_norm_pair_rows_kernel<TO, N, G>, dim3((unsigned)R), dim3(shape.threads), 0, stream, 1, x, g1, g2, out1, out2, D, eps)
+    const int rows = R >= 1024 && shape.threads <= 64 ? 256 / shape.threads : 1;
+    const dim3 grid((unsigned)((R + rows - 1) / rows)), block(shape.threads, rows);
+#define CALL(N, G) gl_launch(rms_norm_pair_rows_kernel<TO, N, G>, grid, block, 0, stream, 1, x, g1, g2, out1, out2, R, D, eps)
     return ROW_BY_PIECES(shape, CALL);
 #undef CALL
 }

@@ -26,3 +26,16 @@ def test_rows_do_not_depend_on_their_number(D):
     for rows in (1, 63, 64, 299):
         for got, want in zip(all_of(rows), whole):
             assert torch.equal(got, want[:rows]), rows
+
+
+@pytest.mark.parametrize("D", [4, 64, 128, 132, 256, 260, 384, 512])
+def test_many_narrow_rows(D):
+    """Several rows a block (the pair of norms from 1,024 rows on), the last block part empty: the rows of a call of few."""
+    from gopherllm_b200 import ops as o
+    g = torch.Generator().manual_seed(D)
+    x, w1, w2 = torch.randn(1027, D, generator=g).cuda(), torch.randn(D, generator=g).cuda(), torch.randn(D, generator=g).cuda()
+    for dtype in (torch.float32, torch.bfloat16):
+        many = o.rms_norm_pair(x, w1, w2, 1e-6, dtype)
+        for at in (0, 500, 1000):
+            for few, all_rows in zip(o.rms_norm_pair(x[at:at + 27].contiguous(), w1, w2, 1e-6, dtype), many):
+                assert torch.equal(few, all_rows[at:at + 27])
